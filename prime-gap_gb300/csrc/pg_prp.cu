@@ -8,6 +8,10 @@
 // (load_batch_thread, run_gpu_thread, run_overflow_thread,
 // gap_test_gpu.cu:213-640) with device rounds.
 //
+// Numbers wide and many enough are tested in a residue number system on the
+// tensor cores (pg_rns.cu); the limb arithmetic here takes the others, and the
+// few that the residue form leaves.
+//
 // Numbers: n = 8L little-endian 32-bit limbs over a group of 8 lanes of a
 // warp, lane t holding limbs [tL, tL + L).  N < 2^(32n - 4), so R = 2^(32n) is
 // at least 16N and Montgomery products of inputs below 4N stay below 2N: 2^d
@@ -32,6 +36,7 @@
 
 #include "pg_arith.cuh"
 #include "pg_host.h"
+#include "pg_rns.h"
 
 namespace pg {
 
@@ -289,21 +294,18 @@ __device__ bool prp2(const Grp &g, const Num<L> &n, const uint32_t *sn) {
     }
 }
 
-struct PrpItem {
-    uint32_t row;  // row of the base numbers
-    int32_t x;     // N = base[row] + x
-};
-
+// list: the items to test where not all are
 template <int L>
 __global__ void __launch_bounds__(kPrpThreads)
     prp_kernel(const uint32_t *__restrict__ bases, const PrpItem *__restrict__ items,
-               const unsigned long long *count, uint64_t max_items, uint8_t *__restrict__ result) {
+               const uint32_t *__restrict__ list, const unsigned long long *count, uint64_t max_items, uint8_t *__restrict__ result) {
     __shared__ uint32_t s_n[kGroups][8 * L];
     const Grp g = group_of_lane();
     const uint32_t gi = threadIdx.x / kTPI;
-    const uint64_t i = (uint64_t)blockIdx.x * kGroups + gi;
+    uint64_t i = (uint64_t)blockIdx.x * kGroups + gi;
     const uint64_t n_items = count ? min((uint64_t)*count, max_items) : max_items;
     if (i >= n_items) return;  // the whole group leaves together
+    if (list) i = list[i];
     const PrpItem it = items[i];
     const uint32_t *src = bases + (uint64_t)it.row * (8 * L) + g.t * L;
     Num<L> n;
@@ -318,13 +320,13 @@ __global__ void __launch_bounds__(kPrpThreads)
     if (g.t == 0) result[i] = r ? 1 : 0;
 }
 
-cudaError_t launch_prp(int L, const uint32_t *bases, const PrpItem *items, const unsigned long long *count,
-                       uint64_t max_items, uint8_t *result, cudaStream_t s) {
+cudaError_t launch_prp(int L, const uint32_t *bases, const PrpItem *items, const uint32_t *list,
+                       const unsigned long long *count, uint64_t max_items, uint8_t *result, cudaStream_t s) {
     if (max_items == 0) return cudaSuccess;
     const unsigned blocks = (unsigned)((max_items + kGroups - 1) / kGroups);
 #define PG_PRP_CASE(LL)                                                                               \
     case LL:                                                                                          \
-        prp_kernel<LL><<<blocks, kPrpThreads, 0, s>>>(bases, items, count, max_items, result);        \
+        prp_kernel<LL><<<blocks, kPrpThreads, 0, s>>>(bases, items, list, count, max_items, result);  \
         break;
     switch (L) {
         PG_PRP_CASE(1)
@@ -352,6 +354,57 @@ cudaError_t launch_prp(int L, const uint32_t *bases, const PrpItem *items, const
 
 // Limbs per lane for numbers of `bits` bits: 32*8L >= bits + 4.
 int limbs_per_lane(uint32_t bits) { return (int)((bits + 4 + 255) / 256); }
+
+// How a call's numbers are tested: on the tensor cores where their width allows
+// it (pg_rns.cu) with what is left over tested limb by limb, or limb by limb.
+struct PrpPlan {
+    int L = 0;
+    uint32_t bits = 0;
+    bool rns = false;
+    RnsLayout layout{};
+    size_t work_bytes() const { return rns ? layout.total : 0; }
+};
+
+// Where the residue form is the faster one, in ms for 16 numbers and for 19456
+// (limbs, residues): 200 bits 0.21, 0.32 and 0.44, 0.51; 256 bits 0.46, 0.39 and
+// 1.21, 0.61; 712 bits 1.61, 1.74 and 4.94, 2.07 (5000 numbers: 2.15, 1.85); 1100
+// bits 4.36, 3.58; 1400 bits 6.33, 5.98 and 29.9, 6.7; 2136 bits 16.0, 13.3 and 105,
+// 14.8.  So from two limbs per lane on; with two or three chunks of slots and
+// fewer than three limbs per lane only for enough numbers to fill the limb form.
+bool rns_pays(uint32_t bits, uint64_t max_items) {
+    const uint32_t n = rns_chunks(bits);
+    if (bits < 253 || n == 0) return false;
+    return n == 1 || bits >= 765 || max_items >= 4096;
+}
+
+PrpPlan prp_plan(uint32_t bits, uint64_t max_items) {
+    PrpPlan p;
+    p.bits = bits;
+    p.L = limbs_per_lane(bits);
+    p.rns = rns_pays(bits, max_items);
+    if (p.rns) p.layout = rns_layout(bits, 8u * (uint32_t)p.L, max_items);
+    return p;
+}
+
+cudaError_t prp_begin(const PrpPlan &p, void *work, cudaStream_t s) {
+    return p.rns ? rns_begin(p.layout, p.bits, work, s) : cudaSuccess;
+}
+
+cudaError_t prp_launch(const PrpPlan &p, void *work, const uint32_t *bases, const PrpItem *items,
+                       const unsigned long long *count, uint64_t max_items, uint8_t *result, cudaStream_t s) {
+    if (!p.rns) return launch_prp(p.L, bases, items, nullptr, count, max_items, result, s);
+    const cudaError_t e = rns_test(p.layout, p.bits, work, bases, items, count, max_items, result, s);
+    if (e != cudaSuccess) return e;
+    return launch_prp(p.L, bases, items, rns_fallback_list(p.layout, work), rns_fallback_count(p.layout, work),
+                      max_items, result, s);
+}
+
+// *error (host) = nonzero after a wait on the device that gave up
+cudaError_t prp_error(const PrpPlan &p, void *work, unsigned long long *error, cudaStream_t s) {
+    *error = 0;
+    return p.rns ? cudaMemcpyAsync(error, rns_error(p.layout, work), sizeof(*error), cudaMemcpyDeviceToHost, s)
+                 : cudaSuccess;
+}
 
 // ---------------------------------------------------------------------------
 // gap search
@@ -618,8 +671,8 @@ int pgs_prp_test(pgs_ctx *ctx, const uint32_t *limbs, uint32_t n_limbs, size_t c
         dev_rows.push_back(i);
     }
     if (dev_rows.empty()) return PGS_OK;
-    const int L = pg::limbs_per_lane(max_bits);
-    const uint32_t n = 8u * (uint32_t)L;
+    const pg::PrpPlan plan = pg::prp_plan(max_bits, dev_rows.size());
+    const uint32_t n = 8u * (uint32_t)plan.L;
     std::vector<uint32_t> packed(dev_rows.size() * n, 0u);
     std::vector<pg::PrpItem> items(dev_rows.size());
     for (size_t j = 0; j < dev_rows.size(); j++) {
@@ -628,21 +681,29 @@ int pgs_prp_test(pgs_ctx *ctx, const uint32_t *limbs, uint32_t n_limbs, size_t c
         items[j] = pg::PrpItem{(uint32_t)j, 0};
     }
     const cudaStream_t s = ctx->stream;
-    DevBuf d_nums, d_items, d_res;
-    DevBuf *bufs[] = {&d_nums, &d_items, &d_res};
+    DevBuf d_nums, d_items, d_res, d_work;
+    DevBuf *bufs[] = {&d_nums, &d_items, &d_res, &d_work};
     for (DevBuf *b : bufs) b->pool = &ctx->dpool;
     std::vector<uint8_t> res(dev_rows.size());
     cudaError_t e = upload(d_nums, packed, s);
     if (e == cudaSuccess) e = upload(d_items, items, s);
     if (e == cudaSuccess) e = d_res.ensure(dev_rows.size());
+    if (e == cudaSuccess) e = d_work.ensure(plan.work_bytes());
+    if (e == cudaSuccess) e = pg::prp_begin(plan, d_work.p, s);
     if (e == cudaSuccess)
-        e = pg::launch_prp(L, d_nums.as<uint32_t>(), d_items.as<pg::PrpItem>(), nullptr, dev_rows.size(),
+        e = pg::prp_launch(plan, d_work.p, d_nums.as<uint32_t>(), d_items.as<pg::PrpItem>(), nullptr, dev_rows.size(),
                            d_res.as<uint8_t>(), s);
+    unsigned long long gave_up = 0;
+    if (e == cudaSuccess) e = pg::prp_error(plan, d_work.p, &gave_up, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(res.data(), d_res.p, res.size(), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     cudaStreamSynchronize(s);
     for (DevBuf *b : bufs) b->release();
     if (e != cudaSuccess) return fail(ctx, e, "pgs_prp_test");
+    if (gave_up) {
+        ctx->err = "pgs_prp_test: a wait on the device gave up";
+        return PGS_ETIMEOUT;
+    }
     for (size_t j = 0; j < dev_rows.size(); j++) out[dev_rows[j]] = res[j];
     return PGS_OK;
 }
@@ -673,22 +734,22 @@ int prp_gaps_core(pgs_ctx *ctx, const pgs_gap_params *prm, uint64_t rows, const 
         ctx->err = "pgs_prp_gaps: m*K above 4092 bits";
         return PGS_EINVAL;
     }
-    const int L = pg::limbs_per_lane(bits);
-    const uint32_t n = 8u * (uint32_t)L;
+    const uint64_t max_items = std::max<uint64_t>(rows, kRoundTarget + kMaxSpec);
+    const pg::PrpPlan plan = pg::prp_plan(bits, max_items);
+    const uint32_t n = 8u * (uint32_t)plan.L;
     std::vector<uint32_t> skip(rows, 0u);
     if (prm->one_side_skip) {
         const double klog = k_log(k);
         for (uint64_t r = 0; r < rows; r++) skip[r] = skip_threshold(klog, h_m[r], prm->min_merit);
     }
     const cudaStream_t s = ctx->stream;
-    DevBuf d_k, d_kp, d_skip, d_centers, d_state, d_items, d_res, d_out, d_ctr;
-    DevBuf *bufs[] = {&d_k, &d_kp, &d_skip, &d_centers, &d_state, &d_items, &d_res, &d_out, &d_ctr};
+    DevBuf d_k, d_kp, d_skip, d_centers, d_state, d_items, d_res, d_out, d_ctr, d_work;
+    DevBuf *bufs[] = {&d_k, &d_kp, &d_skip, &d_centers, &d_state, &d_items, &d_res, &d_out, &d_ctr, &d_work};
     for (DevBuf *b : bufs) b->pool = &ctx->dpool;
     auto cleanup = [&] {
         cudaStreamSynchronize(s);
         for (DevBuf *b : bufs) b->release();
     };
-    const uint64_t max_items = std::max<uint64_t>(rows, kRoundTarget + kMaxSpec);
     cudaError_t e = upload(d_k, k, s);
     if (e == cudaSuccess) e = upload(d_kp, kprimes, s);
     if (e == cudaSuccess) e = upload(d_skip, skip, s);
@@ -698,6 +759,8 @@ int prp_gaps_core(pgs_ctx *ctx, const pgs_gap_params *prm, uint64_t rows, const 
     if (e == cudaSuccess) e = d_res.ensure(max_items);
     if (e == cudaSuccess) e = d_out.ensure(rows * sizeof(pgs_gap_result));
     if (e == cudaSuccess) e = d_ctr.ensure(32);
+    if (e == cudaSuccess) e = d_work.ensure(plan.work_bytes());
+    if (e == cudaSuccess) e = pg::prp_begin(plan, d_work.p, s);
     if (e != cudaSuccess) {
         cleanup();
         return fail(ctx, e, "pgs_prp_gaps setup");
@@ -723,8 +786,11 @@ int prp_gaps_core(pgs_ctx *ctx, const pgs_gap_params *prm, uint64_t rows, const 
                                              (uint32_t)kprimes.size(), x_limit, d_items.as<pg::PrpItem>(),
                                              max_items, ctr, ctr + 2);
         const uint64_t bound = std::min<uint64_t>(max_items, active * spec);
-        e = pg::launch_prp(L, d_centers.as<uint32_t>(), d_items.as<pg::PrpItem>(), ctr, bound,
+        e = pg::prp_launch(plan, d_work.p, d_centers.as<uint32_t>(), d_items.as<pg::PrpItem>(), ctr, bound,
                            d_res.as<uint8_t>(), s);
+        if (e) break;
+        unsigned long long gave_up = 0;
+        e = pg::prp_error(plan, d_work.p, &gave_up, s);
         if (e) break;
         pg::resolve_kernel<<<rb, 256, 0, s>>>(d_state.as<pg::GapRow>(), rows, ls, d_items.as<pg::PrpItem>(),
                                               d_res.as<uint8_t>(), prm->sieve_length, d_out.as<pgs_gap_result>(),
@@ -733,6 +799,11 @@ int prp_gaps_core(pgs_ctx *ctx, const pgs_gap_params *prm, uint64_t rows, const 
         if (e == cudaSuccess) e = cudaMemcpyAsync(host_ctr, ctr, 24, cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e) break;
+        if (gave_up) {
+            cleanup();
+            ctx->err = "pgs_prp_gaps: a wait on the device gave up";
+            return PGS_ETIMEOUT;
+        }
         launched += host_ctr[0];
         active = host_ctr[1];
         if (++rounds > (1u << 22)) {

@@ -1,0 +1,951 @@
+// Base-2 strong probable-prime tests on the tensor cores.
+//
+// Replaces, for many numbers of one size, the limb arithmetic of the reference's
+// kernel_miller_rabin (miller_rabin.h:154-267).  A test is a chain of about
+// log2 N squarings mod N, and a chain of squarings of different numbers has no
+// matrix product in it -- unless the numbers are held as residues: Montgomery
+// reduction in a residue number system (Posch and Posch 1995; Bajard, Didier and
+// Kornerup 1998; the quotient's rank as in Kawamura et al. 2000) needs two base
+// extensions per squaring, and a base extension is a product with a matrix of
+// constants that every number shares.
+//
+// Two bases of pairwise coprime moduli up to 4096: A (primes) and B.  x is held
+// as |x| <= cN in both.  With xi_i = x_i^2 (-N^-1) (A/m_i)^-1 mod m_i,
+// q = sum xi_i A/m_i is congruent to -x^2/N mod A, |q| <= A k/2, and
+// (x^2 + q N)/A is again below cN when 4c^2 N <= A (x^2 may come doubled twice).
+// First extension (q to B): q_j = sum_i xi_i ((A/m_i) mod m_j).  Then in B
+// r_j = (x_j^2 + q_j N_j)/A, held as xi_j = r_j (B/m_j)^-1.  Second extension
+// (r back to A): r_i = sum_j xi_j ((B/m_j) mod m_i) - a (B mod m_i), with
+// a = round(sum_j xi_j / m_j), exact since |r| <= B/4.
+//
+// Exact arithmetic in floating point.  Residues are balanced, |xi| <= 2048, so
+// one f16 holds one; a matrix entry is split as c = lo + hi, |lo| <= 32 and hi a
+// multiple of 64, each exact in f16, and the two sums stay below 2^24 (times 64
+// for hi): the tensor core's f32 accumulators hold them exactly.  Everything
+// between the products is f32 multiply-adds whose results are whole numbers
+// below 2^24 (the remainder of T by m: q = rint(T/m) by adding 1.5 2^23, then
+// T - q m, exact in a fused multiply-add).
+//
+// A pair of CTAs takes 256 numbers, 128 TMEM lanes each, a lane a number.  The
+// two matrices (K x 2K f16) stay in the pair's shared memory for the whole
+// chain, half the columns in each CTA (cta_group::2), so nothing but the
+// numbers' own constants is read again.  The residues are the A operand and lie
+// in TMEM, written there by the threads that compute them.  Output columns come
+// in blocks of 64 slots (128 columns); while 16 warps turn a block of sums into
+// residues, 32 slots at a time, the tensor cores work on the next one, and the next
+// product's first block accumulates slice by slice as the residues appear.
+//
+// Measured (2136-bit numbers, 19456 at once): 14.8 ms, 1.32e6 tests/s, where the
+// limb form takes 105 ms; a squaring step 6.2 us per pair, of which the products
+// alone take 2.9 (128 columns cost 78 cycles per 16 of K; 64 columns cost the same,
+// the A operand's read, hence blocks of 128) and the residues' f32 operations 3.4.
+#include "pg_rns.h"
+
+#include <cuda_fp16.h>
+
+#include <cmath>
+#include <cstring>
+#include <map>
+#include <memory>
+#include <mutex>
+#include <vector>
+
+namespace pg {
+
+namespace {
+
+constexpr uint32_t kSlots = 32;                        // residue slots per chunk
+constexpr uint32_t kMaxK = kSlots * kRnsMaxChunks;     // 224
+constexpr uint32_t kWarps = 16;                        // warps that compute residues
+constexpr uint32_t kThreads = 32 * (kWarps + 1);       // and one that issues products
+constexpr float kMagic = 12582912.0f;                  // 1.5 2^23
+
+// Constants of two neighbouring slots, as the paired f32 operations read them.
+struct SlotPair {
+    float neg_m[2], inv_m[2], c[2];  // -m, 1/m; A: -(B mod m), B: (B/m) / A mod m
+    float pad[2];
+};
+struct RnsConst {
+    SlotPair a[kMaxK / 2], b[kMaxK / 2];
+};
+
+// What the kernels around the chain need of each slot.
+struct RnsSlots {
+    uint16_t ma[kMaxK], mb[kMaxK];   // moduli (base A: slot 0 is the rank's column, modulus 1)
+    uint16_t am[kMaxK];              // A/m_i mod m_i
+    uint16_t ab[kMaxK];              // A mod m_j
+    uint16_t gb[kMaxK];              // (B/m_j)^-1 mod m_j
+    uint16_t ba[kMaxK];              // B mod m_i
+    uint32_t b_primes;               // the first moduli of B, prime
+};
+
+struct RnsPlan {
+    RnsConst k;
+    RnsSlots s;
+    double a_mant;        // A = a_mant 2^a_exp, a_mant in [1, 2)
+    int a_exp;
+    uint32_t t_max;       // largest multiple of N between two values of one residue
+};
+
+uint32_t inverse(uint32_t a, uint32_t m) {  // extended Euclid; a and m coprime
+    int64_t r0 = m, r1 = a % m, t0 = 0, t1 = 1;
+    while (r1) {
+        const int64_t q = r0 / r1;
+        const int64_t r2 = r0 - q * r1, t2 = t0 - q * t1;
+        r0 = r1, r1 = r2, t0 = t1, t1 = t2;
+    }
+    return (uint32_t)(t0 < 0 ? t0 + m : t0);
+}
+
+float balanced(uint32_t x, uint32_t m) { return x > m / 2 ? (float)x - (float)m : (float)x; }
+
+// The moduli of 32n slots in each base and the bits that they hold.  A takes
+// primes alone (N has to be a unit there); B ends with composite moduli near
+// 4096 made of small primes of their own, which hold more than the primes that
+// they stand in for (2136-bit numbers fit six chunks, not seven).
+struct RnsModuli {
+    std::vector<uint32_t> a, b;
+    uint32_t b_primes = 0;
+    double bits = 0;  // numbers below 2^bits
+};
+
+double log2_product(const std::vector<uint32_t> &v) {
+    double l = 0;
+    for (uint32_t q : v) l += std::log2((double)q);
+    return l;
+}
+
+// |x| <= c N; 4 c^2 N <= A and c N <= B / 4
+double coefficient(size_t k) { return 0.5 * (double)k + 1; }
+double a_capacity(double log_a, size_t k) { return log_a - 2 - 2 * std::log2(coefficient(k)); }
+
+RnsModuli make_moduli(uint32_t n) {
+    const uint32_t k = kSlots * n;
+    std::vector<uint8_t> comp(4097, 0), used(4097, 0);
+    std::vector<uint32_t> primes, extra;
+    for (uint32_t q = 2; q <= 4096; q++) {
+        if (comp[q]) continue;
+        primes.push_back(q);
+        for (uint32_t t = q * q; t <= 4096; t += q) comp[t] = 1;
+    }
+    for (uint32_t c = 4096; c > 3900; c--) {
+        std::vector<uint32_t> f;
+        uint32_t rest = c;
+        for (uint32_t q : primes) {
+            if (q > 200) break;
+            if (rest % q == 0 && !used[q]) f.push_back(q);
+            while (rest % q == 0 && !used[q]) rest /= q;
+        }
+        if (!comp[c] || rest != 1) continue;
+        for (uint32_t q : f) used[q] = 1;
+        extra.push_back(c);
+    }
+    // A needs log2 c + 2 more bits than B: it gets the first `lead` primes
+    RnsModuli best;
+    for (uint32_t lead = 0; lead < 24; lead++) {
+        RnsModuli m;
+        size_t top = primes.size();
+        while (m.a.size() + 1 < k || m.b.size() + extra.size() < k) {
+            const uint32_t q = primes[--top];
+            const bool b_full = m.b.size() + extra.size() >= k;
+            (m.a.size() + 1 < k && (b_full || m.a.size() < m.b.size() + lead) ? m.a : m.b).push_back(q);
+        }
+        m.b_primes = (uint32_t)m.b.size();
+        m.b.insert(m.b.end(), extra.begin(), extra.end());
+        const double c = coefficient(m.a.size());
+        m.bits = std::fmin(a_capacity(log2_product(m.a), m.a.size()), log2_product(m.b) - 2 - std::log2(c));
+        if (m.bits > best.bits) best = m;
+    }
+    return best;
+}
+
+const RnsModuli &moduli_of(uint32_t n) {
+    static const std::vector<RnsModuli> all = [] {
+        std::vector<RnsModuli> v(kRnsMaxChunks + 1);
+        for (uint32_t i = 1; i <= kRnsMaxChunks; i++) v[i] = make_moduli(i);
+        return v;
+    }();
+    return all[n];
+}
+
+// How many of A's moduli numbers below 2^bits take: no more, so that A / N stays
+// small (the start needs A mod N).
+uint32_t a_count(uint32_t n, uint32_t bits) {
+    const RnsModuli &mod = moduli_of(n);
+    double la = 0;
+    uint32_t k = 0;
+    while (k < mod.a.size() && (k == 0 || a_capacity(la, k) - 1e-6 < (double)bits)) la += std::log2((double)mod.a[k++]);
+    return k;
+}
+
+void make_plan(uint32_t n, uint32_t ka, RnsPlan &p) {
+    const RnsModuli &mod = moduli_of(n);
+    const uint32_t k = kSlots * n;
+    const std::vector<uint32_t> a(mod.a.begin(), mod.a.begin() + ka);
+    std::memset(&p, 0, sizeof(p));
+    p.t_max = (uint32_t)(2 * coefficient(a.size()) + 4);
+    p.a_mant = 1;
+    for (uint32_t q : a) {
+        int e;
+        p.a_mant = std::frexp(p.a_mant * q, &e);
+        p.a_exp += e;
+    }
+    auto prod = [](const std::vector<uint32_t> &v, uint32_t m, uint32_t but) {
+        uint32_t r = 1;
+        for (uint32_t q : v)
+            if (q != but) r = r * q % m;  // below 2^24
+        return r;
+    };
+    p.s.b_primes = mod.b_primes;
+    for (uint32_t i = 0; i < k; i++) {
+        p.s.ma[i] = 1;
+        if (i == 0 || i > a.size()) continue;
+        const uint32_t m = a[i - 1];
+        p.s.ma[i] = (uint16_t)m;
+        p.s.am[i] = (uint16_t)prod(a, m, m);
+        p.s.ba[i] = (uint16_t)prod(mod.b, m, 0);
+    }
+    for (uint32_t j = 0; j < k; j++) {
+        const uint32_t m = mod.b[j];
+        p.s.mb[j] = (uint16_t)m;
+        p.s.ab[j] = (uint16_t)prod(a, m, 0);
+        p.s.gb[j] = (uint16_t)inverse(prod(mod.b, m, m), m);
+    }
+    for (uint32_t i = 0; i < k; i++) {
+        SlotPair &pa = p.k.a[i / 2], &pb = p.k.b[i / 2];
+        const uint32_t h = i & 1;
+        const uint32_t ma = p.s.ma[i], mb = p.s.mb[i];
+        pa.neg_m[h] = -(float)ma;
+        pa.inv_m[h] = 1.0f / (float)ma;
+        pa.c[h] = ma > 1 ? -balanced(p.s.ba[i], ma) : 0.0f;
+        pb.neg_m[h] = -(float)mb;
+        pb.inv_m[h] = 1.0f / (float)mb;
+        pb.c[h] = balanced(inverse(p.s.gb[i], mb) * inverse(p.s.ab[i], mb) % mb, mb);
+    }
+}
+
+// One plan per (n, moduli of A): constants, made on first use and kept for the
+// process, at most about kMaxK of 10 KB.
+const RnsPlan &plan_of(uint32_t n, uint32_t bits) {
+    static std::mutex mu;
+    static std::map<uint32_t, std::unique_ptr<RnsPlan>> plans;
+    const uint32_t ka = a_count(n, bits);
+    std::lock_guard<std::mutex> g(mu);
+    std::unique_ptr<RnsPlan> &p = plans[n << 16 | ka];
+    if (!p) {
+        p.reset(new RnsPlan);
+        make_plan(n, ka, *p);
+    }
+    return *p;
+}
+
+// ---------------------------------------------------------------------------
+// device arithmetic on residues below 4096
+
+// v mod m; inv32 = floor((2^32 - 1) / m): the quotient is at most one short
+__device__ __forceinline__ uint32_t mod_small(uint32_t v, uint32_t m, uint32_t inv32) {
+    uint32_t r = v - __umulhi(v, inv32) * m;
+    return r >= m ? r - m : r;
+}
+
+__device__ uint32_t pow_small(uint32_t x, uint32_t e, uint32_t m, uint32_t inv32) {
+    uint32_t r = 1;
+    for (; e; e >>= 1) {
+        if (e & 1) r = mod_small(r * x, m, inv32);
+        x = mod_small(x * x, m, inv32);
+    }
+    return r;
+}
+
+// a^-1 mod m (m not always prime), by Euclid; a and m coprime
+__device__ uint32_t inverse_small(uint32_t a, uint32_t m) {
+    int r0 = (int)m, r1 = (int)(a % m), t0 = 0, t1 = 1;
+    while (r1) {
+        const int q = r0 / r1, r2 = r0 - q * r1, t2 = t0 - q * t1;
+        r0 = r1, r1 = r2, t0 = t1, t1 = t2;
+    }
+    return (uint32_t)(t0 < 0 ? t0 + (int)m : t0);
+}
+
+__device__ __forceinline__ int balance(uint32_t x, uint32_t m) { return x > m / 2 ? (int)x - (int)m : (int)x; }
+
+__device__ __forceinline__ uint32_t inv32_of(uint32_t m) { return m > 1 ? 0xFFFFFFFFu / m : 0u; }
+
+// The matrices as the tensor cores read them from shared memory.  Per CTA of
+// the pair (0: the low parts, 1: the high parts), product (0: xi of B into A,
+// 1: xi of A into B) and block of 64 output slots (the last may have 32), 8 x 8
+// pieces of 128 bytes, neighbouring outputs together: [k/8][slot/8][slot%8][k%8].
+__global__ void matrix_kernel(const __grid_constant__ RnsSlots p, uint32_t chunks, __half *__restrict__ out) {
+    const uint32_t k = kSlots * chunks;
+    const uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= 2 * k * k) return;
+    const uint32_t product = idx / (k * k), in = idx % (k * k) / k, o = idx % k;
+    float lo = 0, hi = 0;
+    if (product == 0) {
+        const uint32_t mj = p.mb[in];
+        const uint32_t m = p.ma[o], inv = inv32_of(m);  // m prime, or 1
+        if (o == 0) {
+            lo = 4096.0f / (float)mj;  // the rank's column: xi_j / m_j
+        } else if (m > 1) {
+            const int c = balance(mod_small(p.ba[o] * pow_small(mj % m, m - 2, m, inv), m, inv), m);
+            const int l = ((c + 32) & 63) - 32;
+            lo = (float)l, hi = (float)(c - l);
+        }
+    } else if (p.ma[in] > 1) {
+        const uint32_t m = p.mb[o];
+        const int c = balance(mod_small(p.ab[o] * inverse_small(p.ma[in], m), m, inv32_of(m)), m);
+        const int l = ((c + 32) & 63) - 32;
+        lo = (float)l, hi = (float)(c - l);
+    }
+    const uint32_t block = o / 64, slot = o % 64, rows = min(64u, k - 64 * block);
+    const uint64_t at = (uint64_t)product * k * k + block * 64 * k +
+                        (in / 8 * (rows / 8) + slot / 8) * 64 + slot % 8 * 8 + in % 8;
+    out[at] = __float2half_rn(lo);
+    out[at + 2ull * k * k] = __float2half_rn(hi);
+}
+
+// Halves of a number's slots lie as the chain's threads load them: 8 slots of
+// one warp group per 16 bytes, neighbouring numbers together.
+__device__ __forceinline__ uint64_t slot_at(uint32_t chunks, uint64_t number, uint32_t slot) {
+    const uint64_t tile = number / 128, row = number % 128;
+    return ((tile * chunks * 4 + slot / 8) * 128 + row) * 8 + slot % 8;
+}
+
+enum { kFlagRun = 0, kFlagComposite = 1, kFlagOther = 2 };
+
+// Per number: its limbs, its constants in every slot, its start (the Montgomery
+// form of 1).  A block takes 8 numbers; a thread one slot of each base.
+// Bound by the remainders' Horner chains (two multiplies per 16 bits): about 2 %
+// of the chain's time.
+constexpr uint32_t kSetupNumbers = 8;
+__global__ void setup_kernel(const __grid_constant__ RnsSlots p, uint32_t chunks, uint32_t bits, double a_mant,
+                             int a_exp, uint32_t limbs, const uint32_t *__restrict__ bases,
+                             const PrpItem *__restrict__ items, const unsigned long long *count, uint64_t max_items,
+                             __half *__restrict__ num_a, __half *__restrict__ num_b, __half *__restrict__ state,
+                             uint32_t *__restrict__ nums, long long *__restrict__ quot, uint32_t *__restrict__ flag) {
+    __shared__ uint32_t s_n[kSetupNumbers][128];
+    __shared__ long long s_q[kSetupNumbers];
+    __shared__ uint32_t s_f[kSetupNumbers];
+    const uint64_t n_items = count ? min((uint64_t)*count, max_items) : max_items;
+    const uint64_t padded = (n_items + kRnsTile - 1) / kRnsTile * kRnsTile;
+    const uint64_t first = (uint64_t)blockIdx.x * kSetupNumbers;
+    if (first >= padded) return;
+    if (threadIdx.x < kSetupNumbers) {
+        const uint32_t g = threadIdx.x;
+        const uint64_t i = first + g;
+        long long q = 0;
+        uint32_t f = kFlagComposite;
+        if (i < n_items) {
+            const PrpItem it = items[i];
+            const uint32_t *src = bases + (uint64_t)it.row * limbs;
+            uint32_t *dst = nums + i * limbs;
+            int64_t carry = it.x;
+            int top = -1;
+            for (uint32_t w = 0; w < limbs; w++) {
+                const int64_t v = (int64_t)src[w] + carry;
+                const uint32_t lo = (uint32_t)v;
+                carry = v >> 32;
+                s_n[g][w] = lo;
+                dst[w] = lo;
+                if (lo) top = (int)w;
+            }
+            // floor(A / N) from the leading words; N within 20 bits of the widest
+            f = kFlagOther;
+            if (top >= 3) {
+                const double n = ((double)s_n[g][top] * 4294967296.0 + (double)s_n[g][top - 1]) * 4294967296.0 +
+                                 (double)s_n[g][top - 2];
+                const double len = log2(n) + 32.0 * (top - 2);
+                if (len > (double)bits - 20.0) {
+                    q = (long long)floor(ldexp(a_mant / n, a_exp - 32 * (top - 2)));
+                    f = kFlagRun;
+                }
+            }
+        }
+        s_q[g] = q;
+        s_f[g] = f;
+    }
+    __syncthreads();
+    const uint32_t t = threadIdx.x;
+    const uint32_t ma = p.ma[t], mb = p.mb[t];
+    const uint32_t ia = inv32_of(ma), ib = inv32_of(mb);
+    const uint32_t ainv = inverse_small(p.ab[t], mb);
+    for (uint32_t g = 0; g < kSetupNumbers; g++) {
+        const uint64_t i = first + g;
+        const uint64_t at = slot_at(chunks, i, t);
+        if (s_f[g] != kFlagRun) {  // an all-zero lane
+            num_a[at] = __half(0.0f);
+            num_b[at] = __half(0.0f);
+            state[at] = __half(0.0f);
+            continue;
+        }
+        uint32_t ra = 0, rb = 0;
+        for (int w = (int)limbs - 1; w >= 0; w--) {
+            const uint32_t v = s_n[g][w];
+            ra = mod_small((ra << 16) | (v >> 16), ma, ia);
+            rb = mod_small((rb << 16) | (v >> 16), mb, ib);
+            ra = mod_small((ra << 16) | (v & 0xFFFFu), ma, ia);
+            rb = mod_small((rb << 16) | (v & 0xFFFFu), mb, ib);
+        }
+        int ca = 0;
+        if (ma > 1) {
+            if (ra == 0) {
+                // m divides N: no chain in base A.  N is no base-2 pseudoprime
+                // unless 2^(N-1) = 1 mod m (m prime, N - 1 taken mod m - 1)
+                const uint32_t e = ma - 1, ie = inv32_of(e);
+                uint32_t r = 0;
+                for (int w = (int)limbs - 1; w >= 0; w--) {
+                    const uint32_t v = s_n[g][w];
+                    r = mod_small((r << 16) | (v >> 16), e, ie);
+                    r = mod_small((r << 16) | (v & 0xFFFFu), e, ie);
+                }
+                r = r ? r - 1 : e - 1;
+                atomicOr(&s_f[g], pow_small(2, r, ma, ia) == 1 ? kFlagOther * 4u : kFlagComposite * 4u);
+            } else {
+                // -1 / (N (A/m))
+                const uint32_t d = mod_small(ra * p.am[t], ma, ia);
+                ca = -balance(pow_small(d, ma - 2, ma, ia), ma);
+            }
+        }
+        num_a[at] = __float2half_rn((float)ca);
+        // n = N (B/m)^-1 / A;  start xi = ((B/m)^-1 - q n) A
+        const uint32_t gb = p.gb[t], ab = p.ab[t];
+        const uint32_t nb = mod_small(mod_small(rb * gb, mb, ib) * ainv, mb, ib);
+        num_b[at] = __float2half_rn((float)balance(nb, mb));
+        const uint32_t qm = (uint32_t)((uint64_t)s_q[g] % mb);
+        const uint32_t d = mod_small(gb + mb - mod_small(qm * nb, mb, ib), mb, ib);
+        state[at] = __float2half_rn((float)balance(mod_small(d * ab, mb, ib), mb));
+    }
+    __syncthreads();
+    if (t < kSetupNumbers && first + t < n_items) {
+        // one prime factor that rules N out is enough
+        const uint32_t f = s_f[t];
+        flag[first + t] = f & kFlagComposite * 4u ? kFlagComposite : f & kFlagOther * 4u ? kFlagOther : f;
+        quot[first + t] = s_q[t];
+    }
+}
+
+// ---------------------------------------------------------------------------
+// the chain of squarings
+
+__device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t n) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(n) : "memory");
+}
+
+// Wait for the barrier's completion of the given parity; gives up after about
+// a second (gone: the caller stops waiting altogether).
+__device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, bool &gone) {
+    if (gone) return;
+    uint32_t ok = 0;
+    for (uint32_t i = 0; i < (1u << 20); i++) {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (ok) return;
+    }
+    gone = true;
+}
+
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ void tmem_ld8(uint32_t (&r)[8], uint32_t addr) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(addr));
+}
+__device__ __forceinline__ void tmem_ld4(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr));
+}
+__device__ __forceinline__ void tmem_ld1(uint32_t &r, uint32_t addr) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(r) : "r"(addr));
+}
+__device__ __forceinline__ void tmem_st4(uint32_t addr, const uint32_t (&r)[4]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(r[0]), "r"(r[1]),
+                 "r"(r[2]), "r"(r[3])
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+
+// Two f32 in one register pair, an operation on both per instruction.
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 pack2(float a, float b) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ f2 pack2u(uint32_t a, uint32_t b) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(a), "r"(b));
+    return r;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+    f2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint32_t to_half2(f2 a) {
+    float x, y;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a));
+    uint32_t r;
+    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(y), "f"(x));
+    return r;
+}
+__device__ __forceinline__ f2 from_half2(uint32_t h) {
+    const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&h));
+    return pack2(f.x, f.y);
+}
+__device__ __forceinline__ uint32_t hmul2(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+
+// T mod m, balanced: T - m rint(T / m)
+__device__ __forceinline__ f2 red2(f2 t, f2 neg_m, f2 inv_m, f2 magic, f2 neg_magic) {
+    const f2 q = add2(fma2(t, inv_m, magic), neg_magic);
+    return fma2(q, neg_m, t);
+}
+// (lo + hi) mod m, hi a multiple of 64 up to 2^30: the quotient from the rounded
+// sum, the remainder's two parts exact
+__device__ __forceinline__ f2 red_sum2(f2 lo, f2 hi, f2 neg_m, f2 inv_m, f2 magic, f2 neg_magic) {
+    const f2 q = add2(fma2(add2(lo, hi), inv_m, magic), neg_magic);
+    return add2(fma2(q, neg_m, hi), lo);
+}
+
+struct ChainArgs {
+    const uint4 *matrices;   // [cta of the pair][product][chunk]
+    const uint4 *num_a, *num_b;
+    const uint4 *state;      // start
+    uint4 *dumps;            // the last kRnsDumps values, the last first
+    const uint32_t *nums;
+    const unsigned long long *count;
+    uint64_t max_items, dump_stride;  // in uint4
+    unsigned long long *error;
+    uint32_t limbs, steps;
+};
+
+template <uint32_t N>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+    chain_kernel(const __grid_constant__ RnsConst kc, const __grid_constant__ ChainArgs a) {
+    constexpr uint32_t K = kSlots * N;
+    constexpr uint32_t kBlocks = (N + 1) / 2;  // of 64 slots, the last of 32 for odd N
+    constexpr uint32_t kBuffers = 2;           // of 128 accumulator columns
+    constexpr uint32_t kCols = K + 128 * kBuffers <= 256 ? 256 : 512;
+    static_assert(K + 128 * kBuffers <= kCols, "TMEM");
+    extern __shared__ __align__(128) uint8_t smem[];
+    __shared__ uint32_t s_tmem;
+    __shared__ __align__(8) uint64_t s_done[N], s_free[kBuffers], s_full[kBuffers], s_end;
+
+    const uint64_t n_items = a.count ? min((uint64_t)*a.count, a.max_items) : a.max_items;
+    const uint32_t pair = blockIdx.x / 2, rank = blockIdx.x & 1;
+    if ((uint64_t)pair * kRnsTile >= n_items) return;  // both CTAs of the pair
+
+    const uint32_t warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x / 32, 0);
+    const uint32_t lane = threadIdx.x & 31;
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&s_tmem)),
+                     "r"(kCols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
+    }
+    if (threadIdx.x == 0) {
+        for (uint32_t i = 0; i < N; i++) mbar_init(smem_addr(&s_done[i]), 2 * kWarps);
+        for (uint32_t i = 0; i < kBuffers; i++) mbar_init(smem_addr(&s_full[i]), 1), mbar_init(smem_addr(&s_free[i]), 2 * kWarps);
+        mbar_init(smem_addr(&s_end), 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    {
+        const uint4 *src = a.matrices + (uint64_t)rank * (2 * K * K / 8);
+        uint4 *dst = reinterpret_cast<uint4 *>(smem);
+        for (uint32_t i = threadIdx.x; i < 2 * K * K / 8; i += kThreads) dst[i] = src[i];
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the tensor cores read it
+    fence_before();
+    __syncthreads();
+    cluster_sync();
+    fence_after();
+    const uint32_t tmem = s_tmem;
+    constexpr uint32_t kX1 = 0, kX2 = K / 2, kAcc = K;
+    bool gone = false;
+
+    if (warp < kWarps) {
+        const uint32_t wg = warp / 4;                           // its 8 slots of each chunk
+        const uint32_t lanes = tmem + ((32 * (warp % 4)) << 16);  // its TMEM lanes
+        const uint32_t row = 32 * (warp % 4) + lane;
+        const uint64_t tile = (uint64_t)pair * 2 + rank;
+        const uint64_t at0 = (tile * N * 4 + wg) * 128 + row;  // + 512 per chunk
+        const uint64_t number = tile * 128 + row;
+        const uint32_t *n_limbs = a.nums + (number < n_items ? number : 0) * a.limbs;
+        uint32_t done0, free0;  // the leader's barriers
+        asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(done0) : "r"(smem_addr(&s_done[0])));
+        asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(free0) : "r"(smem_addr(&s_free[0])));
+        auto arrive = [&](uint32_t bar) {
+            fence_before();
+            __syncwarp();
+            if (lane == 0) asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+        };
+        for (uint32_t c = 0; c < N; c++) {
+            const uint4 v = a.state[at0 + 512 * c];
+            const uint32_t x[4] = {v.x, v.y, v.z, v.w};
+            tmem_st4(lanes + kX2 + 16 * c + 4 * wg, x);
+            tmem_wait_st();
+            arrive(done0 + 8 * c);
+        }
+        const f2 magic = pack2(kMagic, kMagic), neg_magic = pack2(-kMagic, -kMagic);
+        uint32_t seq = 0;  // blocks seen
+        uint32_t word = 0;
+        const auto load = [&](const uint4 *p, uint32_t c, uint32_t (&w)[4]) {
+            const uint4 v = __ldg(p + at0 + 512 * c);
+            w[0] = v.x, w[1] = v.y, w[2] = v.z, w[3] = v.w;
+        };
+        // One product's sums to the residues of the next: blocks of two chunks (8 slots each
+        // per thread), the numbers' constants loaded a block ahead.
+        const auto product = [&](const uint4 *nums, const uint4 *next, uint32_t (&cw)[2][4], uint32_t x_at,
+                                 auto &&first, auto &&residues) {
+#pragma unroll 1
+            for (uint32_t b = 0; b < kBlocks; b++, seq++) {
+                const bool two = 2 * b + 1 < N;
+                const uint32_t acc = lanes + kAcc + 128 * (seq & 1) + 8 * wg, hi_at = two ? 64 : 32;
+                mbar_wait(smem_addr(&s_full[seq & 1]), (seq >> 1) & 1, gone);
+                fence_after();
+                uint32_t lo[2][8], hi[2][8], x[2][4];
+                tmem_ld8(lo[0], acc);
+                tmem_ld8(hi[0], acc + hi_at);
+                if (two) {
+                    tmem_ld8(lo[1], acc + 32);
+                    tmem_ld8(hi[1], acc + hi_at + 32);
+                }
+                if (b == 0) first(acc - 8 * wg);
+                tmem_wait_ld();
+                arrive(free0 + 8 * (seq & 1));
+                residues(2 * b, lo[0], hi[0], cw[0], x[0]);
+                tmem_st4(lanes + x_at + 32 * b + 4 * wg, x[0]);
+                // the next block's constants, or the next product's first
+                const uint4 *from = b + 1 < kBlocks ? nums : next;
+                const uint32_t at = b + 1 < kBlocks ? 2 * b + 2 : 0;
+                load(from, at, cw[0]);
+                if (two) residues(2 * b + 1, lo[1], hi[1], cw[1], x[1]);
+                tmem_wait_st();
+                arrive(done0 + 16 * b);
+                if (two) tmem_st4(lanes + x_at + 32 * b + 16 + 4 * wg, x[1]);
+                if (at + 1 < N) load(from, at + 1, cw[1]);
+                if (two) {
+                    tmem_wait_st();
+                    arrive(done0 + 16 * b + 8);
+                }
+            }
+        };
+        uint32_t cw[2][4];
+        load(a.num_a, 0, cw[0]);
+        if (N > 1) load(a.num_a, 1, cw[1]);
+#pragma unroll 1
+        for (uint32_t step = 0; step < a.steps; step++) {
+            // the doubling that the last step's exponent bit asked for, squared
+            uint32_t four = 0x3C003C00u;  // 1, 1
+            if (step > 0) {
+                const uint32_t at = a.steps - step + 1;  // bit of N: bit steps - step of (N - 1)/2
+                if (step == 1 || (at & 31) == 31) word = n_limbs[at >> 5];
+                if ((word >> (at & 31)) & 1) four = 0x44004400u;  // 4, 4
+            }
+            // sums of xi over B -> x in A -> xi in A
+            f2 rank2 = 0;
+            uint32_t rk = 0;
+            product(
+                a.num_a, a.num_b, cw, kX1, [&](uint32_t column) { tmem_ld1(rk, column); },
+                [&](uint32_t c, const uint32_t (&lo)[8], const uint32_t (&hi)[8], const uint32_t (&w)[4],
+                    uint32_t (&x)[4]) {
+                    if (c == 0) {
+                        const float f = __fadd_rn(__fmaf_rn(__uint_as_float(rk), 1.0f / 4096.0f, kMagic), -kMagic);
+                        rank2 = pack2(f, f);
+                    }
+                    const SlotPair *sp = kc.a + (16 * c + 4 * wg);
+#pragma unroll
+                    for (uint32_t j = 0; j < 4; j++) {
+                        const f2 nm = pack2(sp[j].neg_m[0], sp[j].neg_m[1]), im = pack2(sp[j].inv_m[0], sp[j].inv_m[1]);
+                        const f2 l = fma2(rank2, pack2(sp[j].c[0], sp[j].c[1]), pack2u(lo[2 * j], lo[2 * j + 1]));
+                        const f2 r = red_sum2(l, pack2u(hi[2 * j], hi[2 * j + 1]), nm, im, magic, neg_magic);
+                        const f2 u = red2(mul2(r, r), nm, im, magic, neg_magic);
+                        const f2 v = mul2(u, from_half2(hmul2(w[j], four)));
+                        x[j] = to_half2(red2(v, nm, im, magic, neg_magic));
+                    }
+                });
+            // sums of xi over A -> q in B -> xi in B
+            const bool dump = step + kRnsDumps >= a.steps;
+            uint4 *const to = a.dumps + (a.steps - 1 - step) * a.dump_stride + at0;
+            product(
+                a.num_b, a.num_a, cw, kX2, [](uint32_t) {},
+                [&](uint32_t c, const uint32_t (&lo)[8], const uint32_t (&hi)[8], const uint32_t (&w)[4],
+                    uint32_t (&x)[4]) {
+                    uint32_t old[4];
+                    tmem_ld4(old, lanes + kX2 + 16 * c + 4 * wg);
+                    tmem_wait_ld();
+                    const SlotPair *sp = kc.b + (16 * c + 4 * wg);
+#pragma unroll
+                    for (uint32_t j = 0; j < 4; j++) {
+                        const f2 nm = pack2(sp[j].neg_m[0], sp[j].neg_m[1]), im = pack2(sp[j].inv_m[0], sp[j].inv_m[1]);
+                        const f2 r = red_sum2(pack2u(lo[2 * j], lo[2 * j + 1]), pack2u(hi[2 * j], hi[2 * j + 1]), nm, im,
+                                              magic, neg_magic);
+                        const f2 t = mul2(from_half2(hmul2(old[j], four)), from_half2(old[j]));
+                        const f2 u = red2(t, nm, im, magic, neg_magic);
+                        const f2 v = fma2(r, from_half2(w[j]), mul2(u, pack2(sp[j].c[0], sp[j].c[1])));
+                        x[j] = to_half2(red2(v, nm, im, magic, neg_magic));
+                    }
+                    if (dump) to[512 * c] = make_uint4(x[0], x[1], x[2], x[3]);
+                });
+        }
+    } else if (rank == 0 && lane == 0) {
+        // f16 operands, f32 sums, both K-major, M = 256
+        constexpr uint32_t kInstr = (1u << 4) | ((256 / 16) << 24);
+        const uint32_t base = smem_addr(smem);
+        auto multiply = [&](uint32_t d, uint32_t x, uint32_t b, uint32_t kk) {
+            const uint32_t slots = 2 * b + 1 < N ? 64 : 32;  // N = twice that
+            // 8 x 8 pieces of 128 bytes, unswizzled: slots 128 bytes apart, k a row of them
+            const uint32_t row = slots / 8 * 128;
+            const uint32_t from = base + (x == tmem + kX1 ? 2 * K * K : 0) + b * (64 * K * 2) + kk * 2 * row;
+            const uint64_t desc = (uint64_t)((from & 0x3FFFF) >> 4) | ((uint64_t)(row / 16) << 16) |
+                                  ((uint64_t)(128 / 16) << 32) | (1ull << 46);
+            asm volatile(
+                "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
+                "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d),
+                "r"(x + 8 * kk), "l"(desc), "r"(kInstr | (slots * 2 / 8) << 17), "r"(kk)
+                : "memory");
+        };
+        uint32_t seq = 0;
+        for (uint32_t ph = 0; ph < 2 * a.steps; ph++) {
+            const uint32_t x = tmem + (ph & 1 ? kX1 : kX2);
+            for (uint32_t b = 0; b < kBlocks; b++, seq++) {
+                const uint32_t d = tmem + kAcc + 128 * (seq & 1);
+                // the buffer's last sums have been read
+                if (seq >= kBuffers) {
+                    mbar_wait(smem_addr(&s_free[seq & 1]), (seq / kBuffers - 1) & 1, gone);
+                    fence_after();
+                }
+                if (b == 0) {  // slice by slice, as the residues appear
+                    for (uint32_t i = 0; i < N; i++) {
+                        mbar_wait(smem_addr(&s_done[i]), ph & 1, gone);
+                        fence_after();
+                        multiply(d, x, b, 2 * i);
+                        multiply(d, x, b, 2 * i + 1);
+                    }
+                } else {
+                    for (uint32_t kk = 0; kk < 2 * N; kk++) multiply(d, x, b, kk);
+                }
+                asm volatile(
+                    "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::
+                        "r"(smem_addr(&s_full[seq & 1])),
+                    "h"((uint16_t)3)
+                    : "memory");
+            }
+        }
+    }
+    if (gone) {
+        atomicExch(a.error, 1ull);
+        if (warp == kWarps) {  // products still in flight end before TMEM is given back
+            asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                             smem_addr(&s_end))
+                         : "memory");
+            bool late = false;
+            mbar_wait(smem_addr(&s_end), 0, late);
+        }
+    }
+    fence_before();
+    __syncthreads();
+    cluster_sync();
+    fence_after();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols));
+}
+
+// ---------------------------------------------------------------------------
+// verdicts: a warp per number.  The value after the last squarings (f times, f
+// its exponent bit's doubling) is +-1 exactly when f x -+ (A mod N) is t N for
+// one small t, in every modulus of B (their product is above the difference's
+// range): f xi/A -+ ((B/m)^-1 - q n) = t n mod m.
+__global__ void verdict_kernel(const __grid_constant__ RnsSlots p, uint32_t chunks, uint32_t steps, uint32_t t_max,
+                               uint32_t limbs, const unsigned long long *count, uint64_t max_items,
+                               const __half *__restrict__ num_b, const __half *__restrict__ dumps, uint64_t dump_stride,
+                               const uint32_t *__restrict__ nums, const long long *__restrict__ quot,
+                               const uint32_t *__restrict__ flag, uint8_t *__restrict__ result,
+                               uint32_t *__restrict__ list, unsigned long long *__restrict__ listed) {
+    const uint64_t n_items = count ? min((uint64_t)*count, max_items) : max_items;
+    const uint64_t i = (uint64_t)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
+    if (i >= n_items) return;
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t f = flag[i];
+    const uint32_t *n = nums + i * limbs;
+    if (f == kFlagRun) {
+        uint32_t s = 0;  // trailing zeros of N - 1
+        for (uint32_t w = 0; w < limbs; w++) {
+            const uint32_t v = n[w] - (w == 0);
+            if (v) {
+                s = 32 * w + (uint32_t)__ffs(v) - 1;
+                break;
+            }
+        }
+        const uint32_t k = kSlots * chunks;
+        const long long q = quot[i];
+        const uint32_t last = min(min(kRnsDumps, s), steps);
+        f = kFlagOther;
+        bool prime = false;
+        for (uint32_t d = 0; d < last && f == kFlagOther; d++) {
+            const int twice = (int)((n[(d + 1) >> 5] >> ((d + 1) & 31)) & 1) + 1;
+            int sign = 1;
+            bool have = true, ok = false;
+            for (; sign >= -1 && !ok && have; sign -= 2) {
+                int t = 0;
+                ok = true;
+                for (uint32_t base = 0; base < k && ok; base += 32) {
+                    const uint32_t j = base + lane;
+                    const int m = (int)p.mb[j];
+                    const uint64_t at = slot_at(chunks, i, j);
+                    const int xi = (int)__half2float(dumps[d * dump_stride + at]), nb = (int)__half2float(num_b[at]);
+                    const int ainv = (int)inverse_small(p.ab[j], (uint32_t)m);
+                    const int one = ((int)p.gb[j] - (int)(q % m) * nb) % m;
+                    int lhs = (twice * xi % m * ainv - sign * one) % m;
+                    if (lhs < 0) lhs += m;
+                    const uint32_t nn = (uint32_t)(nb < 0 ? nb + m : nb);
+                    if (base == 0) {  // t from the first prime modulus that N is a unit of
+                        const uint32_t units = __ballot_sync(0xFFFFFFFFu, nn != 0 && j < p.b_primes);
+                        have = units != 0;
+                        const uint32_t inv = inv32_of((uint32_t)m);
+                        const int w = balance(
+                            mod_small((uint32_t)lhs * pow_small(nn, (uint32_t)m - 2, (uint32_t)m, inv), (uint32_t)m, inv),
+                            (uint32_t)m);
+                        t = __shfl_sync(0xFFFFFFFFu, w, have ? __ffs(units) - 1 : 0);
+                        ok = have && (uint32_t)abs(t) <= t_max;
+                    }
+                    ok = __all_sync(0xFFFFFFFFu, (lhs - t * (int)nn) % m == 0) && ok;
+                }
+            }
+            if (!have) break;                                     // N shares a factor with them all
+            if (!ok) f = kFlagRun;                                // neither: composite
+            else if (sign == -3) f = kFlagRun, prime = true;      // -1 on the way
+            else if (d + 1 == s) f = kFlagRun, prime = true;      // 1 from the start
+        }
+        if (f == kFlagRun && lane == 0) result[i] = prime;
+    } else if (f == kFlagComposite && lane == 0) {
+        result[i] = 0;
+    }
+    if (f == kFlagOther && lane == 0) list[atomicAdd(listed, 1ull)] = (uint32_t)i;
+}
+
+template <uint32_t N>
+cudaError_t launch_chain(const RnsPlan &p, const ChainArgs &a, uint64_t tiles, cudaStream_t s) {
+    // at least half of the SM's shared memory: a second CTA would wait for TMEM
+    // columns, and two pairs could each hold what the other waits for
+    constexpr uint32_t matrices = 2 * (kSlots * N) * (kSlots * N) * 2;
+    constexpr uint32_t bytes = matrices > 118 * 1024 ? matrices : 118 * 1024;
+    cudaError_t e = cudaFuncSetAttribute(chain_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess) return e;
+    chain_kernel<N><<<(unsigned)(2 * tiles), kThreads, bytes, s>>>(p.k, a);
+    return cudaGetLastError();
+}
+
+template <typename T>
+T *at(void *work, size_t off) {
+    return reinterpret_cast<T *>((char *)work + off);
+}
+
+}  // namespace
+
+uint32_t rns_chunks(uint32_t bits) {
+    for (uint32_t n = 1; n <= kRnsMaxChunks; n++)
+        if ((double)bits + 1e-6 <= moduli_of(n).bits) return n;
+    return 0;
+}
+
+RnsLayout rns_layout(uint32_t bits, uint32_t limbs, uint64_t max_items) {
+    RnsLayout l{};
+    l.chunks = rns_chunks(bits);
+    l.limbs = limbs;
+    l.tiles = (max_items + kRnsTile - 1) / kRnsTile;
+    const size_t k = kSlots * l.chunks, numbers = l.tiles * kRnsTile;
+    size_t off = 0;
+    auto take = [&](size_t bytes) {
+        const size_t o = off;
+        off += (bytes + 255) & ~(size_t)255;
+        return o;
+    };
+    l.matrices = take(2 * 2 * k * k * 2);
+    l.num_a = take(numbers * k * 2);
+    l.num_b = take(numbers * k * 2);
+    l.state = take(numbers * k * 2);
+    l.dumps = take(kRnsDumps * numbers * k * 2);
+    l.nums = take(numbers * limbs * 4);
+    l.quot = take(numbers * 8);
+    l.flag = take(numbers * 4);
+    l.list = take(numbers * 4);
+    l.counters = take(16);
+    l.total = off;
+    return l;
+}
+
+cudaError_t rns_begin(const RnsLayout &l, uint32_t bits, void *work, cudaStream_t s) {
+    const RnsPlan &p = plan_of(l.chunks, bits);
+    const uint32_t k = kSlots * l.chunks;
+    matrix_kernel<<<(2 * k * k + 255) / 256, 256, 0, s>>>(p.s, l.chunks, at<__half>(work, l.matrices));
+    const cudaError_t e = cudaGetLastError();
+    return e != cudaSuccess ? e : cudaMemsetAsync(at<char>(work, l.counters), 0, 16, s);
+}
+
+cudaError_t rns_test(const RnsLayout &l, uint32_t bits, void *work, const uint32_t *bases, const PrpItem *items,
+                     const unsigned long long *count, uint64_t max_items, uint8_t *result, cudaStream_t s) {
+    if (max_items == 0) return cudaSuccess;
+    const RnsPlan &p = plan_of(l.chunks, bits);
+    const uint32_t k = kSlots * l.chunks;
+    const uint64_t tiles = (max_items + kRnsTile - 1) / kRnsTile, numbers = l.tiles * kRnsTile;
+    const uint32_t steps = bits - 1;
+    cudaError_t e = cudaMemsetAsync(at<char>(work, l.counters), 0, 8, s);
+    if (e != cudaSuccess) return e;
+    setup_kernel<<<(unsigned)(tiles * (kRnsTile / kSetupNumbers)), k, 0, s>>>(
+        p.s, l.chunks, bits, p.a_mant, p.a_exp, l.limbs, bases, items, count, max_items, at<__half>(work, l.num_a),
+        at<__half>(work, l.num_b), at<__half>(work, l.state), at<uint32_t>(work, l.nums), at<long long>(work, l.quot),
+        at<uint32_t>(work, l.flag));
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    const ChainArgs a{at<uint4>(work, l.matrices), at<uint4>(work, l.num_a), at<uint4>(work, l.num_b),
+                      at<uint4>(work, l.state),    at<uint4>(work, l.dumps), at<uint32_t>(work, l.nums),
+                      count,                       max_items,                numbers * k / 8,
+                      at<unsigned long long>(work, l.counters) + 1,          l.limbs,
+                      steps};
+    switch (l.chunks) {
+        case 1: e = launch_chain<1>(p, a, tiles, s); break;
+        case 2: e = launch_chain<2>(p, a, tiles, s); break;
+        case 3: e = launch_chain<3>(p, a, tiles, s); break;
+        case 4: e = launch_chain<4>(p, a, tiles, s); break;
+        case 5: e = launch_chain<5>(p, a, tiles, s); break;
+        case 6: e = launch_chain<6>(p, a, tiles, s); break;
+        case 7: e = launch_chain<7>(p, a, tiles, s); break;
+        default: return cudaErrorInvalidValue;
+    }
+    if (e != cudaSuccess) return e;
+    verdict_kernel<<<(unsigned)((max_items + 3) / 4), 128, 0, s>>>(
+        p.s, l.chunks, steps, p.t_max, l.limbs, count, max_items, at<__half>(work, l.num_b), at<__half>(work, l.dumps),
+        numbers * k, at<uint32_t>(work, l.nums), at<long long>(work, l.quot), at<uint32_t>(work, l.flag), result,
+        at<uint32_t>(work, l.list), at<unsigned long long>(work, l.counters));
+    return cudaGetLastError();
+}
+
+}  // namespace pg

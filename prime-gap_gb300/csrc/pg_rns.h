@@ -1,0 +1,48 @@
+// Base-2 strong probable-prime tests of many numbers of one size on the tensor
+// cores (pg_rns.cu): residue number system, Montgomery reduction with both base
+// extensions as matrix products shared by every number.
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+namespace pg {
+
+constexpr uint32_t kRnsMaxChunks = 7;   // 32 residue slots each
+constexpr uint32_t kRnsDumps = 8;       // last values kept for the strong test's verdict
+constexpr uint32_t kRnsTile = 256;      // numbers per pair of CTAs
+
+struct PrpItem {
+    uint32_t row;  // row of the base numbers
+    int32_t x;     // N = base[row] + x
+};
+
+// Chunks of residue slots that numbers below 2^bits take; 0: too wide.
+uint32_t rns_chunks(uint32_t bits);
+
+// Device workspace of a call over at most max_items numbers.
+struct RnsLayout {
+    uint32_t chunks, limbs;
+    uint64_t tiles;  // of kRnsTile numbers
+    size_t matrices, num_a, num_b, state, dumps, nums, quot, flag, list, counters, total;
+};
+RnsLayout rns_layout(uint32_t bits, uint32_t limbs, uint64_t max_items);
+
+// Tests items[0 .. min(*count, max_items)) (count == nullptr: max_items) and
+// writes result; numbers that this form does not decide (their number at
+// rns_fallback_count, their places at rns_fallback_list, their limbs at
+// rns_numbers) are left for the caller.
+cudaError_t rns_begin(const RnsLayout &l, uint32_t bits, void *work, cudaStream_t s);
+cudaError_t rns_test(const RnsLayout &l, uint32_t bits, void *work, const uint32_t *bases, const PrpItem *items,
+                     const unsigned long long *count, uint64_t max_items, uint8_t *result, cudaStream_t s);
+inline const unsigned long long *rns_fallback_count(const RnsLayout &l, void *work) {
+    return (const unsigned long long *)((char *)work + l.counters);
+}
+inline const uint32_t *rns_fallback_list(const RnsLayout &l, void *work) {
+    return (const uint32_t *)((char *)work + l.list);
+}
+// Set by a wait that gave up.
+inline const unsigned long long *rns_error(const RnsLayout &l, void *work) {
+    return (const unsigned long long *)((char *)work + l.counters) + 1;
+}
+
+}  // namespace pg

@@ -1,0 +1,67 @@
+"""The tensor-core probable-prime tests (residue number system) against the
+oracle's strong test, at the sizes where they can go wrong: the widths where the
+number of residue slots changes, counts around a tile of 128 and a pair of 256
+numbers, and numbers that leave the common path."""
+from __future__ import annotations
+
+import random
+
+import pytest
+
+import prp_oracle as po
+
+pytestmark = pytest.mark.gpu
+
+SMALL = [p for p in range(3, 4096) if all(p % q for q in range(2, int(p**0.5) + 1))]
+
+
+def _numbers(rng, bits, count):
+    return [rng.getrandbits(bits - 1) | (1 << (bits - 1)) | 1 for _ in range(count)]
+
+
+# the last widths of one to seven chunks of 32 slots and the ones after them
+@pytest.mark.parametrize("bits", [252, 253, 367, 368, 741, 742, 1107, 1108, 1465, 1466, 1812, 1813, 2146, 2147,
+                                  2461, 2462])
+def test_rns_widths(sieve, bits):
+    rng = random.Random(bits)
+    nums = _numbers(rng, bits, 20) + [(1 << bits) - 1, (1 << (bits - 1)) + 1]
+    nums += _numbers(rng, bits - 19, 3) + _numbers(rng, bits - 21, 3) + _numbers(rng, 100, 2)
+    if bits <= 800:  # primes
+        for i in range(12):
+            while not po.strong_prp2(nums[i]):
+                nums[i] += 2
+    assert sieve.prp_test(nums) == [po.strong_prp2(n) for n in nums]
+
+
+@pytest.mark.parametrize("count", [1, 31, 127, 128, 129, 255, 256, 257, 1300])
+def test_rns_counts(sieve, count):
+    rng = random.Random(count)
+    prime = rng.getrandbits(300) | (1 << 300) | 1
+    while not po.strong_prp2(prime):
+        prime += 2
+    nums = _numbers(rng, 301, count)
+    for i in range(0, count, 7):
+        nums[i] = prime
+    assert sieve.prp_test(nums) == [po.strong_prp2(n) for n in nums]
+
+
+@pytest.mark.parametrize("p", [137, 151, 359, 1069])
+def test_rns_pseudoprimes_and_near_misses(sieve, p):
+    """(4^p + 1)/5 passes the strong test (2^(2p) = -1), (4^p - 1)/3 only
+    Fermat's (2^p is another root of 1); multiples of the residue system's own
+    primes; long runs of zeros in N - 1."""
+    strong, fermat = (4**p + 1) // 5, (4**p - 1) // 3
+    bits = 2 * p - 2
+    assert po.strong_prp2(strong) and not po.strong_prp2(fermat) and pow(2, fermat - 1, fermat) == 1
+    rng = random.Random(p)
+    nums = [strong, fermat]
+    nums += [q * (rng.getrandbits(bits - 12) | 1 << (bits - 12) | 1) for q in rng.sample(SMALL[-300:], 12)]
+    for t in (2, 5, 9, 10, 40, bits // 2):
+        nums.append((_numbers(rng, bits - t, 1)[0] << t) + 1)
+    if bits < 800:  # primes that are 1 modulo a high power of two: many square roots on the way
+        for t in (3, 4, 6, 8, 11):
+            k = rng.getrandbits(bits - t) | 1 << (bits - t - 1)
+            while not po.strong_prp2((k << t) + 1):
+                k += 1
+            nums.append((k << t) + 1)
+    assert sieve.prp_test(nums) == [po.strong_prp2(n) for n in nums]
