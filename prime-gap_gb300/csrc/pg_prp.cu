@@ -431,20 +431,24 @@ __global__ void centers_kernel(const uint32_t *__restrict__ k, uint32_t nk, cons
     }
 }
 
-struct GapRow {
-    uint32_t side;        // 0: previous prime, 1: next prime, 2: done
-    uint32_t idx;         // next unknown to test on this side
-    uint32_t past;        // 1 while this side searches past the sieve length
-    uint32_t past_x;      // next distance to scan past the sieve length
+// One side of one m: the search for the nearest probable prime.  Both sides of
+// an m are searched at once unless the next side may be skipped.
+struct GapSearch {
+    uint32_t state;      // kWaiting (for the previous side), kActive, kDone
+    uint32_t idx;        // next unknown to test
+    uint32_t past;       // 1 past the sieve length
+    uint32_t past_x;     // next distance there
     uint32_t item_base, item_cnt;
-    uint32_t skip_below;  // next side skipped when prev_p < skip_below (0: never)
-    uint32_t center_odd;  // parity of m*K
 };
+enum { kWaiting, kActive, kDone };
 
 struct GapLists {
     const uint64_t *start;
     const uint32_t *n_prev, *n_next, *dist;
 };
+
+// Distances past the sieve length that are coprime to K, a bit each from sl + 1.
+constexpr uint32_t kPastBits = 1u << 17;
 
 __device__ __forceinline__ bool coprime_to_k(uint32_t x, const uint32_t *kp, uint32_t nkp) {
     for (uint32_t i = 0; i < nkp; i++)
@@ -452,75 +456,124 @@ __device__ __forceinline__ bool coprime_to_k(uint32_t x, const uint32_t *kp, uin
     return true;
 }
 
-// Candidates of this round: up to spec per active row, nearest first; past
-// the sieve length, the next spec distances that keep N odd and coprime to K.
-__global__ void select_kernel(GapRow *rows_st, uint64_t rows, GapLists ls, uint32_t spec, const uint32_t *kp,
-                              uint32_t nkp, uint32_t x_limit, PrpItem *items, uint64_t max_items,
-                              unsigned long long *n_items, unsigned long long *errors) {
-    const uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= rows) return;
-    GapRow st = rows_st[r];
-    st.item_cnt = 0;
-    if (st.side < 2) {
-        const int32_t sign = st.side == 0 ? -1 : 1;
-        if (!st.past) {
-            const uint32_t nlist = st.side == 0 ? ls.n_prev[r] : ls.n_next[r];
-            const uint32_t *lst = ls.dist + ls.start[r] + (st.side == 0 ? 0u : ls.n_prev[r]);
-            uint32_t cnt = min(spec, nlist - st.idx);
-            const uint64_t base = atomicAdd(n_items, (unsigned long long)cnt);
-            if (base + cnt > max_items) {  // the host sizes rounds so that this never happens
-                atomicAdd(errors, 1ull);
-                st.side = 2;
-                cnt = 0;
-            }
-            for (uint32_t j = 0; j < cnt; j++) items[base + j] = PrpItem{(uint32_t)r, sign * (int32_t)lst[st.idx + j]};
-            st.item_base = (uint32_t)base;
-            st.item_cnt = cnt;
-        } else {
-            const uint64_t base = atomicAdd(n_items, (unsigned long long)spec);
-            uint32_t x = st.past_x, cnt = 0;
-            if (base + spec > max_items) {
-                atomicAdd(errors, 1ull);
-                st.side = 2;
-                rows_st[r] = st;
-                return;
-            }
-            // N = m*K +- x odd: x of the other parity than m*K
-            if ((x & 1u) == st.center_odd) x++;
-            while (cnt < spec && x < x_limit) {
-                if (coprime_to_k(x, kp, nkp)) items[base + cnt++] = PrpItem{(uint32_t)r, sign * (int32_t)x};
-                x += 2;
-            }
-            if (cnt < spec) {
-                atomicAdd(errors, 1ull);  // no prime within the scan limit: report, stop the row
-                st.side = 2;
-                // the reserved slots left over get a harmless item (N = m*K)
-                for (uint32_t j = cnt; j < spec; j++) items[base + j] = PrpItem{(uint32_t)r, 0};
-            }
-            st.item_base = (uint32_t)base;
-            st.item_cnt = cnt;
-            st.past_x = x;
-        }
-    }
-    rows_st[r] = st;
+__global__ void past_kernel(const uint32_t *kp, uint32_t nkp, uint32_t sl, uint32_t *__restrict__ bits) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= kPastBits) return;
+    const uint32_t w = __ballot_sync(0xFFFFFFFFu, coprime_to_k(sl + 1 + i, kp, nkp));
+    if ((i & 31) == 0) bits[i >> 5] = w;
 }
 
-__global__ void resolve_kernel(GapRow *rows_st, uint64_t rows, GapLists ls, const PrpItem *items,
-                               const uint8_t *result, uint32_t sl, pgs_gap_result *out,
-                               unsigned long long *active) {
-    const uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= rows) return;
-    GapRow st = rows_st[r];
-    if (st.side >= 2 || st.item_cnt == 0) return;
-    int first = -1;
-    for (uint32_t j = 0; j < st.item_cnt; j++)
-        if (result[st.item_base + j]) {
-            first = (int)j;
-            break;
+// A round's candidates, nearest first: spec for each active search and one more
+// for the first `extra` that ask; past the sieve length, the next distances
+// that keep N odd and coprime to K.  A warp per search.
+__global__ void select_kernel(GapSearch *searches, uint64_t rows, GapLists ls, const uint32_t *centers, uint32_t n,
+                              uint32_t spec, uint32_t extra, const uint32_t *kp, uint32_t nkp,
+                              const uint32_t *__restrict__ past_bits, uint32_t sl, uint32_t x_limit, PrpItem *items,
+                              uint64_t max_items, unsigned long long *n_items, unsigned long long *asked,
+                              unsigned long long *errors) {
+    const uint64_t e = (uint64_t)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
+    if (e >= 2 * rows) return;
+    const uint32_t lane = threadIdx.x & 31;
+    GapSearch st = searches[e];
+    if (st.state != kActive) return;
+    const uint64_t r = e >> 1;
+    const bool next = e & 1;
+    const int32_t sign = next ? 1 : -1;
+    const uint32_t center_odd = centers[r * n] & 1u;
+    uint32_t want = spec;
+    if (extra) {
+        uint32_t more = 0;
+        if (lane == 0) more = atomicAdd(asked, 1ull) < extra;
+        want += __shfl_sync(0xFFFFFFFFu, more, 0);
+    }
+    const uint32_t nlist = next ? ls.n_next[r] : ls.n_prev[r];
+    if (!st.past) want = min(want, nlist - st.idx);
+    unsigned long long base = 0;
+    if (lane == 0 && want) base = atomicAdd(n_items, (unsigned long long)want);
+    base = __shfl_sync(0xFFFFFFFFu, base, 0);
+    if (base + want > max_items) {  // the host sizes rounds so that this never happens
+        if (lane == 0) atomicAdd(errors, 1ull);
+        return;
+    }
+    uint32_t cnt = want;
+    if (!st.past) {
+        const uint32_t *lst = ls.dist + ls.start[r] + (next ? ls.n_prev[r] : 0u) + st.idx;
+        for (uint32_t j = lane; j < want; j += 32) items[base + j] = PrpItem{(uint32_t)r, sign * (int32_t)lst[j]};
+    } else {
+        cnt = 0;
+        uint32_t x = st.past_x;
+        while (cnt < want && x < x_limit) {
+            // 1024 distances, 32 a lane (32 past the bitmap, one a lane): those
+            // coprime to K, not before x, of the other parity than m*K
+            const uint32_t at = x - (sl + 1);
+            const bool table = at < kPastBits;
+            uint32_t from, word;
+            if (table) {
+                const uint32_t w = (at >> 5) + lane;
+                from = sl + 1 + 32 * w;
+                word = w < kPastBits / 32 ? past_bits[w] : 0u;
+                if (lane == 0) word &= 0xFFFFFFFFu << (at & 31);
+                word &= ((from & 1u) == center_odd) ? 0xAAAAAAAAu : 0x55555555u;
+            } else {
+                from = x + lane;
+                word = from < x_limit && (from & 1u) != center_odd && coprime_to_k(from, kp, nkp);
+            }
+            const uint32_t mine = __popc(word);
+            uint32_t before = mine;
+            for (uint32_t o = 1; o < 32; o <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, before, o);
+                if (lane >= o) before += v;
+            }
+            const uint32_t all = __shfl_sync(0xFFFFFFFFu, before, 31);
+            before -= mine;
+            uint32_t k = cnt + before, last = 0;
+            while (word && k < want) {
+                const uint32_t bit = (uint32_t)__ffs(word) - 1;
+                word &= word - 1;
+                last = from + bit;
+                items[base + k++] = PrpItem{(uint32_t)r, sign * (int32_t)last};
+            }
+            if (cnt + all >= want) {
+                x = __reduce_max_sync(0xFFFFFFFFu, last) + 1;
+                cnt = want;
+            } else {
+                cnt += all;
+                x = table ? min(sl + 1 + kPastBits, sl + 1 + 32 * (at >> 5) + 1024u) : x + 32;
+            }
         }
-    pgs_gap_result o = out[r];
-    const uint32_t nlist = st.side == 0 ? ls.n_prev[r] : ls.n_next[r];
-    if (first < 0) {
+        if (cnt < want) {
+            // no prime within the scan limit: report, stop the search; the slots
+            // left over get a harmless odd number
+            if (lane == 0) atomicAdd(errors, 1ull);
+            for (uint32_t j = cnt + lane; j < want; j += 32) items[base + j] = PrpItem{(uint32_t)r, 1 + (int32_t)center_odd};
+            st.state = kDone;
+        }
+        st.past_x = x;
+    }
+    st.item_base = (uint32_t)base;
+    st.item_cnt = cnt;
+    if (lane == 0) searches[e] = st;
+}
+
+// The round's results: a warp per search finds its first probable prime.
+__global__ void resolve_kernel(GapSearch *searches, uint64_t rows, GapLists ls, const uint32_t *skip_below,
+                               const PrpItem *items, const uint8_t *result, uint32_t sl, pgs_gap_result *out,
+                               unsigned long long *active, unsigned long long *found) {
+    const uint64_t e = (uint64_t)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
+    if (e >= 2 * rows) return;
+    const uint32_t lane = threadIdx.x & 31;
+    GapSearch st = searches[e];
+    if (st.state != kActive || st.item_cnt == 0) return;
+    uint32_t first = 0xFFFFFFFFu;
+    for (uint32_t j = 0; j < st.item_cnt && first == 0xFFFFFFFFu; j += 32) {
+        const uint32_t hit = __ballot_sync(0xFFFFFFFFu, j + lane < st.item_cnt && result[st.item_base + j + lane]);
+        if (hit) first = j + (uint32_t)__ffs(hit) - 1;
+    }
+    if (lane) return;
+    const uint64_t r = e >> 1;
+    const bool next = e & 1;
+    const uint32_t nlist = next ? ls.n_next[r] : ls.n_prev[r];
+    if (first == 0xFFFFFFFFu) {
         if (!st.past) {
             st.idx += st.item_cnt;
             if (st.idx >= nlist) st.past = 1, st.past_x = sl + 1;
@@ -528,44 +581,41 @@ __global__ void resolve_kernel(GapRow *rows_st, uint64_t rows, GapLists ls, cons
     } else {
         const int32_t xs = items[st.item_base + first].x;
         const uint32_t x = (uint32_t)(xs < 0 ? -xs : xs);
-        const uint32_t tests = st.past ? nlist : st.idx + (uint32_t)first + 1u;
-        if (st.side == 0) {
-            o.prev_p = (int32_t)x;
-            o.p_tests = tests;
-            o.flags |= st.past ? 1u : 0u;
-            if (x < st.skip_below) {
-                st.side = 2;
-                o.flags |= 4u;
-            } else {
-                st.side = 1;
-                st.idx = 0;
-                st.past = ls.n_next[r] == 0 ? 1u : 0u;
-                st.past_x = sl + 1;
+        const uint32_t tests = st.past ? nlist : st.idx + first + 1u;
+        pgs_gap_result *o = out + r;
+        st.state = kDone;
+        bool more = false;
+        if (!next) {
+            o->prev_p = (int32_t)x;
+            o->p_tests = tests;
+            if (st.past) atomicOr(&o->flags, 1u);
+            if (skip_below) {
+                if (x < skip_below[r]) atomicOr(&o->flags, 4u);
+                else more = true, searches[e + 1].state = kActive;
             }
         } else {
-            o.next_p = (int32_t)x;
-            o.n_tests = tests;
-            o.flags |= st.past ? 2u : 0u;
-            st.side = 2;
+            o->next_p = (int32_t)x;
+            o->n_tests = tests;
+            if (st.past) atomicOr(&o->flags, 2u);
         }
-        out[r] = o;
+        if (!more) atomicAdd(active, ~0ull);  // one fewer
+        atomicAdd(found, 1ull);
     }
-    rows_st[r] = st;
-    if (st.side < 2) atomicAdd(active, 1ull);
+    st.item_cnt = 0;
+    searches[e] = st;
 }
 
-__global__ void gap_init_kernel(GapRow *rows_st, uint64_t rows, GapLists ls, const uint32_t *skip_below,
-                                const uint32_t *centers, uint32_t n, uint32_t sl, pgs_gap_result *out) {
-    const uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= rows) return;
-    GapRow st{};
-    st.side = 0;
-    st.past = ls.n_prev[r] == 0 ? 1u : 0u;
+__global__ void gap_init_kernel(GapSearch *searches, uint64_t rows, GapLists ls, bool may_skip, uint32_t sl,
+                                pgs_gap_result *out) {
+    const uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= 2 * rows) return;
+    const uint64_t r = e >> 1;
+    GapSearch st{};
+    st.state = (e & 1) && may_skip ? kWaiting : kActive;
+    st.past = ((e & 1) ? ls.n_next[r] : ls.n_prev[r]) == 0 ? 1u : 0u;
     st.past_x = sl + 1;
-    st.skip_below = skip_below ? skip_below[r] : 0u;
-    st.center_odd = centers[r * n] & 1u;
-    rows_st[r] = st;
-    out[r] = pgs_gap_result{};
+    searches[e] = st;
+    if (!(e & 1)) out[r] = pgs_gap_result{};
 }
 
 }  // namespace
@@ -632,8 +682,8 @@ uint32_t skip_threshold(double klog, uint64_t m, float min_merit) {
     return hi;
 }
 
-constexpr uint64_t kRoundTarget = 1ull << 15;  // candidates per round when few rows remain
-constexpr uint32_t kMaxSpec = 64;
+constexpr uint64_t kRoundTarget = 1ull << 15;  // candidates per round of the limb form
+constexpr uint32_t kMaxSpec = 512;             // candidates per search and round
 constexpr uint32_t kPastScanSpan = 1u << 24;   // distances scanned past SL before giving up
 
 }  // namespace
@@ -734,8 +784,13 @@ int prp_gaps_core(pgs_ctx *ctx, const pgs_gap_params *prm, uint64_t rows, const 
         ctx->err = "pgs_prp_gaps: m*K above 4092 bits";
         return PGS_EINVAL;
     }
-    const uint64_t max_items = std::max<uint64_t>(rows, kRoundTarget + kMaxSpec);
-    const pg::PrpPlan plan = pg::prp_plan(bits, max_items);
+    // A round is a wave of the residue form (its time is the same for fewer), or
+    // enough to fill the GPU with the limb form
+    const bool may_skip = prm->one_side_skip != 0;
+    const uint64_t searches = 2 * rows;
+    const uint64_t limb_round = std::max<uint64_t>(searches, kRoundTarget);
+    const pg::PrpPlan plan = pg::prp_plan(bits, std::max<uint64_t>(limb_round, pg::rns_wave(bits, true)));
+    const uint64_t max_items = plan.rns ? pg::rns_wave(bits, true) : limb_round;
     const uint32_t n = 8u * (uint32_t)plan.L;
     std::vector<uint32_t> skip(rows, 0u);
     if (prm->one_side_skip) {
@@ -743,8 +798,8 @@ int prp_gaps_core(pgs_ctx *ctx, const pgs_gap_params *prm, uint64_t rows, const 
         for (uint64_t r = 0; r < rows; r++) skip[r] = skip_threshold(klog, h_m[r], prm->min_merit);
     }
     const cudaStream_t s = ctx->stream;
-    DevBuf d_k, d_kp, d_skip, d_centers, d_state, d_items, d_res, d_out, d_ctr, d_work;
-    DevBuf *bufs[] = {&d_k, &d_kp, &d_skip, &d_centers, &d_state, &d_items, &d_res, &d_out, &d_ctr, &d_work};
+    DevBuf d_k, d_kp, d_skip, d_centers, d_state, d_items, d_res, d_out, d_ctr, d_work, d_past;
+    DevBuf *bufs[] = {&d_past, &d_k, &d_kp, &d_skip, &d_centers, &d_state, &d_items, &d_res, &d_out, &d_ctr, &d_work};
     for (DevBuf *b : bufs) b->pool = &ctx->dpool;
     auto cleanup = [&] {
         cudaStreamSynchronize(s);
@@ -752,13 +807,14 @@ int prp_gaps_core(pgs_ctx *ctx, const pgs_gap_params *prm, uint64_t rows, const 
     };
     cudaError_t e = upload(d_k, k, s);
     if (e == cudaSuccess) e = upload(d_kp, kprimes, s);
-    if (e == cudaSuccess) e = upload(d_skip, skip, s);
+    if (e == cudaSuccess && may_skip) e = upload(d_skip, skip, s);
+    if (e == cudaSuccess) e = d_past.ensure(pg::kPastBits / 8);
     if (e == cudaSuccess) e = d_centers.ensure(rows * n * 4ull);
-    if (e == cudaSuccess) e = d_state.ensure(rows * sizeof(pg::GapRow));
+    if (e == cudaSuccess) e = d_state.ensure(searches * sizeof(pg::GapSearch));
     if (e == cudaSuccess) e = d_items.ensure(max_items * sizeof(pg::PrpItem));
     if (e == cudaSuccess) e = d_res.ensure(max_items);
     if (e == cudaSuccess) e = d_out.ensure(rows * sizeof(pgs_gap_result));
-    if (e == cudaSuccess) e = d_ctr.ensure(32);
+    if (e == cudaSuccess) e = d_ctr.ensure(40);
     if (e == cudaSuccess) e = d_work.ensure(plan.work_bytes());
     if (e == cudaSuccess) e = pg::prp_begin(plan, d_work.p, s);
     if (e != cudaSuccess) {
@@ -766,46 +822,62 @@ int prp_gaps_core(pgs_ctx *ctx, const pgs_gap_params *prm, uint64_t rows, const 
         return fail(ctx, e, "pgs_prp_gaps setup");
     }
     const pg::GapLists ls{d_start, d_np, d_nn, d_dist};
-    unsigned long long *ctr = d_ctr.as<unsigned long long>();  // items, active, errors
-    const unsigned rb = (unsigned)((rows + 255) / 256);
+    unsigned long long *ctr = d_ctr.as<unsigned long long>();  // items, asked, active, errors, found
+    const uint32_t *skip_below = may_skip ? d_skip.as<uint32_t>() : nullptr;
+    const unsigned rb = (unsigned)((rows + 255) / 256), sb = (unsigned)((searches + 7) / 8);
     pg::centers_kernel<<<rb, 256, 0, s>>>(d_k.as<uint32_t>(), (uint32_t)k.size(), d_m, rows, n,
                                           d_centers.as<uint32_t>());
-    pg::gap_init_kernel<<<rb, 256, 0, s>>>(d_state.as<pg::GapRow>(), rows, ls, d_skip.as<uint32_t>(),
-                                           d_centers.as<uint32_t>(), n, prm->sieve_length,
-                                           d_out.as<pgs_gap_result>());
-    e = cudaMemsetAsync(ctr, 0, 32, s);
-    uint64_t active = rows, rounds = 0, launched = 0;
-    uint64_t host_ctr[3] = {0, 0, 0};
+    pg::past_kernel<<<pg::kPastBits / 256, 256, 0, s>>>(d_kp.as<uint32_t>(), (uint32_t)kprimes.size(),
+                                                        prm->sieve_length, d_past.as<uint32_t>());
+    pg::gap_init_kernel<<<(unsigned)((searches + 255) / 256), 256, 0, s>>>(
+        d_state.as<pg::GapSearch>(), rows, ls, may_skip, prm->sieve_length, d_out.as<pgs_gap_result>());
+    uint64_t active = may_skip ? rows : searches, rounds = 0, launched = 0;
+    unsigned long long host_ctr[5] = {0, 0, active, 0, 0};
+    e = cudaMemcpyAsync(ctr, host_ctr, 40, cudaMemcpyHostToDevice, s);
     const uint32_t x_limit = prm->sieve_length + kPastScanSpan;
     while (e == cudaSuccess && active > 0) {
-        const uint32_t spec =
-            (uint32_t)std::min<uint64_t>(kMaxSpec, std::max<uint64_t>(1, kRoundTarget / active));
-        e = cudaMemsetAsync(ctr, 0, 16, s);  // items, active
+        uint64_t quota = limb_round;
+        if (plan.rns) {
+            // A wave of several tiles per pair tests 1.2-1.4 times as many a second as
+            // a single one, but what lies past a search's end is wasted: with s
+            // candidates per search in the single wave and a chance p of each (found
+            // so far / tested), it resolves more a second where s p is above 0.55
+            // (2136 bits, p 1/39, 21.5 and 13.5 ms: 31.4 against 30.4 searches a ms at
+            // s p = 0.43, 26.0 against 27.3 at 0.66).
+            const uint64_t one = pg::rns_wave(bits, false);
+            const double chance = launched ? (double)host_ctr[4] / (double)launched : 1.0 / 32;
+            quota = (double)one * chance < 0.55 * (double)active ? max_items : one;
+        }
+        quota = std::min(quota, active * kMaxSpec);
+        const uint32_t spec = (uint32_t)(quota / active), extra = (uint32_t)(quota % active);
+        e = cudaMemsetAsync(ctr, 0, 16, s);  // items, asked
         if (e) break;
-        pg::select_kernel<<<rb, 256, 0, s>>>(d_state.as<pg::GapRow>(), rows, ls, spec, d_kp.as<uint32_t>(),
-                                             (uint32_t)kprimes.size(), x_limit, d_items.as<pg::PrpItem>(),
-                                             max_items, ctr, ctr + 2);
-        const uint64_t bound = std::min<uint64_t>(max_items, active * spec);
-        e = pg::prp_launch(plan, d_work.p, d_centers.as<uint32_t>(), d_items.as<pg::PrpItem>(), ctr, bound,
+        pg::select_kernel<<<sb, 256, 0, s>>>(d_state.as<pg::GapSearch>(), rows, ls, d_centers.as<uint32_t>(), n, spec,
+                                             extra, d_kp.as<uint32_t>(), (uint32_t)kprimes.size(),
+                                             d_past.as<uint32_t>(), prm->sieve_length, x_limit,
+                                             d_items.as<pg::PrpItem>(), quota, ctr, ctr + 1, ctr + 3);
+        e = pg::prp_launch(plan, d_work.p, d_centers.as<uint32_t>(), d_items.as<pg::PrpItem>(), ctr, quota,
                            d_res.as<uint8_t>(), s);
         if (e) break;
         unsigned long long gave_up = 0;
         e = pg::prp_error(plan, d_work.p, &gave_up, s);
         if (e) break;
-        pg::resolve_kernel<<<rb, 256, 0, s>>>(d_state.as<pg::GapRow>(), rows, ls, d_items.as<pg::PrpItem>(),
-                                              d_res.as<uint8_t>(), prm->sieve_length, d_out.as<pgs_gap_result>(),
-                                              ctr + 1);
+        pg::resolve_kernel<<<sb, 256, 0, s>>>(d_state.as<pg::GapSearch>(), rows, ls, skip_below,
+                                              d_items.as<pg::PrpItem>(), d_res.as<uint8_t>(), prm->sieve_length,
+                                              d_out.as<pgs_gap_result>(), ctr + 2,
+                                              ctr + 4);
         e = cudaGetLastError();
-        if (e == cudaSuccess) e = cudaMemcpyAsync(host_ctr, ctr, 24, cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(host_ctr, ctr, 40, cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e) break;
+        if (host_ctr[3]) break;  // reported below
         if (gave_up) {
             cleanup();
             ctx->err = "pgs_prp_gaps: a wait on the device gave up";
             return PGS_ETIMEOUT;
         }
         launched += host_ctr[0];
-        active = host_ctr[1];
+        active = host_ctr[2];
         if (++rounds > (1u << 22)) {
             cleanup();
             ctx->err = "pgs_prp_gaps: no progress";
@@ -817,7 +889,7 @@ int prp_gaps_core(pgs_ctx *ctx, const pgs_gap_params *prm, uint64_t rows, const 
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     cleanup();
     if (e != cudaSuccess) return fail(ctx, e, "pgs_prp_gaps");
-    if (host_ctr[2]) {
+    if (host_ctr[3]) {
         ctx->err = "pgs_prp_gaps: a side found no probable prime within 2^24 past the sieve length";
         return PGS_EABORT;
     }

@@ -48,6 +48,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 namespace pg {
@@ -327,7 +328,7 @@ __global__ void setup_kernel(const __grid_constant__ RnsSlots p, uint32_t chunks
     __shared__ long long s_q[kSetupNumbers];
     __shared__ uint32_t s_f[kSetupNumbers];
     const uint64_t n_items = count ? min((uint64_t)*count, max_items) : max_items;
-    const uint64_t padded = (n_items + kRnsTile - 1) / kRnsTile * kRnsTile;
+    const uint64_t padded = ((n_items + kRnsTile - 1) / kRnsTile + kRnsGroup - 1) * kRnsTile;
     const uint64_t first = (uint64_t)blockIdx.x * kSetupNumbers;
     if (first >= padded) return;
     if (threadIdx.x < kSetupNumbers) {
@@ -473,7 +474,16 @@ __device__ __forceinline__ void tmem_st4(uint32_t addr, const uint32_t (&r)[4]) 
                  "r"(r[2]), "r"(r[3])
                  : "memory");
 }
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// ... and what has come is not read before
+__device__ __forceinline__ void tmem_wait_ld(uint32_t (&a)[8], uint32_t (&b)[8], uint32_t &c) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]), "+r"(a[7]),
+                   "+r"(b[0]), "+r"(b[1]), "+r"(b[2]), "+r"(b[3]), "+r"(b[4]), "+r"(b[5]), "+r"(b[6]), "+r"(b[7]),
+                   "+r"(c)::"memory");
+}
+__device__ __forceinline__ void tmem_wait_ld(uint32_t (&a)[4]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3])::"memory");
+}
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -532,6 +542,46 @@ __device__ __forceinline__ f2 red2(f2 t, f2 neg_m, f2 inv_m, f2 magic, f2 neg_ma
 __device__ __forceinline__ f2 red_sum2(f2 lo, f2 hi, f2 neg_m, f2 inv_m, f2 magic, f2 neg_magic) {
     const f2 q = add2(fma2(add2(lo, hi), inv_m, magic), neg_magic);
     return add2(fma2(q, neg_m, hi), lo);
+}
+
+// The sums of one chunk to residues, 8 slots of a lane.  w: the number's own
+// constants, four: 1 or 4 (the squared doubling) in both halves.
+struct Magic {
+    f2 plus, minus;
+};
+__device__ __forceinline__ void residues_a(const SlotPair *sp, const uint32_t (&lo)[8], const uint32_t (&hi)[8],
+                                           f2 rank2, const uint32_t (&w)[4], uint32_t four, const Magic &mg,
+                                           uint32_t (&x)[4]) {
+#pragma unroll
+    for (uint32_t j = 0; j < 4; j++) {
+        const f2 nm = pack2(sp[j].neg_m[0], sp[j].neg_m[1]), im = pack2(sp[j].inv_m[0], sp[j].inv_m[1]);
+        const f2 l = fma2(rank2, pack2(sp[j].c[0], sp[j].c[1]), pack2u(lo[2 * j], lo[2 * j + 1]));
+        const f2 r = red_sum2(l, pack2u(hi[2 * j], hi[2 * j + 1]), nm, im, mg.plus, mg.minus);
+        const f2 u = red2(mul2(r, r), nm, im, mg.plus, mg.minus);
+        const f2 v = mul2(u, from_half2(hmul2(w[j], four)));
+        x[j] = to_half2(red2(v, nm, im, mg.plus, mg.minus));
+    }
+}
+__device__ __forceinline__ void residues_b(const SlotPair *sp, const uint32_t (&lo)[8], const uint32_t (&hi)[8],
+                                           const uint32_t (&old)[4], const uint32_t (&w)[4], uint32_t four,
+                                           const Magic &mg, uint32_t (&x)[4]) {
+    const f2 four2 = from_half2(four);
+#pragma unroll
+    for (uint32_t j = 0; j < 4; j++) {
+        const f2 nm = pack2(sp[j].neg_m[0], sp[j].neg_m[1]), im = pack2(sp[j].inv_m[0], sp[j].inv_m[1]);
+        const f2 r = red_sum2(pack2u(lo[2 * j], lo[2 * j + 1]), pack2u(hi[2 * j], hi[2 * j + 1]), nm, im, mg.plus,
+                              mg.minus);
+        const f2 o = from_half2(old[j]);
+        const f2 t = mul2(mul2(o, o), four2);
+        const f2 u = red2(t, nm, im, mg.plus, mg.minus);
+        const f2 v = fma2(r, from_half2(w[j]), mul2(u, pack2(sp[j].c[0], sp[j].c[1])));
+        x[j] = to_half2(red2(v, nm, im, mg.plus, mg.minus));
+    }
+}
+// round(sum / 4096): the rank from its column
+__device__ __forceinline__ f2 rank_of(uint32_t sum) {
+    const float f = __fadd_rn(__fmaf_rn(__uint_as_float(sum), 1.0f / 4096.0f, kMagic), -kMagic);
+    return pack2(f, f);
 }
 
 struct ChainArgs {
@@ -613,7 +663,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             tmem_wait_st();
             arrive(done0 + 8 * c);
         }
-        const f2 magic = pack2(kMagic, kMagic), neg_magic = pack2(-kMagic, -kMagic);
+        const Magic mg{pack2(kMagic, kMagic), pack2(-kMagic, -kMagic)};
         uint32_t seq = 0;  // blocks seen
         uint32_t word = 0;
         const auto load = [&](const uint4 *p, uint32_t c, uint32_t (&w)[4]) {
@@ -623,7 +673,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         // One product's sums to the residues of the next: blocks of two chunks (8 slots each
         // per thread), the numbers' constants loaded a block ahead.
         const auto product = [&](const uint4 *nums, const uint4 *next, uint32_t (&cw)[2][4], uint32_t x_at,
-                                 auto &&first, auto &&residues) {
+                                 bool rank_too, auto &&residues) {
 #pragma unroll 1
             for (uint32_t b = 0; b < kBlocks; b++, seq++) {
                 const bool two = 2 * b + 1 < N;
@@ -637,16 +687,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                     tmem_ld8(lo[1], acc + 32);
                     tmem_ld8(hi[1], acc + hi_at + 32);
                 }
-                if (b == 0) first(acc - 8 * wg);
-                tmem_wait_ld();
+                uint32_t rk = 0;
+                if (b == 0 && rank_too) tmem_ld1(rk, acc - 8 * wg);
+                tmem_wait_ld(lo[0], hi[0], rk);
+                if (two) tmem_wait_ld(lo[1], hi[1], rk);
                 arrive(free0 + 8 * (seq & 1));
-                residues(2 * b, lo[0], hi[0], cw[0], x[0]);
+                residues(2 * b, lo[0], hi[0], rk, cw[0], x[0]);
                 tmem_st4(lanes + x_at + 32 * b + 4 * wg, x[0]);
                 // the next block's constants, or the next product's first
                 const uint4 *from = b + 1 < kBlocks ? nums : next;
                 const uint32_t at = b + 1 < kBlocks ? 2 * b + 2 : 0;
                 load(from, at, cw[0]);
-                if (two) residues(2 * b + 1, lo[1], hi[1], cw[1], x[1]);
+                if (two) residues(2 * b + 1, lo[1], hi[1], rk, cw[1], x[1]);
                 tmem_wait_st();
                 arrive(done0 + 16 * b);
                 if (two) tmem_st4(lanes + x_at + 32 * b + 16 + 4 * wg, x[1]);
@@ -671,47 +723,24 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             }
             // sums of xi over B -> x in A -> xi in A
             f2 rank2 = 0;
-            uint32_t rk = 0;
             product(
-                a.num_a, a.num_b, cw, kX1, [&](uint32_t column) { tmem_ld1(rk, column); },
-                [&](uint32_t c, const uint32_t (&lo)[8], const uint32_t (&hi)[8], const uint32_t (&w)[4],
+                a.num_a, a.num_b, cw, kX1, true,
+                [&](uint32_t c, const uint32_t (&lo)[8], const uint32_t (&hi)[8], uint32_t rk, const uint32_t (&w)[4],
                     uint32_t (&x)[4]) {
-                    if (c == 0) {
-                        const float f = __fadd_rn(__fmaf_rn(__uint_as_float(rk), 1.0f / 4096.0f, kMagic), -kMagic);
-                        rank2 = pack2(f, f);
-                    }
-                    const SlotPair *sp = kc.a + (16 * c + 4 * wg);
-#pragma unroll
-                    for (uint32_t j = 0; j < 4; j++) {
-                        const f2 nm = pack2(sp[j].neg_m[0], sp[j].neg_m[1]), im = pack2(sp[j].inv_m[0], sp[j].inv_m[1]);
-                        const f2 l = fma2(rank2, pack2(sp[j].c[0], sp[j].c[1]), pack2u(lo[2 * j], lo[2 * j + 1]));
-                        const f2 r = red_sum2(l, pack2u(hi[2 * j], hi[2 * j + 1]), nm, im, magic, neg_magic);
-                        const f2 u = red2(mul2(r, r), nm, im, magic, neg_magic);
-                        const f2 v = mul2(u, from_half2(hmul2(w[j], four)));
-                        x[j] = to_half2(red2(v, nm, im, magic, neg_magic));
-                    }
+                    if (c == 0) rank2 = rank_of(rk);
+                    residues_a(kc.a + (16 * c + 4 * wg), lo, hi, rank2, w, four, mg, x);
                 });
             // sums of xi over A -> q in B -> xi in B
             const bool dump = step + kRnsDumps >= a.steps;
             uint4 *const to = a.dumps + (a.steps - 1 - step) * a.dump_stride + at0;
             product(
-                a.num_b, a.num_a, cw, kX2, [](uint32_t) {},
-                [&](uint32_t c, const uint32_t (&lo)[8], const uint32_t (&hi)[8], const uint32_t (&w)[4],
+                a.num_b, a.num_a, cw, kX2, false,
+                [&](uint32_t c, const uint32_t (&lo)[8], const uint32_t (&hi)[8], uint32_t, const uint32_t (&w)[4],
                     uint32_t (&x)[4]) {
                     uint32_t old[4];
                     tmem_ld4(old, lanes + kX2 + 16 * c + 4 * wg);
-                    tmem_wait_ld();
-                    const SlotPair *sp = kc.b + (16 * c + 4 * wg);
-#pragma unroll
-                    for (uint32_t j = 0; j < 4; j++) {
-                        const f2 nm = pack2(sp[j].neg_m[0], sp[j].neg_m[1]), im = pack2(sp[j].inv_m[0], sp[j].inv_m[1]);
-                        const f2 r = red_sum2(pack2u(lo[2 * j], lo[2 * j + 1]), pack2u(hi[2 * j], hi[2 * j + 1]), nm, im,
-                                              magic, neg_magic);
-                        const f2 t = mul2(from_half2(hmul2(old[j], four)), from_half2(old[j]));
-                        const f2 u = red2(t, nm, im, magic, neg_magic);
-                        const f2 v = fma2(r, from_half2(w[j]), mul2(u, pack2(sp[j].c[0], sp[j].c[1])));
-                        x[j] = to_half2(red2(v, nm, im, magic, neg_magic));
-                    }
+                    tmem_wait_ld(old);
+                    residues_b(kc.b + (16 * c + 4 * wg), lo, hi, old, w, four, mg, x);
                     if (dump) to[512 * c] = make_uint4(x[0], x[1], x[2], x[3]);
                 });
         }
@@ -776,6 +805,244 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     fence_after();
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols));
+}
+
+// The same chain with T tiles of 256 numbers per pair, taken in turn: a tile's
+// two exchanges per squaring (residues written, product, sums ready: some 1300
+// cycles) pass while the other tiles' residues are computed.  A tile has one A
+// operand in TMEM: the next one replaces it when its product's last sums are in,
+// so a product's residues wait in registers; B's residues, needed again for the
+// next square, are kept in shared memory (what does not fit, in TMEM).
+// 38912 numbers of 2136 bits: 23.7 ms against 29.6 ms in two single waves (58368
+// of 712 bits: 4.9 against 6.2), the f32 pipe 68 % busy, the tensor cores 47 %.
+// Reading the next chunk's sums while a chunk's residues are computed changed
+// nothing (24.9 ms).
+template <uint32_t N, uint32_t T>
+struct TilesShape {
+    static constexpr uint32_t K = kSlots * N;
+    static constexpr uint32_t kMatrices = 2 * K * K * 2;
+    static constexpr uint32_t kChunk = 128 * 4 * 16;  // one tile's residues of one chunk, bytes
+    static constexpr uint32_t kRoom = (226 * 1024 - kMatrices) / (T * kChunk);
+    static constexpr uint32_t kOldShared = kRoom < N ? kRoom : N;  // chunks in shared memory
+    static constexpr uint32_t kShared = kMatrices + T * kOldShared * kChunk;
+    static constexpr uint32_t kAcc = T * K / 2, kOld = kAcc + 256;  // TMEM columns
+    static_assert(kOld + T * (N - kOldShared) * 16 <= 512, "TMEM");
+};
+
+template <uint32_t N, uint32_t T>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+    chain_tiles_kernel(const __grid_constant__ RnsConst kc, const __grid_constant__ ChainArgs a) {
+    using S = TilesShape<N, T>;
+    constexpr uint32_t K = S::K;
+    constexpr uint32_t kBlocks = (N + 1) / 2;  // of 64 slots, the last of 32 for odd N
+    constexpr uint32_t kBuffers = 2;           // of 128 accumulator columns
+    extern __shared__ __align__(128) uint8_t smem[];
+    __shared__ uint32_t s_tmem;
+    __shared__ __align__(8) uint64_t s_done[T], s_free[kBuffers], s_full[kBuffers], s_end;
+
+    const uint64_t n_items = a.count ? min((uint64_t)*a.count, a.max_items) : a.max_items;
+    const uint32_t pair = blockIdx.x / 2, rank = blockIdx.x & 1;
+    if ((uint64_t)pair * (T * kRnsTile) >= n_items) return;  // both CTAs of the pair
+
+    const uint32_t warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x / 32, 0);
+    const uint32_t lane = threadIdx.x & 31;
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&s_tmem)),
+                     "r"(512)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
+    }
+    if (threadIdx.x == 0) {
+        for (uint32_t i = 0; i < T; i++) mbar_init(smem_addr(&s_done[i]), 2 * kWarps);
+        for (uint32_t i = 0; i < kBuffers; i++)
+            mbar_init(smem_addr(&s_full[i]), 1), mbar_init(smem_addr(&s_free[i]), 2 * kWarps);
+        mbar_init(smem_addr(&s_end), 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    {
+        const uint4 *src = a.matrices + (uint64_t)rank * (2 * K * K / 8);
+        uint4 *dst = reinterpret_cast<uint4 *>(smem);
+        for (uint32_t i = threadIdx.x; i < 2 * K * K / 8; i += kThreads) dst[i] = src[i];
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the tensor cores read it
+    fence_before();
+    __syncthreads();
+    cluster_sync();
+    fence_after();
+    const uint32_t tmem = s_tmem;
+    bool gone = false;
+
+    if (warp < kWarps) {
+        const uint32_t wg = warp / 4;                           // its 8 slots of each chunk
+        const uint32_t lanes = tmem + ((32 * (warp % 4)) << 16);  // its TMEM lanes
+        const uint32_t row = 32 * (warp % 4) + lane;
+        const uint64_t tile0 = (uint64_t)pair * (2 * T) + rank;  // + 2 per tile
+        const uint64_t at0 = (tile0 * N * 4 + wg) * 128 + row;   // + 512 per chunk
+        constexpr uint32_t kTileStep = 2 * N * 512;
+        uint4 *const old_shared = reinterpret_cast<uint4 *>(smem + S::kMatrices) + wg * 128 + row;
+        uint32_t done0, free0;  // the leader's barriers
+        asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(done0) : "r"(smem_addr(&s_done[0])));
+        asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(free0) : "r"(smem_addr(&s_free[0])));
+        auto arrive = [&](uint32_t bar) {
+            fence_before();
+            __syncwarp();
+            if (lane == 0) asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+        };
+        auto keep = [&](uint32_t t, uint32_t c, const uint32_t (&x)[4]) {
+            if (c < S::kOldShared)
+                old_shared[(t * S::kOldShared + c) * 512] = make_uint4(x[0], x[1], x[2], x[3]);
+            else
+                tmem_st4(lanes + S::kOld + (t * (N - S::kOldShared) + c - S::kOldShared) * 16 + 4 * wg, x);
+        };
+        auto kept = [&](uint32_t t, uint32_t c, uint32_t (&x)[4]) {
+            if (c < S::kOldShared) {
+                const uint4 v = old_shared[(t * S::kOldShared + c) * 512];
+                x[0] = v.x, x[1] = v.y, x[2] = v.z, x[3] = v.w;
+            } else {
+                tmem_ld4(x, lanes + S::kOld + (t * (N - S::kOldShared) + c - S::kOldShared) * 16 + 4 * wg);
+                tmem_wait_ld(x);
+            }
+        };
+        for (uint32_t t = 0; t < T; t++) {
+            for (uint32_t c = 0; c < N; c++) {
+                const uint4 v = a.state[at0 + t * kTileStep + 512 * c];
+                const uint32_t x[4] = {v.x, v.y, v.z, v.w};
+                tmem_st4(lanes + t * (K / 2) + 16 * c + 4 * wg, x);
+                keep(t, c, x);
+            }
+            tmem_wait_st();
+            arrive(done0 + 8 * t);
+        }
+        const Magic mg{pack2(kMagic, kMagic), pack2(-kMagic, -kMagic)};
+        // a tile's limb that holds the exponent bit of a step
+        const auto limb = [&](uint32_t t, uint32_t step) {
+            const uint64_t number = (tile0 + 2 * t) * 128 + row;
+            return __ldg(a.nums + (number < n_items ? number : 0) * a.limbs + ((a.steps - step + 1) >> 5));
+        };
+        const auto load = [&](const uint4 *p, uint32_t t, uint32_t c, uint32_t (&w)[4]) {
+            const uint4 v = __ldg(p + at0 + t * kTileStep + 512 * c);
+            w[0] = v.x, w[1] = v.y, w[2] = v.z, w[3] = v.w;
+        };
+        uint32_t seq = 0;  // blocks seen
+        uint32_t cw[2][4], word = 0;
+        load(a.num_a, 0, 0, cw[0]);
+        if (N > 1) load(a.num_a, 0, 1, cw[1]);
+        // one tile's sums of one product to the A operand of its next; the constants and the
+        // limb of what comes after are loaded on the way
+        const auto product = [&](auto in_b, uint32_t step, uint32_t t) {
+            constexpr bool kB = decltype(in_b)::value;
+            const uint4 *const nums = kB ? a.num_b : a.num_a;
+            const bool last_tile = t + 1 == T;
+            const uint4 *const next = last_tile ? (kB ? a.num_a : a.num_b) : nums;
+            const uint32_t next_t = last_tile ? 0 : t + 1;
+            const uint32_t next_step = last_tile && kB && step + 1 < a.steps ? step + 1 : step;
+            const uint32_t bit = a.steps - step + 1;
+            const uint32_t four = step > 0 && ((word >> (bit & 31)) & 1) ? 0x44004400u : 0x3C003C00u;  // 4, 4 or 1, 1
+            word = limb(next_t, next_step);
+            const bool dump = kB && step + kRnsDumps >= a.steps;
+            f2 rank2 = 0;
+            uint32_t x[2 * kBlocks][4];
+#pragma unroll
+            for (uint32_t b = 0; b < kBlocks; b++) {
+                const bool two = 2 * b + 1 < N;
+                const uint32_t acc = lanes + S::kAcc + 128 * (seq & 1) + 8 * wg, hi_at = two ? 64 : 32;
+                mbar_wait(smem_addr(&s_full[seq & 1]), (seq >> 1) & 1, gone);
+                fence_after();
+                uint32_t lo[2][8], hi[2][8], rk = 0;
+                tmem_ld8(lo[0], acc);
+                tmem_ld8(hi[0], acc + hi_at);
+                if (two) {
+                    tmem_ld8(lo[1], acc + 32);
+                    tmem_ld8(hi[1], acc + hi_at + 32);
+                }
+                if (!kB && b == 0) tmem_ld1(rk, acc - 8 * wg);
+                tmem_wait_ld(lo[0], hi[0], rk);
+                if (two) tmem_wait_ld(lo[1], hi[1], rk);
+                arrive(free0 + 8 * (seq & 1));
+                seq++;
+                if (!kB && b == 0) rank2 = rank_of(rk);
+#pragma unroll
+                for (uint32_t h = 0; h < (two ? 2 : 1); h++) {
+                    const uint32_t c = 2 * b + h;
+                    if (kB) {
+                        uint32_t old[4];
+                        kept(t, c, old);
+                        residues_b(kc.b + (16 * c + 4 * wg), lo[h], hi[h], old, cw[h], four, mg, x[c]);
+                        keep(t, c, x[c]);
+                        if (dump)
+                            a.dumps[(a.steps - 1 - step) * a.dump_stride + at0 + t * kTileStep + 512 * c] =
+                                make_uint4(x[c][0], x[c][1], x[c][2], x[c][3]);
+                    } else {
+                        residues_a(kc.a + (16 * c + 4 * wg), lo[h], hi[h], rank2, cw[h], four, mg, x[c]);
+                    }
+                    const bool more = b + 1 < kBlocks;
+                    const uint32_t at = more ? 2 * b + 2 + h : h;
+                    if (at < N) load(more ? nums : next, more ? t : next_t, at, cw[h]);
+                    // odd N: the second chunk of what comes next, where this block has none
+                    if (!two && !more && N > 1) load(next, next_t, 1, cw[1]);
+                }
+            }
+            // the last block's sums are in: every product with the old operand is done
+#pragma unroll
+            for (uint32_t c = 0; c < N; c++) tmem_st4(lanes + t * (K / 2) + 16 * c + 4 * wg, x[c]);
+            tmem_wait_st();
+            arrive(done0 + 8 * t);
+        };
+#pragma unroll 1
+        for (uint32_t step = 0; step < a.steps; step++) {
+#pragma unroll 1
+            for (uint32_t t = 0; t < T; t++) product(std::false_type{}, step, t);
+#pragma unroll 1
+            for (uint32_t t = 0; t < T; t++) product(std::true_type{}, step, t);
+        }
+    } else if (rank == 0 && lane == 0) {
+        constexpr uint32_t kInstr = (1u << 4) | ((256 / 16) << 24);
+        const uint32_t base = smem_addr(smem);
+        uint32_t seq = 0;
+        for (uint32_t ph = 0; ph < 2 * a.steps; ph++) {
+            for (uint32_t t = 0; t < T; t++) {
+                const uint32_t x = tmem + t * (K / 2);
+                mbar_wait(smem_addr(&s_done[t]), ph & 1, gone);
+                for (uint32_t b = 0; b < kBlocks; b++, seq++) {
+                    const uint32_t d = tmem + S::kAcc + 128 * (seq & 1);
+                    const uint32_t slots = 2 * b + 1 < N ? 64 : 32, r = slots / 8 * 128;
+                    if (seq >= kBuffers) mbar_wait(smem_addr(&s_free[seq & 1]), (seq / kBuffers - 1) & 1, gone);
+                    fence_after();
+                    for (uint32_t kk = 0; kk < 2 * N; kk++) {
+                        const uint32_t from = base + (ph & 1 ? 2 * K * K : 0) + b * (64 * K * 2) + kk * 2 * r;
+                        const uint64_t desc = (uint64_t)((from & 0x3FFFF) >> 4) | ((uint64_t)(r / 16) << 16) |
+                                              ((uint64_t)(128 / 16) << 32) | (1ull << 46);
+                        asm volatile(
+                            "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
+                            "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d),
+                            "r"(x + 8 * kk), "l"(desc), "r"(kInstr | (slots * 2 / 8) << 17), "r"(kk)
+                            : "memory");
+                    }
+                    asm volatile(
+                        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::
+                            "r"(smem_addr(&s_full[seq & 1])),
+                        "h"((uint16_t)3)
+                        : "memory");
+                }
+            }
+        }
+    }
+    if (gone) {
+        atomicExch(a.error, 1ull);
+        if (warp == kWarps) {  // products still in flight end before TMEM is given back
+            asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                             smem_addr(&s_end))
+                         : "memory");
+            bool late = false;
+            mbar_wait(smem_addr(&s_end), 0, late);
+        }
+    }
+    fence_before();
+    __syncthreads();
+    cluster_sync();
+    fence_after();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
 }
 
 // ---------------------------------------------------------------------------
@@ -851,8 +1118,34 @@ __global__ void verdict_kernel(const __grid_constant__ RnsSlots p, uint32_t chun
     if (f == kFlagOther && lane == 0) list[atomicAdd(listed, 1ull)] = (uint32_t)i;
 }
 
+// Tiles per pair: enough that their residues take longer than one tile's exchange.
+constexpr uint32_t kTilesOf[kRnsMaxChunks + 1] = {0, 4, 3, 2, 2, 2, 2, 1};
+
+// Pairs of CTAs that run at once, one CTA per SM.
+uint64_t pairs_at_once() {
+    int device = 0, sms = 0;
+    if (cudaGetDevice(&device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms < 2)
+        return 76;
+    return (uint64_t)sms / 2;
+}
+
+
+template <uint32_t N, uint32_t T>
+cudaError_t launch_tiles(const RnsPlan &p, const ChainArgs &a, uint64_t tiles, cudaStream_t s) {
+    constexpr uint32_t least = 118 * 1024;  // one CTA per SM, as below
+    constexpr uint32_t bytes = TilesShape<N, T>::kShared > least ? TilesShape<N, T>::kShared : least;
+    cudaError_t e = cudaFuncSetAttribute(chain_tiles_kernel<N, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess) return e;
+    chain_tiles_kernel<N, T><<<(unsigned)(2 * ((tiles + T - 1) / T)), kThreads, bytes, s>>>(p.k, a);
+    return cudaGetLastError();
+}
+
 template <uint32_t N>
 cudaError_t launch_chain(const RnsPlan &p, const ChainArgs &a, uint64_t tiles, cudaStream_t s) {
+    if constexpr (N < 7) {
+        if (tiles > pairs_at_once()) return launch_tiles<N, kTilesOf[N]>(p, a, tiles, s);
+    }
     // at least half of the SM's shared memory: a second CTA would wait for TMEM
     // columns, and two pairs could each hold what the other waits for
     constexpr uint32_t matrices = 2 * (kSlots * N) * (kSlots * N) * 2;
@@ -876,11 +1169,15 @@ uint32_t rns_chunks(uint32_t bits) {
     return 0;
 }
 
+uint64_t rns_wave(uint32_t bits, bool full) {
+    return pairs_at_once() * kRnsTile * (full ? kTilesOf[rns_chunks(bits)] : 1);
+}
+
 RnsLayout rns_layout(uint32_t bits, uint32_t limbs, uint64_t max_items) {
     RnsLayout l{};
     l.chunks = rns_chunks(bits);
     l.limbs = limbs;
-    l.tiles = (max_items + kRnsTile - 1) / kRnsTile;
+    l.tiles = (max_items + kRnsTile - 1) / kRnsTile + kRnsGroup - 1;  // a last group's empty tiles
     const size_t k = kSlots * l.chunks, numbers = l.tiles * kRnsTile;
     size_t off = 0;
     auto take = [&](size_t bytes) {
@@ -919,7 +1216,7 @@ cudaError_t rns_test(const RnsLayout &l, uint32_t bits, void *work, const uint32
     const uint32_t steps = bits - 1;
     cudaError_t e = cudaMemsetAsync(at<char>(work, l.counters), 0, 8, s);
     if (e != cudaSuccess) return e;
-    setup_kernel<<<(unsigned)(tiles * (kRnsTile / kSetupNumbers)), k, 0, s>>>(
+    setup_kernel<<<(unsigned)((tiles + kRnsGroup - 1) * (kRnsTile / kSetupNumbers)), k, 0, s>>>(
         p.s, l.chunks, bits, p.a_mant, p.a_exp, l.limbs, bases, items, count, max_items, at<__half>(work, l.num_a),
         at<__half>(work, l.num_b), at<__half>(work, l.state), at<uint32_t>(work, l.nums), at<long long>(work, l.quot),
         at<uint32_t>(work, l.flag));

@@ -9,7 +9,8 @@ namespace pg {
 
 constexpr uint32_t kRnsMaxChunks = 7;   // 32 residue slots each
 constexpr uint32_t kRnsDumps = 8;       // last values kept for the strong test's verdict
-constexpr uint32_t kRnsTile = 256;      // numbers per pair of CTAs
+constexpr uint32_t kRnsTile = 256;      // numbers of a tile, half in each CTA of a pair
+constexpr uint32_t kRnsGroup = 4;       // most tiles that a pair takes in turn
 
 struct PrpItem {
     uint32_t row;  // row of the base numbers
@@ -18,6 +19,10 @@ struct PrpItem {
 
 // Chunks of residue slots that numbers below 2^bits take; 0: too wide.
 uint32_t rns_chunks(uint32_t bits);
+
+// Numbers that run at once in one wave, of single tiles or of full groups of
+// tiles (0 where rns_chunks is 0 and full is asked).
+uint64_t rns_wave(uint32_t bits, bool full);
 
 // Device workspace of a call over at most max_items numbers.
 struct RnsLayout {

@@ -65,3 +65,19 @@ def test_rns_pseudoprimes_and_near_misses(sieve, p):
                 k += 1
             nums.append((k << t) + 1)
     assert sieve.prp_test(nums) == [po.strong_prp2(n) for n in nums]
+
+
+@pytest.mark.parametrize("bits,count", [(301, 20480), (720, 20000), (1000, 19457), (1300, 39169), (1700, 19713),
+                                        (2100, 20100)])
+def test_rns_more_numbers_than_one_wave(sieve, bits, count):
+    """Several tiles per pair of CTAs: the same answers as a few numbers get, at
+    every place (the last group of tiles not full)."""
+    rng = random.Random(bits)
+    few = _numbers(rng, bits, 37)
+    if bits < 400:
+        while not po.strong_prp2(few[5]):
+            few[5] += 2
+    few += [(4**p + 1) // 5 for p in (bits // 2, bits // 2 - 1, bits // 2 + 1) if all(p % q for q in SMALL if q < p)]
+    want = [po.strong_prp2(n) for n in few]
+    got = sieve.prp_test([few[i % len(few)] for i in range(count)])
+    assert all(got[i] == want[i % len(few)] for i in range(count))
