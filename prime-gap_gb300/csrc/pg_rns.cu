@@ -56,7 +56,7 @@ namespace pg {
 namespace {
 
 constexpr uint32_t kSlots = 32;                        // residue slots per chunk
-constexpr uint32_t kMaxK = kSlots * kRnsMaxChunks;     // 224
+constexpr uint32_t kMaxK = kSlots * kRnsMaxChunks;     // 288
 constexpr uint32_t kWarps = 16;                        // warps that compute residues
 constexpr uint32_t kThreads = 32 * (kWarps + 1);       // and one that issues products
 constexpr float kMagic = 12582912.0f;                  // 1.5 2^23
@@ -146,8 +146,9 @@ RnsModuli make_moduli(uint32_t n) {
     for (uint32_t lead = 0; lead < 24; lead++) {
         RnsModuli m;
         size_t top = primes.size();
-        while (m.a.size() + 1 < k || m.b.size() + extra.size() < k) {
+        while (top > 0 && (m.a.size() + 1 < k || m.b.size() + extra.size() < k)) {
             const uint32_t q = primes[--top];
+            if (used[q]) continue;
             const bool b_full = m.b.size() + extra.size() >= k;
             (m.a.size() + 1 < k && (b_full || m.a.size() < m.b.size() + lead) ? m.a : m.b).push_back(q);
         }
@@ -155,6 +156,7 @@ RnsModuli make_moduli(uint32_t n) {
         m.b.insert(m.b.end(), extra.begin(), extra.end());
         const double c = coefficient(m.a.size());
         m.bits = std::fmin(a_capacity(log2_product(m.a), m.a.size()), log2_product(m.b) - 2 - std::log2(c));
+        m.b.resize(k, 1);  // slots left over: modulus 1, all zero
         if (m.bits > best.bits) best = m;
     }
     return best;
@@ -314,8 +316,37 @@ __device__ __forceinline__ uint64_t slot_at(uint32_t chunks, uint64_t number, ui
 
 enum { kFlagRun = 0, kFlagComposite = 1, kFlagOther = 2 };
 
+// Remainder below 2m of v < 2^29 by m, for chains that only need it small.
+__device__ __forceinline__ uint32_t mod_lazy(uint32_t v, uint32_t m, uint32_t inv32) {
+    return v - __umulhi(v, inv32) * m;
+}
+
+// Little-endian limbs mod m.
+__device__ __forceinline__ uint32_t limbs_mod(const uint32_t *n, uint32_t limbs, uint32_t m, uint32_t inv32) {
+    uint32_t r = 0;
+    for (int w = (int)limbs - 1; w >= 0; w--) {
+        const uint32_t v = n[w];
+        r = mod_lazy((r << 16) | (v >> 16), m, inv32);
+        r = mod_lazy((r << 16) | (v & 0xFFFFu), m, inv32);
+    }
+    return r >= m ? r - m : r;
+}
+
+// Whether n (top its highest limb that is not 0) is near enough to 2^bits for
+// its start, and floor(A / n) from its leading words.
+__device__ bool near_widest(const uint32_t *n, int top, uint32_t bits, double a_mant, int a_exp, long long &q) {
+    if (top < 3) return false;
+    const double v = ((double)n[top] * 4294967296.0 + (double)n[top - 1]) * 4294967296.0 + (double)n[top - 2];
+    if (log2(v) + 32.0 * (top - 2) <= (double)bits - 24.0) return false;
+    q = (long long)floor(ldexp(a_mant / v, a_exp - 32 * (top - 2)));
+    return true;
+}
+
 // Per number: its limbs, its constants in every slot, its start (the Montgomery
 // form of 1).  A block takes 8 numbers; a thread one slot of each base.
+// A prime m of base A that divides N leaves no inverse there.  N can still be a
+// pseudoprime only if 2^(N-1) = 1 mod m; then the chain runs mod N/m (the
+// exponent stays N's) and the verdict looks at both.
 // Bound by the remainders' Horner chains (two multiplies per 16 bits): about 2 %
 // of the chain's time.
 constexpr uint32_t kSetupNumbers = 8;
@@ -323,10 +354,13 @@ __global__ void setup_kernel(const __grid_constant__ RnsSlots p, uint32_t chunks
                              int a_exp, uint32_t limbs, const uint32_t *__restrict__ bases,
                              const PrpItem *__restrict__ items, const unsigned long long *count, uint64_t max_items,
                              __half *__restrict__ num_a, __half *__restrict__ num_b, __half *__restrict__ state,
-                             uint32_t *__restrict__ nums, long long *__restrict__ quot, uint32_t *__restrict__ flag) {
+                             uint32_t *__restrict__ nums, long long *__restrict__ quot, uint32_t *__restrict__ flag,
+                             uint32_t *__restrict__ factor) {
     __shared__ uint32_t s_n[kSetupNumbers][128];
     __shared__ long long s_q[kSetupNumbers];
     __shared__ uint32_t s_f[kSetupNumbers];
+    // primes of A that divide the number, the last of them, and whether one rules it out
+    __shared__ uint32_t s_divide[kSetupNumbers], s_by[kSetupNumbers], s_out[kSetupNumbers];
     const uint64_t n_items = count ? min((uint64_t)*count, max_items) : max_items;
     const uint64_t padded = ((n_items + kRnsTile - 1) / kRnsTile + kRnsGroup - 1) * kRnsTile;
     const uint64_t first = (uint64_t)blockIdx.x * kSetupNumbers;
@@ -350,62 +384,30 @@ __global__ void setup_kernel(const __grid_constant__ RnsSlots p, uint32_t chunks
                 dst[w] = lo;
                 if (lo) top = (int)w;
             }
-            // floor(A / N) from the leading words; N within 20 bits of the widest
-            f = kFlagOther;
-            if (top >= 3) {
-                const double n = ((double)s_n[g][top] * 4294967296.0 + (double)s_n[g][top - 1]) * 4294967296.0 +
-                                 (double)s_n[g][top - 2];
-                const double len = log2(n) + 32.0 * (top - 2);
-                if (len > (double)bits - 20.0) {
-                    q = (long long)floor(ldexp(a_mant / n, a_exp - 32 * (top - 2)));
-                    f = kFlagRun;
-                }
-            }
+            f = near_widest(s_n[g], top, bits, a_mant, a_exp, q) ? kFlagRun : kFlagOther;
         }
         s_q[g] = q;
         s_f[g] = f;
+        s_divide[g] = 0, s_by[g] = 1, s_out[g] = 0;
     }
     __syncthreads();
     const uint32_t t = threadIdx.x;
     const uint32_t ma = p.ma[t], mb = p.mb[t];
     const uint32_t ia = inv32_of(ma), ib = inv32_of(mb);
     const uint32_t ainv = inverse_small(p.ab[t], mb);
-    for (uint32_t g = 0; g < kSetupNumbers; g++) {
-        const uint64_t i = first + g;
-        const uint64_t at = slot_at(chunks, i, t);
-        if (s_f[g] != kFlagRun) {  // an all-zero lane
-            num_a[at] = __half(0.0f);
-            num_b[at] = __half(0.0f);
-            state[at] = __half(0.0f);
-            continue;
-        }
-        uint32_t ra = 0, rb = 0;
-        for (int w = (int)limbs - 1; w >= 0; w--) {
-            const uint32_t v = s_n[g][w];
-            ra = mod_small((ra << 16) | (v >> 16), ma, ia);
-            rb = mod_small((rb << 16) | (v >> 16), mb, ib);
-            ra = mod_small((ra << 16) | (v & 0xFFFFu), ma, ia);
-            rb = mod_small((rb << 16) | (v & 0xFFFFu), mb, ib);
-        }
+    const auto slots = [&](uint32_t g) {
+        const uint64_t at = slot_at(chunks, first + g, t);
+        const uint32_t ra = limbs_mod(s_n[g], limbs, ma, ia), rb = limbs_mod(s_n[g], limbs, mb, ib);
         int ca = 0;
-        if (ma > 1) {
-            if (ra == 0) {
-                // m divides N: no chain in base A.  N is no base-2 pseudoprime
-                // unless 2^(N-1) = 1 mod m (m prime, N - 1 taken mod m - 1)
-                const uint32_t e = ma - 1, ie = inv32_of(e);
-                uint32_t r = 0;
-                for (int w = (int)limbs - 1; w >= 0; w--) {
-                    const uint32_t v = s_n[g][w];
-                    r = mod_small((r << 16) | (v >> 16), e, ie);
-                    r = mod_small((r << 16) | (v & 0xFFFFu), e, ie);
-                }
-                r = r ? r - 1 : e - 1;
-                atomicOr(&s_f[g], pow_small(2, r, ma, ia) == 1 ? kFlagOther * 4u : kFlagComposite * 4u);
-            } else {
-                // -1 / (N (A/m))
-                const uint32_t d = mod_small(ra * p.am[t], ma, ia);
-                ca = -balance(pow_small(d, ma - 2, ma, ia), ma);
-            }
+        if (ma > 1 && ra == 0) {
+            uint32_t r = limbs_mod(s_n[g], limbs, ma - 1, inv32_of(ma - 1));
+            r = r ? r - 1 : ma - 2;
+            atomicAdd(&s_divide[g], 1u);
+            s_by[g] = ma;
+            if (pow_small(2, r, ma, ia) != 1) s_out[g] = 1;
+        } else if (ma > 1) {  // -1 / (N (A/m))
+            const uint32_t d = mod_small(ra * p.am[t], ma, ia);
+            ca = -balance(pow_small(d, ma - 2, ma, ia), ma);
         }
         num_a[at] = __float2half_rn((float)ca);
         // n = N (B/m)^-1 / A;  start xi = ((B/m)^-1 - q n) A
@@ -415,13 +417,44 @@ __global__ void setup_kernel(const __grid_constant__ RnsSlots p, uint32_t chunks
         const uint32_t qm = (uint32_t)((uint64_t)s_q[g] % mb);
         const uint32_t d = mod_small(gb + mb - mod_small(qm * nb, mb, ib), mb, ib);
         state[at] = __float2half_rn((float)balance(mod_small(d * ab, mb, ib), mb));
+    };
+    for (uint32_t g = 0; g < kSetupNumbers; g++) {
+        if (s_f[g] == kFlagRun) {
+            slots(g);
+        } else {  // an all-zero lane
+            const uint64_t at = slot_at(chunks, first + g, t);
+            num_a[at] = num_b[at] = state[at] = __half(0.0f);
+        }
     }
     __syncthreads();
+    for (uint32_t g = 0; g < kSetupNumbers; g++) {
+        if (s_f[g] != kFlagRun || s_divide[g] == 0 || s_out[g]) continue;  // the same for the whole block
+        const bool one = s_divide[g] == 1;
+        __syncthreads();
+        if (t == 0) {
+            uint64_t r = 0;
+            int top = -1;
+            for (int w = (int)limbs - 1; w >= 0; w--) {
+                r = r << 32 | s_n[g][w];
+                s_n[g][w] = (uint32_t)(r / s_by[g]);
+                if (top < 0 && s_n[g][w]) top = w;
+                r %= s_by[g];
+            }
+            s_divide[g] = 0;
+            s_f[g] = one && near_widest(s_n[g], top, bits, a_mant, a_exp, s_q[g]) ? kFlagRun : kFlagOther;
+        }
+        __syncthreads();
+        const uint32_t by = s_by[g];
+        if (s_f[g] == kFlagRun) slots(g);
+        __syncthreads();
+        if (t == 0 && s_divide[g]) s_f[g] = kFlagOther;  // another factor of A in N / m
+        if (t == 0) s_by[g] = by, s_out[g] = 0;
+        __syncthreads();
+    }
     if (t < kSetupNumbers && first + t < n_items) {
-        // one prime factor that rules N out is enough
-        const uint32_t f = s_f[t];
-        flag[first + t] = f & kFlagComposite * 4u ? kFlagComposite : f & kFlagOther * 4u ? kFlagOther : f;
+        flag[first + t] = s_out[t] ? kFlagComposite : s_f[t];
         quot[first + t] = s_q[t];
+        factor[first + t] = s_by[t];
     }
 }
 
@@ -596,17 +629,40 @@ struct ChainArgs {
     uint32_t limbs, steps;
 };
 
+// Up to seven chunks the matrices stay in shared memory and both A operands (of
+// the product under way and of the next) lie in TMEM in full.  Above, the
+// matrices' blocks go round a ring, copied from L2 ahead of each product (2838
+// bits: 14.8 us a step, 12.5 without the copies; 9001 numbers 43 ms where the limb
+// form takes 106), and the
+// chunks from the eighth on have one place in TMEM: their residues are written
+// when the product's last sums are in, and B's (needed again for the next square)
+// are kept in shared memory.
 template <uint32_t N>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+struct ChainShape {
+    static constexpr uint32_t K = kSlots * N;
+    static constexpr uint32_t kBlocks = (N + 1) / 2;          // of 64 slots, the last of 32 for odd N
+    static constexpr uint32_t kTwice = N < 7 ? N : 7;         // chunks with two places
+    static constexpr bool kRing = N > 7;
+    static constexpr uint32_t kWarpsAll = kWarps + (kRing ? 2 : 1);
+    static constexpr uint32_t kBlockBytes = 64 * K * 2;       // of one CTA
+    static constexpr uint32_t kKept = (N - kTwice) * 128 * 4 * 16;
+    static constexpr uint32_t kSlotsOfRing = kRing ? (226 * 1024 - kKept) / kBlockBytes : 1;
+    static constexpr uint32_t kShared = kRing ? kSlotsOfRing * kBlockBytes + kKept : 2 * K * K * 2;
+    static constexpr uint32_t kXb = K / 2, kAcc = K / 2 + 16 * kTwice;  // TMEM columns
+    static_assert(kAcc + 256 <= 512, "TMEM");
+};
+
+template <uint32_t N>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(32 * ChainShape<N>::kWarpsAll, 1)
     chain_kernel(const __grid_constant__ RnsConst kc, const __grid_constant__ ChainArgs a) {
-    constexpr uint32_t K = kSlots * N;
-    constexpr uint32_t kBlocks = (N + 1) / 2;  // of 64 slots, the last of 32 for odd N
-    constexpr uint32_t kBuffers = 2;           // of 128 accumulator columns
-    constexpr uint32_t kCols = K + 128 * kBuffers <= 256 ? 256 : 512;
-    static_assert(K + 128 * kBuffers <= kCols, "TMEM");
+    using S = ChainShape<N>;
+    constexpr uint32_t K = S::K, kBlocks = S::kBlocks, kAcc = S::kAcc;
+    constexpr uint32_t kBuffers = 2;  // of 128 accumulator columns
+    constexpr uint32_t kCols = 512, kRingSlots = S::kSlotsOfRing;
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ uint32_t s_tmem;
     __shared__ __align__(8) uint64_t s_done[N], s_free[kBuffers], s_full[kBuffers], s_end;
+    __shared__ __align__(8) uint64_t s_landed[kRingSlots], s_peer[kRingSlots], s_empty[kRingSlots];
 
     const uint64_t n_items = a.count ? min((uint64_t)*a.count, a.max_items) : a.max_items;
     const uint32_t pair = blockIdx.x / 2, rank = blockIdx.x & 1;
@@ -624,12 +680,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         for (uint32_t i = 0; i < N; i++) mbar_init(smem_addr(&s_done[i]), 2 * kWarps);
         for (uint32_t i = 0; i < kBuffers; i++) mbar_init(smem_addr(&s_full[i]), 1), mbar_init(smem_addr(&s_free[i]), 2 * kWarps);
         mbar_init(smem_addr(&s_end), 1);
+        for (uint32_t i = 0; i < kRingSlots; i++)
+            mbar_init(smem_addr(&s_landed[i]), 1), mbar_init(smem_addr(&s_peer[i]), 1),
+                mbar_init(smem_addr(&s_empty[i]), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    {
-        const uint4 *src = a.matrices + (uint64_t)rank * (2 * K * K / 8);
+    const uint4 *const matrices = a.matrices + (uint64_t)rank * (2 * K * K / 8);
+    if constexpr (!S::kRing) {
         uint4 *dst = reinterpret_cast<uint4 *>(smem);
-        for (uint32_t i = threadIdx.x; i < 2 * K * K / 8; i += kThreads) dst[i] = src[i];
+        for (uint32_t i = threadIdx.x; i < 2 * K * K / 8; i += kThreads) dst[i] = matrices[i];
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the tensor cores read it
     fence_before();
@@ -637,7 +696,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     cluster_sync();
     fence_after();
     const uint32_t tmem = s_tmem;
-    constexpr uint32_t kX1 = 0, kX2 = K / 2, kAcc = K;
+    // chunk c of the A operand of product ph: even ones sum xi of B, odd ones of A
+    const auto x_at = [](uint32_t ph, uint32_t c) { return 16 * c + ((ph & 1) && c < S::kTwice ? S::kXb : 0u); };
     bool gone = false;
 
     if (warp < kWarps) {
@@ -656,10 +716,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             __syncwarp();
             if (lane == 0) asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
         };
+        uint4 *const kept = reinterpret_cast<uint4 *>(smem + S::kShared - S::kKept) + wg * 128 + row;
         for (uint32_t c = 0; c < N; c++) {
             const uint4 v = a.state[at0 + 512 * c];
             const uint32_t x[4] = {v.x, v.y, v.z, v.w};
-            tmem_st4(lanes + kX2 + 16 * c + 4 * wg, x);
+            tmem_st4(lanes + x_at(0, c) + 4 * wg, x);
+            if (c >= S::kTwice) kept[(c - S::kTwice) * 512] = v;
             tmem_wait_st();
             arrive(done0 + 8 * c);
         }
@@ -672,8 +734,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         };
         // One product's sums to the residues of the next: blocks of two chunks (8 slots each
         // per thread), the numbers' constants loaded a block ahead.
-        const auto product = [&](const uint4 *nums, const uint4 *next, uint32_t (&cw)[2][4], uint32_t x_at,
+        const auto product = [&](const uint4 *nums, const uint4 *next, uint32_t (&cw)[2][4], uint32_t to,
                                  bool rank_too, auto &&residues) {
+            [[maybe_unused]] uint32_t late[N - S::kTwice + 1][4];
 #pragma unroll 1
             for (uint32_t b = 0; b < kBlocks; b++, seq++) {
                 const bool two = 2 * b + 1 < N;
@@ -693,20 +756,34 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                 if (two) tmem_wait_ld(lo[1], hi[1], rk);
                 arrive(free0 + 8 * (seq & 1));
                 residues(2 * b, lo[0], hi[0], rk, cw[0], x[0]);
-                tmem_st4(lanes + x_at + 32 * b + 4 * wg, x[0]);
+                const bool now0 = 2 * b < S::kTwice, now1 = two && 2 * b + 1 < S::kTwice;
+                if (now0) tmem_st4(lanes + x_at(to, 2 * b) + 4 * wg, x[0]);
+                if constexpr (N > 8)
+                    if (2 * b == 8) late[1][0] = x[0][0], late[1][1] = x[0][1], late[1][2] = x[0][2], late[1][3] = x[0][3];
                 // the next block's constants, or the next product's first
                 const uint4 *from = b + 1 < kBlocks ? nums : next;
                 const uint32_t at = b + 1 < kBlocks ? 2 * b + 2 : 0;
                 load(from, at, cw[0]);
                 if (two) residues(2 * b + 1, lo[1], hi[1], rk, cw[1], x[1]);
-                tmem_wait_st();
-                arrive(done0 + 16 * b);
-                if (two) tmem_st4(lanes + x_at + 32 * b + 16 + 4 * wg, x[1]);
+                if (now0) {
+                    tmem_wait_st();
+                    arrive(done0 + 16 * b);
+                }
+                if (now1) tmem_st4(lanes + x_at(to, 2 * b + 1) + 4 * wg, x[1]);
+                if constexpr (N > 7)
+                    if (2 * b + 1 == 7) late[0][0] = x[1][0], late[0][1] = x[1][1], late[0][2] = x[1][2], late[0][3] = x[1][3];
                 if (at + 1 < N) load(from, at + 1, cw[1]);
-                if (two) {
+                if (now1) {
                     tmem_wait_st();
                     arrive(done0 + 16 * b + 8);
                 }
+            }
+            if constexpr (N > 7) {  // the last block's sums are in: the product is done with their place
+#pragma unroll
+                for (uint32_t c = 7; c < N; c++) tmem_st4(lanes + x_at(to, c) + 4 * wg, late[c - 7]);
+                tmem_wait_st();
+#pragma unroll
+                for (uint32_t c = 7; c < N; c++) arrive(done0 + 8 * c);
             }
         };
         uint32_t cw[2][4];
@@ -724,7 +801,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             // sums of xi over B -> x in A -> xi in A
             f2 rank2 = 0;
             product(
-                a.num_a, a.num_b, cw, kX1, true,
+                a.num_a, a.num_b, cw, 1, true,
                 [&](uint32_t c, const uint32_t (&lo)[8], const uint32_t (&hi)[8], uint32_t rk, const uint32_t (&w)[4],
                     uint32_t (&x)[4]) {
                     if (c == 0) rank2 = rank_of(rk);
@@ -734,64 +811,114 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             const bool dump = step + kRnsDumps >= a.steps;
             uint4 *const to = a.dumps + (a.steps - 1 - step) * a.dump_stride + at0;
             product(
-                a.num_b, a.num_a, cw, kX2, false,
+                a.num_b, a.num_a, cw, 0, false,
                 [&](uint32_t c, const uint32_t (&lo)[8], const uint32_t (&hi)[8], uint32_t, const uint32_t (&w)[4],
                     uint32_t (&x)[4]) {
                     uint32_t old[4];
-                    tmem_ld4(old, lanes + kX2 + 16 * c + 4 * wg);
-                    tmem_wait_ld(old);
+                    if (c < S::kTwice) {
+                        tmem_ld4(old, lanes + x_at(0, c) + 4 * wg);
+                        tmem_wait_ld(old);
+                    } else {
+                        const uint4 v = kept[(c - S::kTwice) * 512];
+                        old[0] = v.x, old[1] = v.y, old[2] = v.z, old[3] = v.w;
+                    }
                     residues_b(kc.b + (16 * c + 4 * wg), lo, hi, old, w, four, mg, x);
-                    if (dump) to[512 * c] = make_uint4(x[0], x[1], x[2], x[3]);
+                    const uint4 v = make_uint4(x[0], x[1], x[2], x[3]);
+                    if (c >= S::kTwice) kept[(c - S::kTwice) * 512] = v;
+                    if (dump) to[512 * c] = v;
                 });
         }
-    } else if (rank == 0 && lane == 0) {
+    } else if (warp == kWarps && rank == 0 && lane == 0) {
         // f16 operands, f32 sums, both K-major, M = 256
         constexpr uint32_t kInstr = (1u << 4) | ((256 / 16) << 24);
         const uint32_t base = smem_addr(smem);
-        auto multiply = [&](uint32_t d, uint32_t x, uint32_t b, uint32_t kk) {
-            const uint32_t slots = 2 * b + 1 < N ? 64 : 32;  // N = twice that
-            // 8 x 8 pieces of 128 bytes, unswizzled: slots 128 bytes apart, k a row of them
-            const uint32_t row = slots / 8 * 128;
-            const uint32_t from = base + (x == tmem + kX1 ? 2 * K * K : 0) + b * (64 * K * 2) + kk * 2 * row;
-            const uint64_t desc = (uint64_t)((from & 0x3FFFF) >> 4) | ((uint64_t)(row / 16) << 16) |
-                                  ((uint64_t)(128 / 16) << 32) | (1ull << 46);
-            asm volatile(
-                "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
-                "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d),
-                "r"(x + 8 * kk), "l"(desc), "r"(kInstr | (slots * 2 / 8) << 17), "r"(kk)
-                : "memory");
-        };
         uint32_t seq = 0;
         for (uint32_t ph = 0; ph < 2 * a.steps; ph++) {
-            const uint32_t x = tmem + (ph & 1 ? kX1 : kX2);
             for (uint32_t b = 0; b < kBlocks; b++, seq++) {
                 const uint32_t d = tmem + kAcc + 128 * (seq & 1);
-                // the buffer's last sums have been read
-                if (seq >= kBuffers) {
-                    mbar_wait(smem_addr(&s_free[seq & 1]), (seq / kBuffers - 1) & 1, gone);
-                    fence_after();
+                const uint32_t slots = 2 * b + 1 < N ? 64 : 32;  // columns: twice that
+                const uint32_t ring = seq % kRingSlots;
+                const uint32_t block = base + (S::kRing ? ring * S::kBlockBytes : (ph & 1) * (2 * K * K) + b * S::kBlockBytes);
+                // 8 x 8 pieces of 128 bytes, unswizzled: slots 128 bytes apart, k a row of them
+                const uint32_t row = slots / 8 * 128;
+                const auto multiply = [&](uint32_t kk) {
+                    const uint64_t desc = (uint64_t)(((block + kk * 2 * row) & 0x3FFFF) >> 4) |
+                                          ((uint64_t)(row / 16) << 16) | ((uint64_t)(128 / 16) << 32) | (1ull << 46);
+                    asm volatile(
+                        "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
+                        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d),
+                        "r"(tmem + x_at(ph, kk / 2) + 8 * (kk & 1)), "l"(desc), "r"(kInstr | (slots * 2 / 8) << 17),
+                        "r"(kk)
+                        : "memory");
+                };
+                // the buffer's last sums have been read; the block is there in both CTAs
+                if (seq >= kBuffers) mbar_wait(smem_addr(&s_free[seq & 1]), (seq / kBuffers - 1) & 1, gone);
+                if constexpr (S::kRing) {
+                    mbar_wait(smem_addr(&s_landed[ring]), (seq / kRingSlots) & 1, gone);
+                    mbar_wait(smem_addr(&s_peer[ring]), (seq / kRingSlots) & 1, gone);
                 }
+                fence_after();
                 if (b == 0) {  // slice by slice, as the residues appear
+#pragma unroll(S::kRing ? 1 : N)
                     for (uint32_t i = 0; i < N; i++) {
                         mbar_wait(smem_addr(&s_done[i]), ph & 1, gone);
                         fence_after();
-                        multiply(d, x, b, 2 * i);
-                        multiply(d, x, b, 2 * i + 1);
+                        multiply(2 * i);
+                        multiply(2 * i + 1);
                     }
                 } else {
-                    for (uint32_t kk = 0; kk < 2 * N; kk++) multiply(d, x, b, kk);
+#pragma unroll(S::kRing ? 1 : 2 * N)
+                    for (uint32_t kk = 0; kk < 2 * N; kk++) multiply(kk);
                 }
+                const auto commit = [](uint64_t *bar) {  // in both CTAs
+                    asm volatile(
+                        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::
+                            "r"(smem_addr(bar)),
+                        "h"((uint16_t)3)
+                        : "memory");
+                };
+                commit(&s_full[seq & 1]);
+                if constexpr (S::kRing) commit(&s_empty[ring]);
+            }
+        }
+    } else if (S::kRing && warp == kWarps && lane == 0) {
+        // the other CTA's half of each block has landed: tell the one that multiplies
+        uint32_t peer0;
+        asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(peer0) : "r"(smem_addr(&s_peer[0])));
+        for (uint32_t seq = 0; seq < 2 * a.steps * kBlocks; seq++) {
+            mbar_wait(smem_addr(&s_landed[seq % kRingSlots]), (seq / kRingSlots) & 1, gone);
+            asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(peer0 + 8 * (seq % kRingSlots)) : "memory");
+        }
+    } else if (S::kRing && warp == kWarps + 1 && lane == 0) {
+        // this CTA's half of each block, in the order in which the products use them
+        uint32_t seq = 0;
+        for (uint32_t ph = 0; ph < 2 * a.steps; ph++) {
+            for (uint32_t b = 0; b < kBlocks; b++, seq++) {
+                const uint32_t ring = seq % kRingSlots;
+                const uint32_t bytes = 2 * b + 1 < N ? S::kBlockBytes : S::kBlockBytes / 2;
+                if (seq >= kRingSlots) mbar_wait(smem_addr(&s_empty[ring]), (seq / kRingSlots - 1) & 1, gone);
+                if (gone) break;  // nothing more is asked for
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(&s_landed[ring])),
+                             "r"(bytes)
+                             : "memory");
                 asm volatile(
-                    "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::
-                        "r"(smem_addr(&s_full[seq & 1])),
-                    "h"((uint16_t)3)
+                    "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                        smem_addr(smem + ring * S::kBlockBytes)),
+                    "l"((const char *)matrices + (size_t)(ph & 1) * (2 * K * K) + (size_t)b * S::kBlockBytes), "r"(bytes),
+                    "r"(smem_addr(&s_landed[ring]))
                     : "memory");
             }
+            if (gone) break;
+        }
+        if (gone) {  // copies in flight land before the CTA ends
+            bool late = false;
+            for (uint32_t i = seq > kRingSlots ? seq - kRingSlots : 0; i < seq; i++)
+                mbar_wait(smem_addr(&s_landed[i % kRingSlots]), (i / kRingSlots) & 1, late);
         }
     }
     if (gone) {
         atomicExch(a.error, 1ull);
-        if (warp == kWarps) {  // products still in flight end before TMEM is given back
+        if (warp == kWarps && rank == 0) {  // products still in flight end before TMEM is given back
             asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                              smem_addr(&s_end))
                          : "memory");
@@ -1054,8 +1181,8 @@ __global__ void verdict_kernel(const __grid_constant__ RnsSlots p, uint32_t chun
                                uint32_t limbs, const unsigned long long *count, uint64_t max_items,
                                const __half *__restrict__ num_b, const __half *__restrict__ dumps, uint64_t dump_stride,
                                const uint32_t *__restrict__ nums, const long long *__restrict__ quot,
-                               const uint32_t *__restrict__ flag, uint8_t *__restrict__ result,
-                               uint32_t *__restrict__ list, unsigned long long *__restrict__ listed) {
+                               const uint32_t *__restrict__ flag, const uint32_t *__restrict__ factor,
+                               uint8_t *__restrict__ result, uint32_t *__restrict__ list, unsigned long long *__restrict__ listed) {
     const uint64_t n_items = count ? min((uint64_t)*count, max_items) : max_items;
     const uint64_t i = (uint64_t)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
     if (i >= n_items) return;
@@ -1107,6 +1234,20 @@ __global__ void verdict_kernel(const __grid_constant__ RnsSlots p, uint32_t chun
                 }
             }
             if (!have) break;                                     // N shares a factor with them all
+            const uint32_t by = factor[i];
+            if (ok && by > 1) {
+                // the chain ran mod N / by: the value mod by, 2^((N - 1) / 2^(d + 1)), has to agree
+                const uint32_t e = by - 1, ie = inv32_of(e), sh = d + 1;
+                uint32_t r = 0;
+                for (int w = (int)limbs - 1; w >= 0; w--) {
+                    const uint32_t up = w + 1 < (int)limbs ? n[w + 1] : 0u;
+                    const uint32_t v = __funnelshift_r(n[w], up, sh);
+                    r = mod_lazy((r << 16) | (v >> 16), e, ie);
+                    r = mod_lazy((r << 16) | (v & 0xFFFFu), e, ie);
+                }
+                const uint32_t z = pow_small(2, r, by, inv32_of(by));
+                ok = z == (sign == -3 ? by - 1 : 1u);
+            }
             if (!ok) f = kFlagRun;                                // neither: composite
             else if (sign == -3) f = kFlagRun, prime = true;      // -1 on the way
             else if (d + 1 == s) f = kFlagRun, prime = true;      // 1 from the start
@@ -1119,7 +1260,7 @@ __global__ void verdict_kernel(const __grid_constant__ RnsSlots p, uint32_t chun
 }
 
 // Tiles per pair: enough that their residues take longer than one tile's exchange.
-constexpr uint32_t kTilesOf[kRnsMaxChunks + 1] = {0, 4, 3, 2, 2, 2, 2, 1};
+constexpr uint32_t kTilesOf[kRnsMaxChunks + 1] = {0, 4, 3, 2, 2, 2, 2, 1, 1, 1};
 
 // Pairs of CTAs that run at once, one CTA per SM.
 uint64_t pairs_at_once() {
@@ -1148,11 +1289,11 @@ cudaError_t launch_chain(const RnsPlan &p, const ChainArgs &a, uint64_t tiles, c
     }
     // at least half of the SM's shared memory: a second CTA would wait for TMEM
     // columns, and two pairs could each hold what the other waits for
-    constexpr uint32_t matrices = 2 * (kSlots * N) * (kSlots * N) * 2;
-    constexpr uint32_t bytes = matrices > 118 * 1024 ? matrices : 118 * 1024;
+    using S = ChainShape<N>;
+    constexpr uint32_t bytes = S::kShared > 118 * 1024 ? S::kShared : 118 * 1024;
     cudaError_t e = cudaFuncSetAttribute(chain_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return e;
-    chain_kernel<N><<<(unsigned)(2 * tiles), kThreads, bytes, s>>>(p.k, a);
+    chain_kernel<N><<<(unsigned)(2 * tiles), 32 * S::kWarpsAll, bytes, s>>>(p.k, a);
     return cudaGetLastError();
 }
 
@@ -1193,6 +1334,7 @@ RnsLayout rns_layout(uint32_t bits, uint32_t limbs, uint64_t max_items) {
     l.nums = take(numbers * limbs * 4);
     l.quot = take(numbers * 8);
     l.flag = take(numbers * 4);
+    l.factor = take(numbers * 4);
     l.list = take(numbers * 4);
     l.counters = take(16);
     l.total = off;
@@ -1219,7 +1361,7 @@ cudaError_t rns_test(const RnsLayout &l, uint32_t bits, void *work, const uint32
     setup_kernel<<<(unsigned)((tiles + kRnsGroup - 1) * (kRnsTile / kSetupNumbers)), k, 0, s>>>(
         p.s, l.chunks, bits, p.a_mant, p.a_exp, l.limbs, bases, items, count, max_items, at<__half>(work, l.num_a),
         at<__half>(work, l.num_b), at<__half>(work, l.state), at<uint32_t>(work, l.nums), at<long long>(work, l.quot),
-        at<uint32_t>(work, l.flag));
+        at<uint32_t>(work, l.flag), at<uint32_t>(work, l.factor));
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const ChainArgs a{at<uint4>(work, l.matrices), at<uint4>(work, l.num_a), at<uint4>(work, l.num_b),
@@ -1235,12 +1377,15 @@ cudaError_t rns_test(const RnsLayout &l, uint32_t bits, void *work, const uint32
         case 5: e = launch_chain<5>(p, a, tiles, s); break;
         case 6: e = launch_chain<6>(p, a, tiles, s); break;
         case 7: e = launch_chain<7>(p, a, tiles, s); break;
+        case 8: e = launch_chain<8>(p, a, tiles, s); break;
+        case 9: e = launch_chain<9>(p, a, tiles, s); break;
         default: return cudaErrorInvalidValue;
     }
     if (e != cudaSuccess) return e;
     verdict_kernel<<<(unsigned)((max_items + 3) / 4), 128, 0, s>>>(
         p.s, l.chunks, steps, p.t_max, l.limbs, count, max_items, at<__half>(work, l.num_b), at<__half>(work, l.dumps),
-        numbers * k, at<uint32_t>(work, l.nums), at<long long>(work, l.quot), at<uint32_t>(work, l.flag), result,
+        numbers * k, at<uint32_t>(work, l.nums), at<long long>(work, l.quot), at<uint32_t>(work, l.flag),
+        at<uint32_t>(work, l.factor), result,
         at<uint32_t>(work, l.list), at<unsigned long long>(work, l.counters));
     return cudaGetLastError();
 }

@@ -7,7 +7,7 @@
 
 namespace pg {
 
-constexpr uint32_t kRnsMaxChunks = 7;   // 32 residue slots each
+constexpr uint32_t kRnsMaxChunks = 9;   // 32 residue slots each
 constexpr uint32_t kRnsDumps = 8;       // last values kept for the strong test's verdict
 constexpr uint32_t kRnsTile = 256;      // numbers of a tile, half in each CTA of a pair
 constexpr uint32_t kRnsGroup = 4;       // most tiles that a pair takes in turn
@@ -28,7 +28,7 @@ uint64_t rns_wave(uint32_t bits, bool full);
 struct RnsLayout {
     uint32_t chunks, limbs;
     uint64_t tiles;  // of kRnsTile numbers
-    size_t matrices, num_a, num_b, state, dumps, nums, quot, flag, list, counters, total;
+    size_t matrices, num_a, num_b, state, dumps, nums, quot, flag, factor, list, counters, total;
 };
 RnsLayout rns_layout(uint32_t bits, uint32_t limbs, uint64_t max_items);
 

@@ -19,9 +19,9 @@ def _numbers(rng, bits, count):
     return [rng.getrandbits(bits - 1) | (1 << (bits - 1)) | 1 for _ in range(count)]
 
 
-# the last widths of one to seven chunks of 32 slots and the ones after them
+# the last widths of one to nine chunks of 32 slots and the ones after them
 @pytest.mark.parametrize("bits", [252, 253, 367, 368, 741, 742, 1107, 1108, 1465, 1466, 1812, 1813, 2146, 2147,
-                                  2461, 2462])
+                                  2461, 2462, 2748, 2749, 2895, 2910])
 def test_rns_widths(sieve, bits):
     rng = random.Random(bits)
     nums = _numbers(rng, bits, 20) + [(1 << bits) - 1, (1 << (bits - 1)) + 1]
@@ -68,7 +68,7 @@ def test_rns_pseudoprimes_and_near_misses(sieve, p):
 
 
 @pytest.mark.parametrize("bits,count", [(301, 20480), (720, 20000), (1000, 19457), (1300, 39169), (1700, 19713),
-                                        (2100, 20100)])
+                                        (2100, 20100), (2300, 19460), (2800, 19460)])
 def test_rns_more_numbers_than_one_wave(sieve, bits, count):
     """Several tiles per pair of CTAs: the same answers as a few numbers get, at
     every place (the last group of tiles not full)."""
@@ -81,3 +81,37 @@ def test_rns_more_numbers_than_one_wave(sieve, bits, count):
     want = [po.strong_prp2(n) for n in few]
     got = sieve.prp_test([few[i % len(few)] for i in range(count)])
     assert all(got[i] == want[i % len(few)] for i in range(count))
+
+
+@pytest.mark.parametrize("bits", [300, 720, 1300, 2100, 2800])
+def test_rns_multiples_of_the_bases_primes(sieve, bits):
+    """N = q c with q a prime of the residue system and 2^(N-1) = 1 mod q, the
+    ones that q alone does not rule out; also with two such factors."""
+    rng = random.Random(bits)
+    nums = []
+    for q in [x for x in SMALL if x > 2600]:
+        order = next(o for o in range(1, q) if pow(2, o, q) == 1)
+        if order > 400:
+            continue
+        c = rng.getrandbits(bits - 12) | 1 << (bits - 12) | 1
+        while (q * c) % (2 * order) != 1:
+            c += 2
+        nums += [q * c, q * c + 2]
+        c = rng.getrandbits(bits - 24) | 1 << (bits - 24) | 1
+        while (q * q * c) % (2 * order) != 1:
+            c += 2
+        nums.append(q * q * c)
+    assert len(nums) == 60
+    assert sieve.prp_test(nums) == [po.strong_prp2(n) for n in nums]
+
+
+def test_rns_strong_pseudoprimes_with_a_factor_of_the_base(sieve):
+    """(4^p + 1)/5 with a prime factor 4pk + 1 below 4096: probable primes whose
+    chain runs without that factor."""
+    nums = []
+    for p in [x for x in SMALL if 131 <= x < 1000]:
+        if any(q in SMALL and pow(4, p, q) == q - 1 for q in range(4 * p + 1, 4096, 4 * p)):
+            nums += [(4**p + 1) // 5, (4**p + 1) // 5 + 2, (4**p - 1) // 3]
+    assert len(nums) >= 12
+    for n in nums:  # one width at a time: each its own plan
+        assert sieve.prp_test([n, n]) == [po.strong_prp2(n)] * 2, n
