@@ -368,8 +368,8 @@ struct PrpPlan {
 // Where the residue form is the faster one, in ms for 16 numbers and for 19456
 // (limbs, residues): 200 bits 0.21, 0.32 and 0.44, 0.51; 256 bits 0.46, 0.39 and
 // 1.21, 0.61; 712 bits 1.61, 1.74 and 4.94, 2.07 (5000 numbers: 2.15, 1.85); 1100
-// bits 4.36, 3.58; 1400 bits 6.33, 5.98 and 29.9, 6.7; 2136 bits 16.0, 13.3 and 105,
-// 14.7; 2838 bits (9001 numbers) 106, 43.  So from two limbs per lane on; with two or three chunks of slots and
+// bits 4.36, 3.58; 1400 bits 6.33, 5.31 and 29.9, 6.7; 2136 bits 16.0, 11.6 and 105,
+// 12.9; 2838 bits (9001 numbers) 106, 30.  So from two limbs per lane on; with two or three chunks of slots and
 // fewer than three limbs per lane only for enough numbers to fill the limb form.
 bool rns_pays(uint32_t bits, uint64_t max_items) {
     const uint32_t n = rns_chunks(bits);
@@ -838,15 +838,14 @@ int prp_gaps_core(pgs_ctx *ctx, const pgs_gap_params *prm, uint64_t rows, const 
     while (e == cudaSuccess && active > 0) {
         uint64_t quota = limb_round;
         if (plan.rns) {
-            // A wave of several tiles per pair tests 1.2-1.4 times as many a second as
+            // A wave of several tiles per pair tests 1.1-1.2 times as many a second as
             // a single one, but what lies past a search's end is wasted: with s
             // candidates per search in the single wave and a chance p of each (found
-            // so far / tested), it resolves more a second where s p is above 0.55
-            // (2136 bits, p 1/39, 21.5 and 13.5 ms: 31.4 against 30.4 searches a ms at
-            // s p = 0.43, 26.0 against 27.3 at 0.66).
+            // so far / tested), it resolves more a second where s p is below 0.45
+            // (2136 bits, p 1/39, 20.5 and 12.4 ms: 33 searches a ms each at s p = 0.43).
             const uint64_t one = pg::rns_wave(bits, false);
             const double chance = launched ? (double)host_ctr[4] / (double)launched : 1.0 / 32;
-            quota = (double)one * chance < 0.55 * (double)active ? max_items : one;
+            quota = (double)one * chance < 0.45 * (double)active ? max_items : one;
         }
         quota = std::min(quota, active * kMaxSpec);
         const uint32_t spec = (uint32_t)(quota / active), extra = (uint32_t)(quota % active);

@@ -35,8 +35,8 @@
 // residues, 32 slots at a time, the tensor cores work on the next one, and the next
 // product's first block accumulates slice by slice as the residues appear.
 //
-// Measured (2136-bit numbers, 19456 at once): 14.8 ms, 1.32e6 tests/s, where the
-// limb form takes 105 ms; a squaring step 6.2 us per pair, of which the products
+// Measured (2136-bit numbers, 19456 at once): 12.9 ms, 1.5e6 tests/s, where the
+// limb form takes 105 ms; a squaring step 5.4 us per pair, of which the products
 // alone take 2.9 (128 columns cost 78 cycles per 16 of K; 64 columns cost the same,
 // the A operand's read, hence blocks of 128) and the residues' f32 operations 3.4.
 #include "pg_rns.h"
@@ -489,6 +489,36 @@ __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+// One lane of a warp that is all here.
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r;
+}
+
+// Product d (+)= x b of the pair, issued by the lane that has `one`: the whole warp
+// keeps its addresses, so that they stay in uniform registers (a single lane's
+// would be moved there for every product: 2838 bits 14.8 us a step so, 10.0 now;
+// 2136 bits 6.2 and 5.4).
+__device__ __forceinline__ void multiply_pair(uint32_t one, uint32_t d, uint32_t x, uint64_t b, uint32_t instr,
+                                              uint32_t add) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %4, 0;\n\tsetp.ne.u32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d),
+        "r"(x), "l"(b), "r"(instr), "r"(add), "r"(one)
+        : "memory");
+}
+
+// The barrier of both CTAs completes when the products issued so far are done.
+__device__ __forceinline__ void commit_pair(uint32_t one, uint32_t bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t"
+        "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}" ::
+            "r"(bar),
+        "h"((uint16_t)3), "r"(one)
+        : "memory");
+}
+
 __device__ __forceinline__ void tmem_ld8(uint32_t (&r)[8], uint32_t addr) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
@@ -632,8 +662,7 @@ struct ChainArgs {
 // Up to seven chunks the matrices stay in shared memory and both A operands (of
 // the product under way and of the next) lie in TMEM in full.  Above, the
 // matrices' blocks go round a ring, copied from L2 ahead of each product (2838
-// bits: 14.8 us a step, 12.5 without the copies; 9001 numbers 43 ms where the limb
-// form takes 106), and the
+// bits: 10.0 us a step; 9001 numbers 29.7 ms where the limb form takes 106), and the
 // chunks from the eighth on have one place in TMEM: their residues are written
 // when the product's last sums are in, and B's (needed again for the next square)
 // are kept in shared memory.
@@ -828,7 +857,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(32 * ChainShape<N>::
                     if (dump) to[512 * c] = v;
                 });
         }
-    } else if (warp == kWarps && rank == 0 && lane == 0) {
+    } else if (warp == kWarps && rank == 0) {
+        const uint32_t one = elect_one();
         // f16 operands, f32 sums, both K-major, M = 256
         constexpr uint32_t kInstr = (1u << 4) | ((256 / 16) << 24);
         const uint32_t base = smem_addr(smem);
@@ -841,15 +871,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(32 * ChainShape<N>::
                 const uint32_t block = base + (S::kRing ? ring * S::kBlockBytes : (ph & 1) * (2 * K * K) + b * S::kBlockBytes);
                 // 8 x 8 pieces of 128 bytes, unswizzled: slots 128 bytes apart, k a row of them
                 const uint32_t row = slots / 8 * 128;
+                const uint64_t desc = (uint64_t)((block & 0x3FFFF) >> 4) | ((uint64_t)(row / 16) << 16) |
+                                      ((uint64_t)(128 / 16) << 32) | (1ull << 46);
+                const uint32_t instr = kInstr | (slots * 2 / 8) << 17;
                 const auto multiply = [&](uint32_t kk) {
-                    const uint64_t desc = (uint64_t)(((block + kk * 2 * row) & 0x3FFFF) >> 4) |
-                                          ((uint64_t)(row / 16) << 16) | ((uint64_t)(128 / 16) << 32) | (1ull << 46);
-                    asm volatile(
-                        "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
-                        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d),
-                        "r"(tmem + x_at(ph, kk / 2) + 8 * (kk & 1)), "l"(desc), "r"(kInstr | (slots * 2 / 8) << 17),
-                        "r"(kk)
-                        : "memory");
+                    multiply_pair(one, d, tmem + x_at(ph, kk / 2) + 8 * (kk & 1), desc + kk * (2 * row / 16), instr, kk);
                 };
                 // the buffer's last sums have been read; the block is there in both CTAs
                 if (seq >= kBuffers) mbar_wait(smem_addr(&s_free[seq & 1]), (seq / kBuffers - 1) & 1, gone);
@@ -859,7 +885,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(32 * ChainShape<N>::
                 }
                 fence_after();
                 if (b == 0) {  // slice by slice, as the residues appear
-#pragma unroll(S::kRing ? 1 : N)
+#pragma unroll
                     for (uint32_t i = 0; i < N; i++) {
                         mbar_wait(smem_addr(&s_done[i]), ph & 1, gone);
                         fence_after();
@@ -867,18 +893,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(32 * ChainShape<N>::
                         multiply(2 * i + 1);
                     }
                 } else {
-#pragma unroll(S::kRing ? 1 : 2 * N)
+#pragma unroll
                     for (uint32_t kk = 0; kk < 2 * N; kk++) multiply(kk);
                 }
-                const auto commit = [](uint64_t *bar) {  // in both CTAs
-                    asm volatile(
-                        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::
-                            "r"(smem_addr(bar)),
-                        "h"((uint16_t)3)
-                        : "memory");
-                };
-                commit(&s_full[seq & 1]);
-                if constexpr (S::kRing) commit(&s_empty[ring]);
+                commit_pair(one, smem_addr(&s_full[seq & 1]));
+                if constexpr (S::kRing) commit_pair(one, smem_addr(&s_empty[ring]));
             }
         }
     } else if (S::kRing && warp == kWarps && lane == 0) {
@@ -919,9 +938,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(32 * ChainShape<N>::
     if (gone) {
         atomicExch(a.error, 1ull);
         if (warp == kWarps && rank == 0) {  // products still in flight end before TMEM is given back
-            asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                             smem_addr(&s_end))
-                         : "memory");
+            if (lane == 0)
+                asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                                 smem_addr(&s_end))
+                             : "memory");
             bool late = false;
             mbar_wait(smem_addr(&s_end), 0, late);
         }
@@ -940,8 +960,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(32 * ChainShape<N>::
 // operand in TMEM: the next one replaces it when its product's last sums are in,
 // so a product's residues wait in registers; B's residues, needed again for the
 // next square, are kept in shared memory (what does not fit, in TMEM).
-// 38912 numbers of 2136 bits: 23.7 ms against 29.6 ms in two single waves (58368
-// of 712 bits: 4.9 against 6.2), the f32 pipe 68 % busy, the tensor cores 47 %.
+// 38912 numbers of 2136 bits: 22.9 ms against 25.8 ms in two single waves (58368
+// of 712 bits: 5.0 against 5.7), the f32 pipe 68 % busy, the tensor cores 47 %.
 // Reading the next chunk's sums while a chunk's residues are computed changed
 // nothing (24.9 ms).
 template <uint32_t N, uint32_t T>
@@ -1122,7 +1142,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 #pragma unroll 1
             for (uint32_t t = 0; t < T; t++) product(std::true_type{}, step, t);
         }
-    } else if (rank == 0 && lane == 0) {
+    } else if (rank == 0) {
+        const uint32_t one = elect_one();
         constexpr uint32_t kInstr = (1u << 4) | ((256 / 16) << 24);
         const uint32_t base = smem_addr(smem);
         uint32_t seq = 0;
@@ -1135,31 +1156,24 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                     const uint32_t slots = 2 * b + 1 < N ? 64 : 32, r = slots / 8 * 128;
                     if (seq >= kBuffers) mbar_wait(smem_addr(&s_free[seq & 1]), (seq / kBuffers - 1) & 1, gone);
                     fence_after();
-                    for (uint32_t kk = 0; kk < 2 * N; kk++) {
-                        const uint32_t from = base + (ph & 1 ? 2 * K * K : 0) + b * (64 * K * 2) + kk * 2 * r;
-                        const uint64_t desc = (uint64_t)((from & 0x3FFFF) >> 4) | ((uint64_t)(r / 16) << 16) |
-                                              ((uint64_t)(128 / 16) << 32) | (1ull << 46);
-                        asm volatile(
-                            "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
-                            "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d),
-                            "r"(x + 8 * kk), "l"(desc), "r"(kInstr | (slots * 2 / 8) << 17), "r"(kk)
-                            : "memory");
-                    }
-                    asm volatile(
-                        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::
-                            "r"(smem_addr(&s_full[seq & 1])),
-                        "h"((uint16_t)3)
-                        : "memory");
+                    const uint32_t from = base + (ph & 1 ? 2 * K * K : 0) + b * (64 * K * 2);
+                    const uint64_t desc = (uint64_t)((from & 0x3FFFF) >> 4) | ((uint64_t)(r / 16) << 16) |
+                                          ((uint64_t)(128 / 16) << 32) | (1ull << 46);
+#pragma unroll
+                    for (uint32_t kk = 0; kk < 2 * N; kk++)
+                        multiply_pair(one, d, x + 8 * kk, desc + kk * (2 * r / 16), kInstr | (slots * 2 / 8) << 17, kk);
+                    commit_pair(one, smem_addr(&s_full[seq & 1]));
                 }
             }
         }
     }
     if (gone) {
         atomicExch(a.error, 1ull);
-        if (warp == kWarps) {  // products still in flight end before TMEM is given back
-            asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                             smem_addr(&s_end))
-                         : "memory");
+        if (warp == kWarps && rank == 0) {  // products still in flight end before TMEM is given back
+            if (lane == 0)
+                asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                                 smem_addr(&s_end))
+                             : "memory");
             bool late = false;
             mbar_wait(smem_addr(&s_end), 0, late);
         }
