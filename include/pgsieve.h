@@ -392,7 +392,9 @@ int pgs_tuning_class(const pgs_job *job, char *buf, size_t cap);
  * pgs_method2) use them; batched and served jobs keep the defaults. */
 int pgs_tuning_set(pgs_ctx *ctx, const pgs_job *job, const pgs_tuning *t);
 /* The knobs jobs of this class get: returns 1 when the class is tuned, 0
- * when it gets the defaults. */
+ * when it gets the defaults (one-job runs of such a class take fewer rows per
+ * CTA, fewer text chunks and the fused K mod p where the job's sizes ask for
+ * it). */
 int pgs_tuning_get(pgs_ctx *ctx, const pgs_job *job, pgs_tuning *out);
 /* Load the file's entries for this device (by name); returns how many, or
  * PGS_EINVAL when the file cannot be read. */

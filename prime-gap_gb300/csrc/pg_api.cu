@@ -126,6 +126,7 @@ int pgs_prepare(pgs_ctx *ctx, const pgs_job *job, pgs_prepared **out) {
         return rc;
     }
     pr->tune = tuning_for(ctx, *job);
+    shape_untuned(ctx, pr->hj, pr->tune);
     CK(cudaSetDevice(ctx->device));
     cudaStream_t s = ctx->stream;
     HostJob &h = pr->hj;

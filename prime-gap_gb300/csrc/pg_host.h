@@ -291,6 +291,8 @@ cudaError_t upload(DevBuf &b, const std::vector<T> &v, cudaStream_t s) {
 pg::JobDev job_dev(pgs_prepared *pr);
 // The tuning jobs of this class get on the context (defaults when untuned).
 pgs_tuning tuning_for(pgs_ctx *ctx, const pgs_job &job);
+// Launch shape by the job's sizes where its class is not tuned.
+void shape_untuned(pgs_ctx *ctx, const HostJob &h, pgs_tuning &t);
 pg::RowsDev rows_dev(pgs_prepared *pr);
 uint32_t rows_per_block(uint32_t nb, int compression, uint32_t cap = 16);
 

@@ -14,6 +14,9 @@
 #include "pg_host.h"
 #include "pg_tuning.h"
 
+#include <algorithm>
+#include <cmath>
+
 using namespace pgh;
 
 namespace pgh {
@@ -22,6 +25,34 @@ pgs_tuning tuning_for(pgs_ctx *ctx, const pgs_job &job) {
     std::lock_guard<std::mutex> g(ctx->tune_mu);
     auto it = ctx->tuning.find(pgt::tuning_class(job));
     return it == ctx->tuning.end() ? pgt::tuning_default() : it->second.t;
+}
+
+void shape_untuned(pgs_ctx *ctx, const HostJob &h, pgs_tuning &t) {
+    {
+        std::lock_guard<std::mutex> g(ctx->tune_mu);
+        if (ctx->tuning.count(pgt::tuning_class(h.job))) return;
+    }
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device) != cudaSuccess || sms < 1) sms = 152;
+    // Rows per CTA: about two CTAs per SM while there are too few rows for more.
+    // Rows stage in us with 1, 2, 4, 8, 16: 53 rows (SL 11000) 31, 31, 33, 41, 55;
+    // 527 rows (SL 20000) 51, 47, 51, 61, 88; 1051 rows 88, 63, 53, 63, 88; 2285 rows
+    // (SL 5000) 65, 43, 31, 31, 37; 7321 rows (SL 9500) 203, 143, 113, 98, 104.
+    const uint64_t rows = h.valid_mi.size(), per = (rows + 2 * sms - 1) / (2 * sms);
+    t.rows_per_cta = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(t.rows_per_cta, per));
+    // One chunk of text until its copy is worth overlapping: a chunk costs some 15 us
+    // of launches and events, 16 MB take 90 us on the link (a whole call with 1, 2, 4
+    // chunks: 0.13 MB 549, 562, 600 us; 8 MB 945, 959, 973; 25 MB 1276, 1260, 1223).
+    const double unknowns = (double)rows * 2.0 * h.job.sieve_length * 0.56 / std::log((double)h.prime_limit + 10.0);
+    const double text = unknowns * (h.job.compression == 0 ? 7.0 : h.job.compression == 1 ? 2.0 : 0.5);
+    t.text_chunks = std::min<uint32_t>(t.text_chunks, 1 + (uint32_t)std::min(8.0, text / (16 << 20)));
+    // K mod p inside the large-prime kernel: up to 4e8, where its launch of its own is
+    // too short to be worth a second pass over the primes, and past 2^32 always.  Whole
+    // job in ms, apart and inside: limit 1.3e8 0.73, 0.67 (5000 m of 1511#/2190) and
+    // 0.92, 0.66 (20000 m of 503#/210); 3e8 1.14, 1.13 and 0.95, 0.95; 5e8 1.66, 1.69
+    // and 1.57, 1.39; 9e8 2.66, 2.72; past 2^32, limit 9e9 34.9, 33.8.
+    if (h.prime_limit <= 400000000ull) t.large_form |= 2u;
+    t.large_form |= 4u;
 }
 
 }  // namespace pgh
