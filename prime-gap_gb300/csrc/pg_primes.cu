@@ -4,8 +4,8 @@
 // (combined_sieve.cpp:1475-1502, 1662-1668, 1851-1852): every prime below
 // the sieve limit is produced on the device and stays resident in HBM.
 //
-// One CTA sieves one segment of kSegBits odd numbers in a 32 KiB shared
-// bitmap (bit set = composite):
+// One CTA sieves one segment of kSegBits odd numbers (or a quarter or a 16th
+// of them, sieve_window) in a 32 KiB shared bitmap (bit set = composite):
 //   * base primes below 64 stamp a precomputed 32-bit pattern into every word;
 //   * base primes in [64, 2048) are marked warp-cooperatively;
 //   * larger base primes are marked one per thread;
@@ -65,7 +65,9 @@ __device__ __forceinline__ uint32_t first_index(uint32_t q, uint64_t seg_lo, boo
 }
 
 // Marks composites of the segment [seg_lo, seg_hi] (seg_lo odd) in `bits`.
-// Primes themselves stay clear; 1 is marked.  Blocks of kSieveThreads.
+// Primes themselves stay clear; 1 is marked.  Blocks of kSieveThreads, segments
+// of up to 32 kWords odd numbers.
+template <uint32_t kWords = kSegWords>
 __device__ void sieve_segment(uint32_t *bits, uint64_t seg_lo, uint64_t seg_hi,
                               const uint32_t *base, uint32_t nbase) {
     const uint32_t nbits = (uint32_t)((seg_hi - seg_lo) / 2 + 1);
@@ -85,7 +87,7 @@ __device__ void sieve_segment(uint32_t *bits, uint64_t seg_lo, uint64_t seg_hi,
         o[t] = (j0 + q - (32u * threadIdx.x) % q) % q;
     }
     constexpr uint32_t wstep = 32u * kSieveThreads;
-    for (uint32_t w = threadIdx.x; w < kSegWords; w += kSieveThreads) {
+    for (uint32_t w = threadIdx.x; w < kWords; w += kSieveThreads) {
         uint32_t word = 0;
 #pragma unroll
         for (int t = 0; t < kTinyCount; t++) {
@@ -146,22 +148,24 @@ __device__ void sieve_segment(uint32_t *bits, uint64_t seg_lo, uint64_t seg_hi,
 }
 
 // Unordered compaction of a window's primes (offsets from win_lo).  Each
-// warp owns kSegWords / 16 consecutive words and writes their primes in
+// warp owns kWords / 16 consecutive words and writes their primes in
 // rounds of 32 words, one word per lane: a round's primes are contiguous in
 // the output, so its stores touch a few cache lines rather than one per lane.
+template <uint32_t kWords>
 __global__ void __launch_bounds__(kSieveThreads)
     sieve_window_kernel(uint64_t win_lo, uint64_t win_hi, uint64_t first_odd, const uint32_t *base,
                         uint32_t nbase, uint32_t *out, uint64_t cap,
                         unsigned long long *count) {
-    constexpr uint32_t kWarps = kSieveThreads / 32, kWarpWords = kSegWords / kWarps;
-    __shared__ uint32_t bits[kSegWords];
+    constexpr uint32_t kWarps = kSieveThreads / 32, kWarpWords = kWords / kWarps;
+    constexpr uint64_t kSpan = 64ull * kWords;
+    __shared__ uint32_t bits[kWords];
     __shared__ uint32_t s_warp[kWarps];
     __shared__ unsigned long long s_base;
-    const uint64_t seg_lo = first_odd + (uint64_t)blockIdx.x * kSegSpan;
+    const uint64_t seg_lo = first_odd + (uint64_t)blockIdx.x * kSpan;
     if (seg_lo > win_hi) return;
-    uint64_t seg_hi = seg_lo + kSegSpan - 2;
+    uint64_t seg_hi = seg_lo + kSpan - 2;
     if (seg_hi > win_hi) seg_hi = win_hi;
-    sieve_segment(bits, seg_lo, seg_hi, base, nbase);
+    sieve_segment<kWords>(bits, seg_lo, seg_hi, base, nbase);
 
     const uint32_t nbits = (uint32_t)((seg_hi - seg_lo) / 2 + 1);
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -461,9 +465,21 @@ cudaError_t sieve_window(const BasePrimes &bp, uint64_t lo, uint64_t hi, uint32_
     uint64_t first_odd = lo | 1;
     if (first_odd < 3) first_odd = 3;
     if (first_odd > hi) return cudaSuccess;
-    uint64_t nseg = (hi - first_odd) / kSegSpan + 1;
-    sieve_window_kernel<<<(unsigned)nseg, kSieveThreads, 0, stream>>>(
-        lo, hi, first_odd, bp.d_primes, bp.count, d_out, cap, d_count);
+    const uint64_t odds = (hi - first_odd) / 2 + 1;
+    const auto launch = [&](auto kernel, uint32_t words) {
+        const uint64_t nseg = (odds + 32ull * words - 1) / (32ull * words);
+        kernel<<<(unsigned)nseg, kSieveThreads, 0, stream>>>(lo, hi, first_odd, bp.d_primes, bp.count, d_out, cap,
+                                                             d_count);
+    };
+    // Segments of 2^18 odd numbers when they fill most of the GPU's 608 places (four
+    // CTAs per SM), shorter ones for shorter windows, where one segment's 70 us latency
+    // is the whole time.  Small-primes and window stages, 2^18, 2^16, 2^14 odd numbers (whole
+    // job): to 1e7 77, 38, 34 us (185, 152, 149); 1e8 99, 78, 132 (388, 367, 425); 2e8
+    // 126, 122, 243 (602, 592, 718); 4e8
+    // 199, 213, 473 (1045, 1039, 1303); 1.07e9 380, 525, 1276.
+    if (odds > 450ull * kSegBits) launch(sieve_window_kernel<kSegWords>, kSegWords);
+    else if (odds > 128ull * (kSegBits / 4)) launch(sieve_window_kernel<kSegWords / 4>, kSegWords / 4);
+    else launch(sieve_window_kernel<kSegWords / 16>, kSegWords / 16);
     return cudaGetLastError();
 }
 
