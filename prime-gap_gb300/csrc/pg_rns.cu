@@ -35,8 +35,8 @@
 // residues, 32 slots at a time, the tensor cores work on the next one, and the next
 // product's first block accumulates slice by slice as the residues appear.
 //
-// Measured (2136-bit numbers, 19456 at once): 12.9 ms, 1.5e6 tests/s, where the
-// limb form takes 105 ms; a squaring step 5.4 us per pair, of which the products
+// Measured (2136-bit numbers, 19456 at once): 12.2 ms, 1.6e6 tests/s, where the
+// limb form takes 105 ms; a squaring step 5.2 us per pair, of which the products
 // alone take 2.9 (128 columns cost 78 cycles per 16 of K; 64 columns cost the same,
 // the A operand's read, hence blocks of 128) and the residues' f32 operations 3.4.
 #include "pg_rns.h"
@@ -595,6 +595,18 @@ __device__ __forceinline__ uint32_t hmul2(uint32_t a, uint32_t b) {
     return r;
 }
 
+// a b of both halves, exact in f32: one mixed-precision multiply-add each, where
+// converting the halves first would take two more operations (2136 bits 12.8 ->
+// 12.2 ms).  |a| <= 2048 and |b| <= 8192 are exact in f16.
+__device__ __forceinline__ f2 mul_half2(uint32_t a, uint32_t b) {
+    float x, y;
+    asm("{\n\t.reg .b16 al, ah, bl, bh;\n\tmov.b32 {al, ah}, %2;\n\tmov.b32 {bl, bh}, %3;\n\t"
+        "fma.rn.f32.f16 %0, al, bl, 0f00000000;\n\tfma.rn.f32.f16 %1, ah, bh, 0f00000000;\n\t}"
+        : "=f"(x), "=f"(y)
+        : "r"(a), "r"(b));
+    return pack2(x, y);
+}
+
 // T mod m, balanced: T - m rint(T / m)
 __device__ __forceinline__ f2 red2(f2 t, f2 neg_m, f2 inv_m, f2 magic, f2 neg_magic) {
     const f2 q = add2(fma2(t, inv_m, magic), neg_magic);
@@ -621,21 +633,19 @@ __device__ __forceinline__ void residues_a(const SlotPair *sp, const uint32_t (&
         const f2 l = fma2(rank2, pack2(sp[j].c[0], sp[j].c[1]), pack2u(lo[2 * j], lo[2 * j + 1]));
         const f2 r = red_sum2(l, pack2u(hi[2 * j], hi[2 * j + 1]), nm, im, mg.plus, mg.minus);
         const f2 u = red2(mul2(r, r), nm, im, mg.plus, mg.minus);
-        const f2 v = mul2(u, from_half2(hmul2(w[j], four)));
+        const f2 v = mul_half2(to_half2(u), hmul2(w[j], four));
         x[j] = to_half2(red2(v, nm, im, mg.plus, mg.minus));
     }
 }
 __device__ __forceinline__ void residues_b(const SlotPair *sp, const uint32_t (&lo)[8], const uint32_t (&hi)[8],
                                            const uint32_t (&old)[4], const uint32_t (&w)[4], uint32_t four,
                                            const Magic &mg, uint32_t (&x)[4]) {
-    const f2 four2 = from_half2(four);
 #pragma unroll
     for (uint32_t j = 0; j < 4; j++) {
         const f2 nm = pack2(sp[j].neg_m[0], sp[j].neg_m[1]), im = pack2(sp[j].inv_m[0], sp[j].inv_m[1]);
         const f2 r = red_sum2(pack2u(lo[2 * j], lo[2 * j + 1]), pack2u(hi[2 * j], hi[2 * j + 1]), nm, im, mg.plus,
                               mg.minus);
-        const f2 o = from_half2(old[j]);
-        const f2 t = mul2(mul2(o, o), four2);
+        const f2 t = mul_half2(old[j], hmul2(old[j], four));
         const f2 u = red2(t, nm, im, mg.plus, mg.minus);
         const f2 v = fma2(r, from_half2(w[j]), mul2(u, pack2(sp[j].c[0], sp[j].c[1])));
         x[j] = to_half2(red2(v, nm, im, mg.plus, mg.minus));
@@ -960,8 +970,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(32 * ChainShape<N>::
 // operand in TMEM: the next one replaces it when its product's last sums are in,
 // so a product's residues wait in registers; B's residues, needed again for the
 // next square, are kept in shared memory (what does not fit, in TMEM).
-// 38912 numbers of 2136 bits: 22.9 ms against 25.8 ms in two single waves (58368
-// of 712 bits: 5.0 against 5.7), the f32 pipe 68 % busy, the tensor cores 47 %.
+// 38912 numbers of 2136 bits: 22.3 ms against 24.4 ms in two single waves (58368
+// of 712 bits: 4.6 against 5.4), the f32 pipe 68 % busy, the tensor cores 47 %.
 // Reading the next chunk's sums while a chunk's residues are computed changed
 // nothing (24.9 ms).
 template <uint32_t N, uint32_t T>
