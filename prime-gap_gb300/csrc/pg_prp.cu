@@ -368,8 +368,8 @@ struct PrpPlan {
 // Where the residue form is the faster one, in ms for 16 numbers and for 19456
 // (limbs, residues): 200 bits 0.21, 0.32 and 0.44, 0.51; 256 bits 0.46, 0.39 and
 // 1.21, 0.61; 712 bits 1.61, 1.74 and 4.94, 2.07 (5000 numbers: 2.15, 1.85); 1100
-// bits 4.36, 3.58; 1400 bits 6.33, 5.31 and 29.9, 6.7; 2136 bits 16.0, 11.6 and 105,
-// 12.9; 2838 bits (9001 numbers) 106, 30.  So from two limbs per lane on; with two or three chunks of slots and
+// bits 4.36, 3.58; 1400 bits 6.33, 5.01 and 29.9, 5.7; 2136 bits 16.0, 11.1 and 105,
+// 12.3; 2838 bits (9001 numbers) 106, 26.  So from two limbs per lane on; with two or three chunks of slots and
 // fewer than three limbs per lane only for enough numbers to fill the limb form.
 bool rns_pays(uint32_t bits, uint64_t max_items) {
     const uint32_t n = rns_chunks(bits);

@@ -619,16 +619,25 @@ __device__ __forceinline__ f2 red_sum2(f2 lo, f2 hi, f2 neg_m, f2 inv_m, f2 magi
     return add2(fma2(q, neg_m, hi), lo);
 }
 
-// The sums of one chunk to residues, 8 slots of a lane.  w: the number's own
-// constants, four: 1 or 4 (the squared doubling) in both halves.
+// The sums of C chunks to residues, 8 slots of a lane each.  w: the number's own
+// constants, four: 1 or 4 (the squared doubling) in both halves.  A chain of some
+// 20 dependent operations per pair of slots: two chunks at once keep eight going (with one
+// store and one arrival per block: 1100 bits 3.9 -> 3.2 ms, 1750 bits 8.3 -> 7.5 for
+// one pair, 2838 bits 27.8 -> 24.9).
 struct Magic {
     f2 plus, minus;
 };
-__device__ __forceinline__ void residues_a(const SlotPair *sp, const uint32_t (&lo)[8], const uint32_t (&hi)[8],
-                                           f2 rank2, const uint32_t (&w)[4], uint32_t four, const Magic &mg,
-                                           uint32_t (&x)[4]) {
+template <uint32_t C>
+__device__ __forceinline__ void residues_a(const SlotPair *chunk, const uint32_t (&lo2)[2][8],
+                                           const uint32_t (&hi2)[2][8], f2 rank2, const uint32_t (&w2)[2][4],
+                                           uint32_t four, const Magic &mg, uint32_t (&x2)[2][4], uint32_t first = 0) {
 #pragma unroll
-    for (uint32_t j = 0; j < 4; j++) {
+    for (uint32_t i = 0; i < 4 * C; i++) {
+        const uint32_t h = first + (i & (C - 1)), j = i / C;  // the chunks' pairs in turn
+        const SlotPair *sp = chunk + 16 * h;
+        const auto &lo = lo2[h], &hi = hi2[h];
+        const auto &w = w2[h];
+        auto &x = x2[h];
         const f2 nm = pack2(sp[j].neg_m[0], sp[j].neg_m[1]), im = pack2(sp[j].inv_m[0], sp[j].inv_m[1]);
         const f2 l = fma2(rank2, pack2(sp[j].c[0], sp[j].c[1]), pack2u(lo[2 * j], lo[2 * j + 1]));
         const f2 r = red_sum2(l, pack2u(hi[2 * j], hi[2 * j + 1]), nm, im, mg.plus, mg.minus);
@@ -637,11 +646,18 @@ __device__ __forceinline__ void residues_a(const SlotPair *sp, const uint32_t (&
         x[j] = to_half2(red2(v, nm, im, mg.plus, mg.minus));
     }
 }
-__device__ __forceinline__ void residues_b(const SlotPair *sp, const uint32_t (&lo)[8], const uint32_t (&hi)[8],
-                                           const uint32_t (&old)[4], const uint32_t (&w)[4], uint32_t four,
-                                           const Magic &mg, uint32_t (&x)[4]) {
+template <uint32_t C>
+__device__ __forceinline__ void residues_b(const SlotPair *chunk, const uint32_t (&lo2)[2][8],
+                                           const uint32_t (&hi2)[2][8], const uint32_t (&old2)[2][4],
+                                           const uint32_t (&w2)[2][4], uint32_t four, const Magic &mg,
+                                           uint32_t (&x2)[2][4], uint32_t first = 0) {
 #pragma unroll
-    for (uint32_t j = 0; j < 4; j++) {
+    for (uint32_t i = 0; i < 4 * C; i++) {
+        const uint32_t h = first + (i & (C - 1)), j = i / C;
+        const SlotPair *sp = chunk + 16 * h;
+        const auto &lo = lo2[h], &hi = hi2[h];
+        const auto &w = w2[h], &old = old2[h];
+        auto &x = x2[h];
         const f2 nm = pack2(sp[j].neg_m[0], sp[j].neg_m[1]), im = pack2(sp[j].inv_m[0], sp[j].inv_m[1]);
         const f2 r = red_sum2(pack2u(lo[2 * j], lo[2 * j + 1]), pack2u(hi[2 * j], hi[2 * j + 1]), nm, im, mg.plus,
                               mg.minus);
@@ -672,7 +688,7 @@ struct ChainArgs {
 // Up to seven chunks the matrices stay in shared memory and both A operands (of
 // the product under way and of the next) lie in TMEM in full.  Above, the
 // matrices' blocks go round a ring, copied from L2 ahead of each product (2838
-// bits: 10.0 us a step; 9001 numbers 29.7 ms where the limb form takes 106), and the
+// bits: 8.8 us a step; 9001 numbers 26 ms where the limb form takes 106), and the
 // chunks from the eighth on have one place in TMEM: their residues are written
 // when the product's last sums are in, and B's (needed again for the next square)
 // are kept in shared memory.
@@ -762,7 +778,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(32 * ChainShape<N>::
             tmem_st4(lanes + x_at(0, c) + 4 * wg, x);
             if (c >= S::kTwice) kept[(c - S::kTwice) * 512] = v;
             tmem_wait_st();
-            arrive(done0 + 8 * c);
+            // one arrival for the two chunks of a block (the late ones have their own)
+            if (c % 2 == 1 || c + 1 >= S::kTwice) arrive(done0 + 8 * (c >= S::kTwice ? c : c & ~1u));
         }
         const Magic mg{pack2(kMagic, kMagic), pack2(-kMagic, -kMagic)};
         uint32_t seq = 0;  // blocks seen
@@ -771,52 +788,101 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(32 * ChainShape<N>::
             const uint4 v = __ldg(p + at0 + 512 * c);
             w[0] = v.x, w[1] = v.y, w[2] = v.z, w[3] = v.w;
         };
-        // One product's sums to the residues of the next: blocks of two chunks (8 slots each
-        // per thread), the numbers' constants loaded a block ahead.
-        const auto product = [&](const uint4 *nums, const uint4 *next, uint32_t (&cw)[2][4], uint32_t to,
-                                 bool rank_too, auto &&residues) {
+        uint32_t lo[2][8], hi[2][8], rk = 0;
+        const auto fetch = [&](uint32_t b, bool rank_too) {
+            const bool two = 2 * b + 1 < N;
+            const uint32_t acc = lanes + kAcc + 128 * (seq & 1) + 8 * wg, hi_at = two ? 64 : 32;
+            mbar_wait(smem_addr(&s_full[seq & 1]), (seq >> 1) & 1, gone);
+            fence_after();
+            tmem_ld8(lo[0], acc);
+            tmem_ld8(hi[0], acc + hi_at);
+            if (two) {
+                tmem_ld8(lo[1], acc + 32);
+                tmem_ld8(hi[1], acc + hi_at + 32);
+            }
+            if (rank_too) tmem_ld1(rk, acc - 8 * wg);
+        };
+        // One product's sums to the residues of the next, a block of two chunks (8 slots each
+        // per thread) at a time.  The numbers' constants are loaded a block ahead; the next
+        // block's sums are on their way while this one's residues are stored.
+        uint32_t cw[2][4];
+        load(a.num_a, 0, cw[0]);
+        if (N > 1) load(a.num_a, 1, cw[1]);
+        f2 rank2 = 0;
+        const auto product = [&](auto in_b, uint32_t four, uint32_t step) {
+            constexpr bool kB = decltype(in_b)::value;
+            constexpr uint32_t to = kB ? 0 : 1;  // parity of the product that these residues go to
+            const uint4 *const nums = kB ? a.num_b : a.num_a, *const next = kB ? a.num_a : a.num_b;
+            uint4 *const dump = kB && step + kRnsDumps >= a.steps
+                                    ? a.dumps + (a.steps - 1 - step) * a.dump_stride + at0
+                                    : nullptr;
             [[maybe_unused]] uint32_t late[N - S::kTwice + 1][4];
-#pragma unroll 1
-            for (uint32_t b = 0; b < kBlocks; b++, seq++) {
-                const bool two = 2 * b + 1 < N;
-                const uint32_t acc = lanes + kAcc + 128 * (seq & 1) + 8 * wg, hi_at = two ? 64 : 32;
-                mbar_wait(smem_addr(&s_full[seq & 1]), (seq >> 1) & 1, gone);
-                fence_after();
-                uint32_t lo[2][8], hi[2][8], x[2][4];
-                tmem_ld8(lo[0], acc);
-                tmem_ld8(hi[0], acc + hi_at);
-                if (two) {
-                    tmem_ld8(lo[1], acc + 32);
-                    tmem_ld8(hi[1], acc + hi_at + 32);
+            const auto block = [&](uint32_t b, auto chunks) {
+                constexpr uint32_t C = decltype(chunks)::value;
+                uint32_t x[2][4];
+                [[maybe_unused]] uint32_t old[2][4];
+                if constexpr (kB) {
+#pragma unroll
+                    for (uint32_t h = 0; h < C; h++) {
+                        const uint32_t c = 2 * b + h;
+                        if (c < S::kTwice) {
+                            tmem_ld4(old[h], lanes + x_at(0, c) + 4 * wg);
+                        } else {
+                            const uint4 v = kept[(c - S::kTwice) * 512];
+                            old[h][0] = v.x, old[h][1] = v.y, old[h][2] = v.z, old[h][3] = v.w;
+                        }
+                    }
                 }
-                uint32_t rk = 0;
-                if (b == 0 && rank_too) tmem_ld1(rk, acc - 8 * wg);
                 tmem_wait_ld(lo[0], hi[0], rk);
-                if (two) tmem_wait_ld(lo[1], hi[1], rk);
-                arrive(free0 + 8 * (seq & 1));
-                residues(2 * b, lo[0], hi[0], rk, cw[0], x[0]);
-                const bool now0 = 2 * b < S::kTwice, now1 = two && 2 * b + 1 < S::kTwice;
-                if (now0) tmem_st4(lanes + x_at(to, 2 * b) + 4 * wg, x[0]);
-                if constexpr (N > 8)
-                    if (2 * b == 8) late[1][0] = x[0][0], late[1][1] = x[0][1], late[1][2] = x[0][2], late[1][3] = x[0][3];
+                if constexpr (C == 2) tmem_wait_ld(lo[1], hi[1], rk);
+                if constexpr (kB) {
+#pragma unroll
+                    for (uint32_t h = 0; h < C; h++)
+                        if (2 * b + h < S::kTwice) tmem_wait_ld(old[h]);
+                }
+                if constexpr (kBlocks > 2) arrive(free0 + 8 * (seq & 1));
+                seq++;
+                if (!kB && b == 0) rank2 = rank_of(rk);
+                constexpr uint32_t kAtOnce = N == 8 ? 1 : C;  // (eight chunks: it would spill)
+#pragma unroll
+                for (uint32_t h = 0; h < C; h += kAtOnce) {
+                    if constexpr (kB)
+                        residues_b<kAtOnce>(kc.b + (32 * b + 4 * wg), lo, hi, old, cw, four, mg, x, h);
+                    else
+                        residues_a<kAtOnce>(kc.a + (32 * b + 4 * wg), lo, hi, rank2, cw, four, mg, x, h);
+                }
+#pragma unroll
+                for (uint32_t h = 0; h < C; h++) {
+                    const uint32_t c = 2 * b + h;
+                    const uint4 v = make_uint4(x[h][0], x[h][1], x[h][2], x[h][3]);
+                    if (c < S::kTwice) tmem_st4(lanes + x_at(to, c) + 4 * wg, x[h]);
+                    if constexpr (N > 7) {
+                        if (c == 7) late[0][0] = v.x, late[0][1] = v.y, late[0][2] = v.z, late[0][3] = v.w;
+                        if constexpr (N > 8)
+                            if (c == 8) late[1][0] = v.x, late[1][1] = v.y, late[1][2] = v.z, late[1][3] = v.w;
+                    }
+                    if constexpr (kB) {
+                        if (c >= S::kTwice) kept[(c - S::kTwice) * 512] = v;
+                        if (dump) dump[512 * c] = v;
+                    }
+                }
                 // the next block's constants, or the next product's first
-                const uint4 *from = b + 1 < kBlocks ? nums : next;
-                const uint32_t at = b + 1 < kBlocks ? 2 * b + 2 : 0;
-                load(from, at, cw[0]);
-                if (two) residues(2 * b + 1, lo[1], hi[1], rk, cw[1], x[1]);
-                if (now0) {
+                const bool more = b + 1 < kBlocks;
+                const uint32_t at = more ? 2 * b + 2 : 0;
+                load(more ? nums : next, at, cw[0]);
+                if (at + 1 < N) load(more ? nums : next, at + 1, cw[1]);
+                if (more) fetch(b + 1, false);
+                if (2 * b < S::kTwice) {
                     tmem_wait_st();
                     arrive(done0 + 16 * b);
                 }
-                if (now1) tmem_st4(lanes + x_at(to, 2 * b + 1) + 4 * wg, x[1]);
-                if constexpr (N > 7)
-                    if (2 * b + 1 == 7) late[0][0] = x[1][0], late[0][1] = x[1][1], late[0][2] = x[1][2], late[0][3] = x[1][3];
-                if (at + 1 < N) load(from, at + 1, cw[1]);
-                if (now1) {
-                    tmem_wait_st();
-                    arrive(done0 + 16 * b + 8);
-                }
+            };
+            fetch(0, !kB);
+            if constexpr (N > 1) {
+#pragma unroll 1
+                for (uint32_t b = 0; b < N / 2; b++) block(b, std::integral_constant<uint32_t, 2>{});
             }
+            if constexpr (N % 2 == 1) block(N / 2, std::integral_constant<uint32_t, 1>{});
             if constexpr (N > 7) {  // the last block's sums are in: the product is done with their place
 #pragma unroll
                 for (uint32_t c = 7; c < N; c++) tmem_st4(lanes + x_at(to, c) + 4 * wg, late[c - 7]);
@@ -825,9 +891,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(32 * ChainShape<N>::
                 for (uint32_t c = 7; c < N; c++) arrive(done0 + 8 * c);
             }
         };
-        uint32_t cw[2][4];
-        load(a.num_a, 0, cw[0]);
-        if (N > 1) load(a.num_a, 1, cw[1]);
 #pragma unroll 1
         for (uint32_t step = 0; step < a.steps; step++) {
             // the doubling that the last step's exponent bit asked for, squared
@@ -837,35 +900,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(32 * ChainShape<N>::
                 if (step == 1 || (at & 31) == 31) word = n_limbs[at >> 5];
                 if ((word >> (at & 31)) & 1) four = 0x44004400u;  // 4, 4
             }
-            // sums of xi over B -> x in A -> xi in A
-            f2 rank2 = 0;
-            product(
-                a.num_a, a.num_b, cw, 1, true,
-                [&](uint32_t c, const uint32_t (&lo)[8], const uint32_t (&hi)[8], uint32_t rk, const uint32_t (&w)[4],
-                    uint32_t (&x)[4]) {
-                    if (c == 0) rank2 = rank_of(rk);
-                    residues_a(kc.a + (16 * c + 4 * wg), lo, hi, rank2, w, four, mg, x);
-                });
-            // sums of xi over A -> q in B -> xi in B
-            const bool dump = step + kRnsDumps >= a.steps;
-            uint4 *const to = a.dumps + (a.steps - 1 - step) * a.dump_stride + at0;
-            product(
-                a.num_b, a.num_a, cw, 0, false,
-                [&](uint32_t c, const uint32_t (&lo)[8], const uint32_t (&hi)[8], uint32_t, const uint32_t (&w)[4],
-                    uint32_t (&x)[4]) {
-                    uint32_t old[4];
-                    if (c < S::kTwice) {
-                        tmem_ld4(old, lanes + x_at(0, c) + 4 * wg);
-                        tmem_wait_ld(old);
-                    } else {
-                        const uint4 v = kept[(c - S::kTwice) * 512];
-                        old[0] = v.x, old[1] = v.y, old[2] = v.z, old[3] = v.w;
-                    }
-                    residues_b(kc.b + (16 * c + 4 * wg), lo, hi, old, w, four, mg, x);
-                    const uint4 v = make_uint4(x[0], x[1], x[2], x[3]);
-                    if (c >= S::kTwice) kept[(c - S::kTwice) * 512] = v;
-                    if (dump) to[512 * c] = v;
-                });
+            product(std::false_type{}, four, step);  // sums of xi over B -> x in A -> xi in A
+            product(std::true_type{}, four, step);   // sums of xi over A -> q in B -> xi in B
         }
     } else if (warp == kWarps && rank == 0) {
         const uint32_t one = elect_one();
@@ -888,7 +924,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(32 * ChainShape<N>::
                     multiply_pair(one, d, tmem + x_at(ph, kk / 2) + 8 * (kk & 1), desc + kk * (2 * row / 16), instr, kk);
                 };
                 // the buffer's last sums have been read; the block is there in both CTAs
-                if (seq >= kBuffers) mbar_wait(smem_addr(&s_free[seq & 1]), (seq / kBuffers - 1) & 1, gone);
+                // (up to two blocks: before any of this product's residues were there)
+                if (kBlocks > 2 && seq >= kBuffers)
+                    mbar_wait(smem_addr(&s_free[seq & 1]), (seq / kBuffers - 1) & 1, gone);
                 if constexpr (S::kRing) {
                     mbar_wait(smem_addr(&s_landed[ring]), (seq / kRingSlots) & 1, gone);
                     mbar_wait(smem_addr(&s_peer[ring]), (seq / kRingSlots) & 1, gone);
@@ -897,8 +935,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(32 * ChainShape<N>::
                 if (b == 0) {  // slice by slice, as the residues appear
 #pragma unroll
                     for (uint32_t i = 0; i < N; i++) {
-                        mbar_wait(smem_addr(&s_done[i]), ph & 1, gone);
-                        fence_after();
+                        if (i % 2 == 0 || i >= S::kTwice) {
+                            mbar_wait(smem_addr(&s_done[i]), ph & 1, gone);
+                            fence_after();
+                        }
                         multiply(2 * i);
                         multiply(2 * i + 1);
                     }
@@ -972,8 +1012,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(32 * ChainShape<N>::
 // next square, are kept in shared memory (what does not fit, in TMEM).
 // 38912 numbers of 2136 bits: 22.3 ms against 24.4 ms in two single waves (58368
 // of 712 bits: 4.6 against 5.4), the f32 pipe 68 % busy, the tensor cores 47 %.
-// Reading the next chunk's sums while a chunk's residues are computed changed
-// nothing (24.9 ms).
+// Reading the next sums while residues are computed made it slower here (24.9 ms;
+// two chunks at once 24.1).
 template <uint32_t N, uint32_t T>
 struct TilesShape {
     static constexpr uint32_t K = kSlots * N;
@@ -1098,7 +1138,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             word = limb(next_t, next_step);
             const bool dump = kB && step + kRnsDumps >= a.steps;
             f2 rank2 = 0;
-            uint32_t x[2 * kBlocks][4];
+            uint32_t x[kBlocks][2][4];
 #pragma unroll
             for (uint32_t b = 0; b < kBlocks; b++) {
                 const bool two = 2 * b + 1 < N;
@@ -1122,15 +1162,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                 for (uint32_t h = 0; h < (two ? 2 : 1); h++) {
                     const uint32_t c = 2 * b + h;
                     if (kB) {
-                        uint32_t old[4];
-                        kept(t, c, old);
-                        residues_b(kc.b + (16 * c + 4 * wg), lo[h], hi[h], old, cw[h], four, mg, x[c]);
-                        keep(t, c, x[c]);
+                        uint32_t old[2][4];
+                        kept(t, c, old[h]);
+                        residues_b<1>(kc.b + (32 * b + 4 * wg), lo, hi, old, cw, four, mg, x[b], h);
+                        keep(t, c, x[b][h]);
                         if (dump)
                             a.dumps[(a.steps - 1 - step) * a.dump_stride + at0 + t * kTileStep + 512 * c] =
-                                make_uint4(x[c][0], x[c][1], x[c][2], x[c][3]);
+                                make_uint4(x[b][h][0], x[b][h][1], x[b][h][2], x[b][h][3]);
                     } else {
-                        residues_a(kc.a + (16 * c + 4 * wg), lo[h], hi[h], rank2, cw[h], four, mg, x[c]);
+                        residues_a<1>(kc.a + (32 * b + 4 * wg), lo, hi, rank2, cw, four, mg, x[b], h);
                     }
                     const bool more = b + 1 < kBlocks;
                     const uint32_t at = more ? 2 * b + 2 + h : h;
@@ -1141,7 +1181,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             }
             // the last block's sums are in: every product with the old operand is done
 #pragma unroll
-            for (uint32_t c = 0; c < N; c++) tmem_st4(lanes + t * (K / 2) + 16 * c + 4 * wg, x[c]);
+            for (uint32_t c = 0; c < N; c++) tmem_st4(lanes + t * (K / 2) + 16 * c + 4 * wg, x[c / 2][c % 2]);
             tmem_wait_st();
             arrive(done0 + 8 * t);
         };
