@@ -437,8 +437,9 @@ struct GapSearch {
     uint32_t state;      // kWaiting (for the previous side), kActive, kDone
     uint32_t idx;        // next unknown to test
     uint32_t past;       // 1 past the sieve length
-    uint32_t past_x;     // next distance there
+    uint32_t past_x;     // next distance there (sl + 1 at first)
     uint32_t item_base, item_cnt;
+    uint32_t item_list;  // the first of them that are unknowns, the others past the sieve length
 };
 enum { kWaiting, kActive, kDone };
 
@@ -464,8 +465,10 @@ __global__ void past_kernel(const uint32_t *kp, uint32_t nkp, uint32_t sl, uint3
 }
 
 // A round's candidates, nearest first: spec for each active search and one more
-// for the first `extra` that ask; past the sieve length, the next distances
-// that keep N odd and coprime to K.  A warp per search.
+// for the first `extra` that ask.  Where the unknowns end, the round goes on past
+// the sieve length with the next distances that keep N odd and coprime to K (a
+// round is a whole wave: a search that ends there does not wait for another one).
+// A warp per search.
 __global__ void select_kernel(GapSearch *searches, uint64_t rows, GapLists ls, const uint32_t *centers, uint32_t n,
                               uint32_t spec, uint32_t extra, const uint32_t *kp, uint32_t nkp,
                               const uint32_t *__restrict__ past_bits, uint32_t sl, uint32_t x_limit, PrpItem *items,
@@ -487,7 +490,6 @@ __global__ void select_kernel(GapSearch *searches, uint64_t rows, GapLists ls, c
         want += __shfl_sync(0xFFFFFFFFu, more, 0);
     }
     const uint32_t nlist = next ? ls.n_next[r] : ls.n_prev[r];
-    if (!st.past) want = min(want, nlist - st.idx);
     unsigned long long base = 0;
     if (lane == 0 && want) base = atomicAdd(n_items, (unsigned long long)want);
     base = __shfl_sync(0xFFFFFFFFu, base, 0);
@@ -495,12 +497,13 @@ __global__ void select_kernel(GapSearch *searches, uint64_t rows, GapLists ls, c
         if (lane == 0) atomicAdd(errors, 1ull);
         return;
     }
-    uint32_t cnt = want;
-    if (!st.past) {
+    uint32_t cnt = st.past ? 0u : min(want, nlist - st.idx);
+    st.item_list = cnt;
+    if (cnt) {
         const uint32_t *lst = ls.dist + ls.start[r] + (next ? ls.n_prev[r] : 0u) + st.idx;
-        for (uint32_t j = lane; j < want; j += 32) items[base + j] = PrpItem{(uint32_t)r, sign * (int32_t)lst[j]};
-    } else {
-        cnt = 0;
+        for (uint32_t j = lane; j < cnt; j += 32) items[base + j] = PrpItem{(uint32_t)r, sign * (int32_t)lst[j]};
+    }
+    if (cnt < want) {
         uint32_t x = st.past_x;
         while (cnt < want && x < x_limit) {
             // 1024 distances, 32 a lane (32 past the bitmap, one a lane): those
@@ -574,11 +577,10 @@ __global__ void resolve_kernel(GapSearch *searches, uint64_t rows, GapLists ls, 
     const bool next = e & 1;
     const uint32_t nlist = next ? ls.n_next[r] : ls.n_prev[r];
     if (first == 0xFFFFFFFFu) {
-        if (!st.past) {
-            st.idx += st.item_cnt;
-            if (st.idx >= nlist) st.past = 1, st.past_x = sl + 1;
-        }
+        st.idx += st.item_list;
+        if (st.idx >= nlist) st.past = 1;
     } else {
+        if (first >= st.item_list) st.past = 1;
         const int32_t xs = items[st.item_base + first].x;
         const uint32_t x = (uint32_t)(xs < 0 ? -xs : xs);
         const uint32_t tests = st.past ? nlist : st.idx + first + 1u;
