@@ -116,6 +116,15 @@ def _hbm_peak() -> tuple[float, str]:
         return 6800.0, "of fallback (6.8 TB/s)"
 
 
+def _tensor_peak() -> tuple[float, str]:
+    """Measured dense 16-bit tensor rate (FLOP/s), or the fallback figure."""
+    f = ROOT / "MEASURED_PEAKS.json"
+    try:
+        return float(json.loads(f.read_text())["bf16_tflops"]) * 1e12, "of measured (MEASURED_PEAKS.json bf16_tflops)"
+    except (OSError, KeyError, ValueError):
+        return 1.9e15, "of fallback (1.9 PFLOP/s)"
+
+
 def _traffic_per_launch() -> float | None:
     if not PROFILE_TRAFFIC.exists():
         return None
@@ -701,6 +710,8 @@ def run_ingest(args, rank, world, local):
     return 0
 
 
+# widest numbers of one, two, ... chunks of 32 residue slots (the probable-prime tests)
+RNS_WIDTHS = (360, 735, 1103, 1463, 1813, 2147, 2462, 2747, 2900)
 PRP_MIN_MERIT = 18.0  # gap_test's default --min-merit (gap_common.h:49)
 PRP_SAMPLE_ROWS = 64  # rows of the all-core reference arm (16 for the one-core baseline)
 
@@ -793,15 +804,15 @@ def run_prp(args, rank, world, local):
         for _ in range(2):
             prep.prp_gaps(min_merit=PRP_MIN_MERIT, one_side_skip=True)
         prepared_ms = (time.perf_counter() - t) / 2 * 1e3
-    peak = sieve.int_peak()
-    # roofline: Montgomery products of n limbs, 2n^2 32-bit multiply-adds
-    # (64-bit results: two IMAD issue slots each) per product, one product per
-    # bit of N, over every test launched
+    # roofline: per test and bit of N two base extensions, each a product with a
+    # matrix of k x 2k f16 (k residue slots: 32 for every step of the widths that
+    # the slots hold), over every test launched
     import prp_oracle as po
 
-    n = st["limbs"]
     bits = po.primorial_k(job["p"], job["d"]).bit_length() + int(max(lists["m"])).bit_length()
-    ops = launched / args.steps * bits * 2 * n * n * 2
+    k = 32 * next(i + 1 for i, b in enumerate(RNS_WIDTHS) if bits <= b)
+    ops = launched / args.steps * bits * 2 * (2 * k * 2 * k)
+    tensor_peak, tensor_source = _tensor_peak()
     cpu = None
     if not args.no_cpu:
         c = _prp_cpu_sample(lists, job, 1, rows=16)
@@ -819,10 +830,11 @@ def run_prp(args, rank, world, local):
                    "value_is": "lists on the host to gaps on the host"},
         "prp_tests_per_s": counted / args.steps / dt, "prp_launched_per_s": launched / args.steps / dt,
         "rounds_per_step": rounds / args.steps, "from_prepared_job_ms": prepared_ms,
-        "roofline": {"kernel": f"prp_kernel<{n // 8}>", "bound": "int", "achieved": ops / dt, "peak": peak,
-                     "unit": "int ops/s", "frac": ops / dt / peak, "traffic": None,
-                     "peak_source": "measured live: IMAD microbenchmark (pgs_int_peak)"},
-        "cpu_baseline": cpu, "clocks": clock_info, "gpu_launches": args.steps * (2 + 3 * rounds // args.steps),
+        "roofline": {"kernel": f"chain_tiles_kernel<{k // 32}>, chain_kernel<{k // 32}>", "bound": "tensor",
+                     "achieved": ops / dt, "peak": tensor_peak, "unit": "FLOP/s", "frac": ops / dt / tensor_peak,
+                     "traffic": None, "peak_source": tensor_source,
+                     "note": "the f32 pipe, which turns the products' sums into residues, is the busier one"},
+        "cpu_baseline": cpu, "clocks": clock_info, "gpu_launches": args.steps * (4 + 6 * rounds // args.steps),
         "e2e": {"value": value, "unit": "m/s", "h2d_bytes_per_step": rows * 24 + 4 * int(len(lists["dist"])),
                 "d2h_bytes_per_step": rows * 20},
     }

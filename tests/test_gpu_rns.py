@@ -20,8 +20,8 @@ def _numbers(rng, bits, count):
 
 
 # the last widths of one to nine chunks of 32 slots and the ones after them
-@pytest.mark.parametrize("bits", [252, 253, 367, 368, 741, 742, 1107, 1108, 1465, 1466, 1812, 1813, 2146, 2147,
-                                  2461, 2462, 2748, 2749, 2895, 2910])
+@pytest.mark.parametrize("bits", [252, 253, 360, 361, 735, 736, 1103, 1104, 1463, 1464, 1813, 1814, 2147, 2148,
+                                  2462, 2463, 2747, 2748, 2900, 2901])
 def test_rns_widths(sieve, bits):
     rng = random.Random(bits)
     nums = _numbers(rng, bits, 20) + [(1 << bits) - 1, (1 << (bits - 1)) + 1]
