@@ -316,7 +316,7 @@ __device__ __forceinline__ uint64_t slot_at(uint32_t chunks, uint64_t number, ui
 
 enum { kFlagRun = 0, kFlagComposite = 1, kFlagOther = 2 };
 
-// Remainder below 2m of v < 2^29 by m, for chains that only need it small.
+// Remainder below 2m (3m for v above 2^31) of v by m, where it only has to be small.
 __device__ __forceinline__ uint32_t mod_lazy(uint32_t v, uint32_t m, uint32_t inv32) {
     return v - __umulhi(v, inv32) * m;
 }
@@ -347,8 +347,7 @@ __device__ bool near_widest(const uint32_t *n, int top, uint32_t bits, double a_
 // A prime m of base A that divides N leaves no inverse there.  N can still be a
 // pseudoprime only if 2^(N-1) = 1 mod m; then the chain runs mod N/m (the
 // exponent stays N's) and the verdict looks at both.
-// Bound by the remainders' Horner chains (two multiplies per 16 bits): about 2 %
-// of the chain's time.
+// Bound by the remainders' multiplies, one per 16 bits, number and modulus.
 constexpr uint32_t kSetupNumbers = 8;
 __global__ void setup_kernel(const __grid_constant__ RnsSlots p, uint32_t chunks, uint32_t bits, double a_mant,
                              int a_exp, uint32_t limbs, const uint32_t *__restrict__ bases,
@@ -365,24 +364,26 @@ __global__ void setup_kernel(const __grid_constant__ RnsSlots p, uint32_t chunks
     const uint64_t padded = ((n_items + kRnsTile - 1) / kRnsTile + kRnsGroup - 1) * kRnsTile;
     const uint64_t first = (uint64_t)blockIdx.x * kSetupNumbers;
     if (first >= padded) return;
+    // the numbers' limbs, together; then a thread per number adds its offset
+    for (uint32_t e = threadIdx.x; e < kSetupNumbers * limbs; e += blockDim.x) {
+        const uint32_t g = e / limbs, w = e % limbs;
+        if (first + g < n_items) s_n[g][w] = bases[(uint64_t)items[first + g].row * limbs + w];
+    }
+    __syncthreads();
     if (threadIdx.x < kSetupNumbers) {
         const uint32_t g = threadIdx.x;
         const uint64_t i = first + g;
         long long q = 0;
         uint32_t f = kFlagComposite;
         if (i < n_items) {
-            const PrpItem it = items[i];
-            const uint32_t *src = bases + (uint64_t)it.row * limbs;
-            uint32_t *dst = nums + i * limbs;
-            int64_t carry = it.x;
+            int64_t carry = items[i].x;
             int top = -1;
             for (uint32_t w = 0; w < limbs; w++) {
-                const int64_t v = (int64_t)src[w] + carry;
-                const uint32_t lo = (uint32_t)v;
+                const uint32_t was = s_n[g][w];
+                const int64_t v = (int64_t)was + carry;
+                if (carry) s_n[g][w] = (uint32_t)v;
                 carry = v >> 32;
-                s_n[g][w] = lo;
-                dst[w] = lo;
-                if (lo) top = (int)w;
+                if ((uint32_t)v) top = (int)w;
             }
             f = near_widest(s_n[g], top, bits, a_mant, a_exp, q) ? kFlagRun : kFlagOther;
         }
@@ -391,13 +392,34 @@ __global__ void setup_kernel(const __grid_constant__ RnsSlots p, uint32_t chunks
         s_divide[g] = 0, s_by[g] = 1, s_out[g] = 0;
     }
     __syncthreads();
+    for (uint32_t e = threadIdx.x; e < kSetupNumbers * limbs; e += blockDim.x) {
+        const uint32_t g = e / limbs, w = e % limbs;
+        if (first + g < n_items) nums[(first + g) * limbs + w] = s_n[g][w];
+    }
     const uint32_t t = threadIdx.x;
     const uint32_t ma = p.ma[t], mb = p.mb[t];
     const uint32_t ia = inv32_of(ma), ib = inv32_of(mb);
     const uint32_t ainv = inverse_small(p.ab[t], mb);
-    const auto slots = [&](uint32_t g) {
+    // the 8 numbers mod this thread's two moduli: sums of 16-bit digits times the
+    // powers of 2^16, which the numbers share (remainders every 8 digits: below 2^32)
+    uint32_t ra[kSetupNumbers], rb[kSetupNumbers];
+#pragma unroll
+    for (uint32_t g = 0; g < kSetupNumbers; g++) ra[g] = rb[g] = 0;
+    uint32_t pa = ma > 1, pb = mb > 1;
+    for (uint32_t w = 0; w < limbs; w++) {
+        const uint32_t qa = mod_small(pa << 16, ma, ia), qb = mod_small(pb << 16, mb, ib);
+        const bool reduce = (w & 3) == 3;
+#pragma unroll
+        for (uint32_t g = 0; g < kSetupNumbers; g++) {
+            const uint32_t v = s_n[g][w], lo = v & 0xFFFFu, hi = v >> 16;
+            ra[g] += lo * pa + hi * qa;
+            rb[g] += lo * pb + hi * qb;
+            if (reduce) ra[g] = mod_lazy(ra[g], ma, ia), rb[g] = mod_lazy(rb[g], mb, ib);
+        }
+        pa = mod_small(qa << 16, ma, ia), pb = mod_small(qb << 16, mb, ib);
+    }
+    const auto slots = [&](uint32_t g, uint32_t ra, uint32_t rb) {
         const uint64_t at = slot_at(chunks, first + g, t);
-        const uint32_t ra = limbs_mod(s_n[g], limbs, ma, ia), rb = limbs_mod(s_n[g], limbs, mb, ib);
         int ca = 0;
         if (ma > 1 && ra == 0) {
             uint32_t r = limbs_mod(s_n[g], limbs, ma - 1, inv32_of(ma - 1));
@@ -418,9 +440,11 @@ __global__ void setup_kernel(const __grid_constant__ RnsSlots p, uint32_t chunks
         const uint32_t d = mod_small(gb + mb - mod_small(qm * nb, mb, ib), mb, ib);
         state[at] = __float2half_rn((float)balance(mod_small(d * ab, mb, ib), mb));
     };
+#pragma unroll
     for (uint32_t g = 0; g < kSetupNumbers; g++) {
         if (s_f[g] == kFlagRun) {
-            slots(g);
+            const uint32_t a = mod_lazy(ra[g], ma, ia), b = mod_lazy(rb[g], mb, ib);
+            slots(g, mod_small(a, ma, ia), mod_small(b, mb, ib));
         } else {  // an all-zero lane
             const uint64_t at = slot_at(chunks, first + g, t);
             num_a[at] = num_b[at] = state[at] = __half(0.0f);
@@ -445,7 +469,7 @@ __global__ void setup_kernel(const __grid_constant__ RnsSlots p, uint32_t chunks
         }
         __syncthreads();
         const uint32_t by = s_by[g];
-        if (s_f[g] == kFlagRun) slots(g);
+        if (s_f[g] == kFlagRun) slots(g, limbs_mod(s_n[g], limbs, ma, ia), limbs_mod(s_n[g], limbs, mb, ib));
         __syncthreads();
         if (t == 0 && s_divide[g]) s_f[g] = kFlagOther;  // another factor of A in N / m
         if (t == 0) s_by[g] = by, s_out[g] = 0;
