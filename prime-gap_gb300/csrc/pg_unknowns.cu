@@ -22,13 +22,31 @@ namespace {
 
 constexpr uint64_t kChunk = 256;  // text bytes per thread when finding line ends
 
+// Calls at(i) for each newline of chunk c, 16 bytes a load (chunks lie on 256-byte
+// boundaries of the text, which starts on one: a byte a load took 35 us for 2.3 MB).
+template <typename F>
+__device__ __forceinline__ void newlines(const char *__restrict__ text, uint64_t len, uint64_t c, F &&at) {
+    const uint64_t b = c * kChunk, e = min(b + kChunk, len);
+    uint64_t i = b;
+    if (((uintptr_t)text & 15u) == 0)
+        for (; i + 16 <= e; i += 16) {
+            const uint4 v = *reinterpret_cast<const uint4 *>(text + i);
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (uint32_t k = 0; k < 4; k++)
+                for (uint32_t m = __vcmpeq4(w[k], 0x0A0A0A0Au) & 0x01010101u; m; m &= m - 1)
+                    at(i + 4 * k + ((uint32_t)__ffs(m) - 1) / 8);
+        }
+    for (; i < e; i++)
+        if (text[i] == '\n') at(i);
+}
+
 __global__ void count_lines_kernel(const char *__restrict__ text, uint64_t len, uint64_t *counts,
                                    uint64_t nchunks) {
     const uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= nchunks) return;
-    const uint64_t b = c * kChunk, e = min(b + kChunk, len);
     uint64_t n = 0;
-    for (uint64_t i = b; i < e; i++) n += text[i] == '\n';
+    newlines(text, len, c, [&](uint64_t) { n++; });
     counts[c] = n;
 }
 
@@ -36,13 +54,11 @@ __global__ void line_ends_kernel(const char *__restrict__ text, uint64_t len, co
                                  uint64_t nchunks, uint64_t rows, uint64_t *line_end) {
     const uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= nchunks) return;
-    const uint64_t b = c * kChunk, e = min(b + kChunk, len);
     uint64_t k = offsets[c];
-    for (uint64_t i = b; i < e; i++)
-        if (text[i] == '\n') {
-            if (k < rows) line_end[k] = i;
-            k++;
-        }
+    newlines(text, len, c, [&](uint64_t i) {
+        if (k < rows) line_end[k] = i;
+        k++;
+    });
 }
 
 // istream-like reads inside one line [p, end)
@@ -87,6 +103,10 @@ struct ParseDev {
     const uint32_t *dist_tab;  // their distances, ascending
     uint32_t nq;               // odd primes of d
     uint32_t q[16], kq[16];    // the primes and K mod each
+    // per prime and residue r a bit for each live distance that is r mod the prime
+    // (words of them at masks + mask_at[t] + r * words; nullptr: too many)
+    const uint32_t *masks;
+    uint32_t mask_at[16], words;
     // per row
     uint64_t *m, *body, *total;
     uint32_t *n_prev, *n_next;
@@ -127,6 +147,112 @@ __global__ void headers_kernel(ParseDev pd) {
 }
 
 __device__ __forceinline__ bool is_digit(char c) { return c >= '0' && c <= '9'; }
+
+// The masks of ParseDev: a thread per prime of d and live distance.
+__global__ void residue_masks_kernel(ParseDev pd, uint32_t *masks) {
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x, t = blockIdx.y;
+    if (k >= pd.H) return;
+    const uint32_t r = pd.dist_tab[k] % pd.q[t];
+    atomicOr(&masks[pd.mask_at[t] + r * pd.words + (k >> 5)], 1u << (k & 31));
+}
+
+// Bodies of bitcompressed rows (gap_common.cpp:1212-1288), a warp per row and a
+// word of 32 live offsets per lane: over the live offsets in increasing x that are
+// not multiples of an odd prime of d for this m, one flag bit each, 7 per byte; a
+// clear bit is an unknown.  The low side runs x = SL - dist (farthest first), then
+// the high side x = SL + dist.  Which offsets have a flag comes a word at a time
+// from the masks; a lane's first flag from a scan over the words before.  (An
+// offset per lane, with a remainder by each prime of d, took 319 us for 7893 rows
+// of 1511#/2190, SL 20000.)
+__global__ void flags_kernel(ParseDev pd, const uint64_t *__restrict__ start, uint32_t *__restrict__ dist) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t row = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (row >= pd.rows) return;
+    const uint64_t b = pd.body[row], e = pd.line_end[row];
+    if (b == 0) return;  // the header failed (flagged)
+    const unsigned char *raw = (const unsigned char *)pd.text + b;
+    const uint64_t nbytes = e - b, m = pd.m[row], room = pd.total[row];
+    uint32_t *out = dist + start[row];
+    const uint32_t W = pd.words;
+    // x = SL -+ d is a multiple of q (with m) where m*K +- d = 0: d = +-m*K mod q;
+    // lane t < nq keeps prime t's mask of the low and the high side
+    uint32_t low = 0, high = 0;
+    if (lane < pd.nq) {
+        const uint32_t q = pd.q[lane], mk = (uint32_t)((m % q) * pd.kq[lane] % q);
+        low = pd.mask_at[lane] + mk * W;
+        high = pd.mask_at[lane] + (mk ? q - mk : 0u) * W;
+    }
+    // flags of word w of a side, and its unknowns once its first flag's index is known
+    const auto flagged = [&](uint32_t w, bool hi) {
+        uint32_t f = w < W ? (32 * w + 32 <= pd.H ? 0xFFFFFFFFu : (1u << (pd.H - 32 * w)) - 1u) : 0u;
+        for (uint32_t t = 0; t < pd.nq; t++) {
+            const uint32_t at = __shfl_sync(0xffffffffu, hi ? high : low, t);
+            if (w < W) f &= ~pd.masks[at + w];
+        }
+        return f;
+    };
+    const auto scan = [&](uint32_t c, uint32_t &all) {
+        uint32_t v = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t u = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= (uint32_t)o) v += u;
+        }
+        all = __shfl_sync(0xffffffffu, v, 31);
+        return v - c;
+    };
+    const auto unknowns = [&](uint32_t f, uint32_t idx, bool hi) {
+        uint32_t um = 0;
+        uint64_t byte = idx / 7;
+        uint32_t bit = idx % 7;
+        uint32_t cur = f && byte < nbytes ? raw[byte] : 0x7Fu;
+        while (f) {
+            const uint32_t k = hi ? (uint32_t)__ffs(f) - 1 : 31u - (uint32_t)__clz(f);
+            f &= ~(1u << k);
+            if (bit == 7) {
+                bit = 0;
+                byte++;
+                cur = byte < nbytes ? raw[byte] : 0x7Fu;
+            }
+            if (((cur >> bit) & 1u) == 0) um |= 1u << k;
+            bit++;
+        }
+        return um;
+    };
+    // low side, farthest first (words and bits downwards): counted, then written
+    // nearest first from its end; then the high side after it
+    uint32_t np = 0, bit_idx = 0, found = 0;
+    for (int pass = 0; pass < 3; pass++) {
+        const bool hi = pass == 2;
+        if (pass < 2) bit_idx = 0;
+        found = 0;
+        for (uint32_t w0 = 0; w0 < W; w0 += 32) {
+            const uint32_t i = w0 + lane, w = i < W ? (hi ? i : W - 1 - i) : W;
+            const uint32_t f = flagged(w, hi);
+            uint32_t flags, all;
+            const uint32_t idx = bit_idx + scan((uint32_t)__popc(f), flags);
+            uint32_t um = unknowns(f, idx, hi);
+            uint32_t j = found + scan((uint32_t)__popc(um), all);
+            if (pass > 0) {
+                while (um) {
+                    const uint32_t k = hi ? (uint32_t)__ffs(um) - 1 : 31u - (uint32_t)__clz(um);
+                    um &= ~(1u << k);
+                    const uint64_t at = hi ? (uint64_t)np + j : (uint64_t)(np - 1 - j);
+                    if (at < room) out[at] = pd.dist_tab[32 * w + k];
+                    j++;
+                }
+            }
+            bit_idx += flags;
+            found += all;
+        }
+        if (pass == 0) np = found;
+    }
+    if (lane == 0) {
+        pd.n_prev[row] = np;
+        pd.n_next[row] = found;
+        if ((uint64_t)np + found != room || (uint64_t)(bit_idx + 6) / 7 != nbytes) flag(pd, row);
+    }
+}
 
 // One warp per line.
 __global__ void bodies_kernel(ParseDev pd, const uint64_t *__restrict__ start, uint32_t *__restrict__ dist) {
@@ -333,8 +459,8 @@ int parse_device_text_packed(pgs_ctx *ctx, const HostJob &h, const char *d_text,
                              PackedLists &pk) {
     const uint64_t rows = h.valid_mi.size();
     const uint64_t nchunks = (len + pg::kChunk - 1) / pg::kChunk;
-    DevBuf counts, offs, tmp, line_end, body, tot, err, misc, dist_tab;
-    DevBuf *bufs[] = {&counts, &offs, &tmp, &line_end, &body, &tot, &err, &misc, &dist_tab};
+    DevBuf counts, offs, tmp, line_end, body, tot, err, misc, dist_tab, masks;
+    DevBuf *bufs[] = {&counts, &offs, &tmp, &line_end, &body, &tot, &err, &misc, &dist_tab, &masks};
     for (DevBuf *b : bufs) b->pool = &ctx->dpool;
     pk.block.pool = &ctx->dpool;
     auto cleanup = [&] {
@@ -421,8 +547,26 @@ int parse_device_text_packed(pgs_ctx *ctx, const HostJob &h, const char *d_text,
             return PGS_EINVAL;
         }
         if (e == cudaSuccess && !bad) {
-            pg::bodies_kernel<<<pg::grid(rows * 32, 256), 256, 0, s>>>(pd, pk.start, pk.dist);
-            e = cudaGetLastError();
+            // masks of up to 64 MB (the primes of d times the live offsets, in bits)
+            pd.words = (h.H + 31) / 32;
+            uint64_t words = 0;
+            for (uint32_t t = 0; t < pd.nq; t++) words += (uint64_t)pd.q[t] * pd.words;
+            if (h.job.compression == 2 && h.H > 0 && words <= (16u << 20)) {
+                e = masks.ensure(words * 4 + 4);
+                if (e == cudaSuccess) e = cudaMemsetAsync(masks.p, 0, words * 4 + 4, s);
+                pd.masks = masks.as<uint32_t>();
+                for (uint32_t t = 0, at = 0; t < pd.nq; t++) {
+                    pd.mask_at[t] = at;
+                    at += pd.q[t] * pd.words;
+                }
+                if (e == cudaSuccess && pd.nq)
+                    pg::residue_masks_kernel<<<dim3((h.H + 255) / 256, pd.nq), 256, 0, s>>>(pd, masks.as<uint32_t>());
+                if (e == cudaSuccess)
+                    pg::flags_kernel<<<pg::grid(rows * 32, 256), 256, 0, s>>>(pd, pk.start, pk.dist);
+            } else {
+                pg::bodies_kernel<<<pg::grid(rows * 32, 256), 256, 0, s>>>(pd, pk.start, pk.dist);
+            }
+            if (e == cudaSuccess) e = cudaGetLastError();
             if (e == cudaSuccess) e = cudaMemcpyAsync(&bad, err.p, 8, cudaMemcpyDeviceToHost, s);
             if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         }
