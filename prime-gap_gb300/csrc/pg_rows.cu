@@ -123,67 +123,10 @@ __global__ void __launch_bounds__(kRowThreads) rows_kernel(RowsDev rd, uint32_t 
     // 3. merge with the large-prime bits and compact, one warp per row
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     const uint32_t H = job.half_cols;
-    if (rd.compression == 2) {
-        // Bitcompressed rows (combined_sieve.cpp:1327-1385): over the offsets
-        // in increasing X that are coprime to K and to every prime of d
-        // (live and not in the d-prime pattern), the composite flags, 7 per
-        // byte with bit 7 set.  The byte list goes to the row's list slot.
-        for (uint32_t j = warp; j < nrows; j += nwarps) {
-            const uint32_t row = r0 + j;
-            const uint32_t *grow = job.comp + (uint64_t)row * job.pitch;
-            uint8_t *bytes = (uint8_t *)(rd.lists + (uint64_t)row * 2 * H);
-            uint32_t unk = 0, nbytes = 0, bit = 0, b = 0x80;
-            for (uint32_t side = 0; side < 2; side++) {
-                for (uint32_t h0 = 0; h0 < H; h0 += 32) {
-                    // side 0 walks its columns backwards: increasing X
-                    const uint32_t k = h0 + lane;
-                    bool fc = false, composite = false;
-                    if (k < H) {
-                        const uint32_t h = side ? k : H - 1 - k;
-                        const uint32_t d = rd.dist[h];
-                        const uint32_t x = side ? sl + d : sl - d;
-                        const uint32_t hx = (x - x_par) >> 1;
-                        const uint32_t pat = (s_pat[j * nbw + (hx >> 5)] >> (hx & 31)) & 1;
-                        const uint32_t sb = (sh[j * nbw + (hx >> 5)] >> (hx & 31)) & 1;
-                        const uint32_t col = side * job.side_pad + h;
-                        const uint32_t gb = (grow[col >> 5] >> (col & 31)) & 1;
-                        fc = !pat;
-                        composite = (sb | gb) != 0;
-                    }
-                    const uint32_t fcm = __ballot_sync(0xFFFFFFFFu, fc);
-                    const uint32_t cm = __ballot_sync(0xFFFFFFFFu, composite);
-                    unk += __popc(fcm & ~cm);
-                    if (lane == 0) {
-                        uint32_t m = fcm;
-                        while (m) {
-                            const uint32_t i = __ffs(m) - 1;
-                            m &= m - 1;
-                            b |= ((cm >> i) & 1u) << bit;
-                            if (++bit == 7) {
-                                bytes[nbytes++] = (uint8_t)b;
-                                b = 0x80;
-                                bit = 0;
-                            }
-                        }
-                    }
-                }
-            }
-            if (lane == 0) {
-                if (bit) bytes[nbytes++] = (uint8_t)b;
-                rd.counts[2 * row] = unk;
-                rd.counts[2 * row + 1] = nbytes;
-                const uint64_t m = job.mstart + s_mi[j];
-                // "m : U B || <bytes>\n"
-                rd.row_bytes[row] = ndigits(m) + ndigits(unk) + ndigits(nbytes) + 9 + nbytes;
-            }
-        }
-        return;
-    }
-    // Plain and RLE rows.  The large-prime marks (one bit per live offset,
-    // in distance order on each side) go into the row's bitmap over offset
-    // indexes, one lane per word of marks; then the live offsets left
-    // unmarked are read off that bitmap a word per lane, nearest to SL first
-    // on each side, each distance following from its index.
+    // The large-prime marks (one bit per live offset, in distance order on
+    // each side) go into the row's bitmap over offset indexes, one lane per
+    // word of marks; then the live offsets are read off that bitmap a word
+    // per lane.
     const uint32_t side_words = job.side_pad >> 5;
     const uint32_t hs = (sl - x_par + 1) >> 1;  // indexes below hs: x < SL
     for (uint32_t j = warp; j < nrows; j += nwarps) {
@@ -205,6 +148,69 @@ __global__ void __launch_bounds__(kRowThreads) rows_kernel(RowsDev rd, uint32_t 
         }
         __syncwarp();
         uint32_t *list = rd.lists + (uint64_t)row * 2 * H;
+        if (rd.compression == 2) {
+            // Bitcompressed rows (combined_sieve.cpp:1327-1385): over the
+            // offsets in increasing X that are coprime to K and to every prime
+            // of d (live and not in the d-prime pattern), the composite flags, 7
+            // per byte with bit 7 set, to the row's list slot.  32 words at a
+            // time: their flags are packed in the 64 words of bitmap and pattern
+            // that they were read from (at most 8 bytes for each word's 32 flags,
+            // 5 and a bit are needed), whole bytes written from there.  (One lane
+            // packing the flags of 32 offsets at a time: the rows stage of 8290
+            // m of 2003#/30030, SL 16500, took 0.47 ms; whole jobs of d = 1 and 57195 m of
+            // 1009#, SL 17000: 6.9 ms, 3.2 now.)
+            uint8_t *bytes = (uint8_t *)list;
+            uint32_t *pm = s_pat + j * nbw;
+            uint32_t unk = 0, nbytes = 0, carry = 0, carry_bits = 0;
+            for (uint32_t k0 = 0; k0 < nbw; k0 += 32) {
+                const uint32_t n = min(32u, nbw - k0), w = k0 + lane;
+                uint32_t f = 0, c = 0;
+                if ((uint32_t)lane < n) {
+                    f = rd.live[w] & ~pm[w];
+                    c = f & bm[w];
+                }
+                unk += __popc(f & ~c);
+                __syncwarp();
+                if ((uint32_t)lane < n) bm[w] = 0, pm[w] = 0;
+                __syncwarp();
+                const auto stage = [&](uint32_t i) { return i < n ? bm + k0 + i : pm + k0 + (i - n); };
+                uint32_t incl = __popc(f);
+#pragma unroll
+                for (uint32_t off = 1; off < 32; off <<= 1) {
+                    const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, off);
+                    if ((uint32_t)lane >= off) incl += t;
+                }
+                const uint32_t total = carry_bits + __shfl_sync(0xFFFFFFFFu, incl, 31);
+                const uint32_t i0 = carry_bits + incl - __popc(f);
+                if (lane == 0 && carry) atomicOr(stage(0), carry);
+                while (c) {
+                    const uint32_t low = c & (0u - c);
+                    c ^= low;
+                    const uint32_t i = i0 + __popc(f & (low - 1)), at = i / 7 * 8 + i % 7;
+                    atomicOr(stage(at >> 5), 1u << (at & 31));
+                }
+                __syncwarp();
+                const uint32_t full = total / 7;
+                for (uint32_t k = lane; k < full; k += 32)
+                    bytes[nbytes + k] = (uint8_t)(0x80u | (*stage(k >> 2) >> (8 * (k & 3))));
+                carry_bits = total - 7 * full;
+                carry = carry_bits ? (*stage(full >> 2) >> (8 * (full & 3))) & 0x7Fu : 0u;
+                nbytes += full;
+                __syncwarp();
+            }
+            unk = __reduce_add_sync(0xFFFFFFFFu, unk);
+            if (lane == 0) {
+                if (carry_bits) bytes[nbytes++] = (uint8_t)(0x80u | carry);
+                rd.counts[2 * row] = unk;
+                rd.counts[2 * row + 1] = nbytes;
+                const uint64_t m = job.mstart + s_mi[j];
+                // "m : U B || <bytes>\n"
+                rd.row_bytes[row] = ndigits(m) + ndigits(unk) + ndigits(nbytes) + 9 + nbytes;
+            }
+            continue;
+        }
+        // Plain and RLE rows: the live offsets left unmarked, nearest to SL
+        // first on each side, each distance following from its index.
         uint64_t body = 0;
         uint32_t cnt_side[2];
         for (uint32_t side = 0; side < 2; side++) {
