@@ -135,7 +135,6 @@ PG_HD float u64_trunc24(uint64_t v) {
 PG_HD float u64_to_f32_rz(uint64_t v) {
     const uint32_t hi = (uint32_t)(v >> 32), lo = (uint32_t)v;
 #if defined(__CUDA_ARCH__)
-    if (hi == 0) return __uint2float_rz(lo);
     return __fadd_rz(__fmul_rz(__uint2float_rz(hi), 4294967296.0f), __uint2float_rz(lo));
 #else
     if (hi == 0) return u32_to_f32_rz(lo);
@@ -206,7 +205,8 @@ PG_HD void udiv2_32(uint32_t n1, uint32_t n2, uint32_t d, uint32_t &q1, uint32_t
 // Two 32-bit quotients by one divisor with the quotients themselves taken in
 // single precision (the bound of udiv2_64 below): one remainder test each
 // instead of two, for two more conversions.
-PG_HD void udiv2f_32(uint32_t n1, uint32_t n2, uint32_t d, uint32_t &q1, uint32_t &q2, int skew = 0) {
+PG_HD void udiv2f_32(uint32_t n1, uint32_t n2, uint32_t d, uint32_t &q1, uint32_t &q2, int skew = 0,
+                     bool *wide = nullptr) {
     float rf = rcp_approx(u32_to_f32_rz(d));
 #if !defined(__CUDA_ARCH__)
     for (; skew > 0; skew--) rf = nextafterf(rf, 2.0f);
@@ -217,7 +217,8 @@ PG_HD void udiv2f_32(uint32_t n1, uint32_t n2, uint32_t d, uint32_t &q1, uint32_
     const float rs = mul_f32_rz(rf, 0.999998092651367188f);  // 1 - 2^-19
     const uint32_t a = f32_to_u32_rz(mul_f32_rz(u32_to_f32_rz(n1), rs));
     const uint32_t b = f32_to_u32_rz(mul_f32_rz(u32_to_f32_rz(n2), rs));
-    if ((a | b) >= (1u << 17)) {
+    if (wide) *wide = (a | b) >= (1u << 17);
+    if (!wide && (a | b) >= (1u << 17)) {
         q1 = n1 / d;
         q2 = n2 / d;
         return;
@@ -234,7 +235,8 @@ PG_HD void udiv2f_32(uint32_t n1, uint32_t n2, uint32_t d, uint32_t &q1, uint32_
 // never exceeds q = floor(n/d) and, while q0 < 2^17 (hence n/d < 2^18), is
 // at least q - 1: one remainder test finishes it.  A larger q0 takes the
 // exact division.
-PG_HD void udiv2_64(uint64_t n1, uint64_t n2, uint64_t d, uint64_t &q1, uint64_t &q2, int skew = 0) {
+PG_HD void udiv2_64(uint64_t n1, uint64_t n2, uint64_t d, uint64_t &q1, uint64_t &q2, int skew = 0,
+                    bool *wide = nullptr) {
     float rf = rcp_approx(u64_to_f32_rz(d));
 #if !defined(__CUDA_ARCH__)
     for (; skew > 0; skew--) rf = nextafterf(rf, 2.0f);
@@ -245,7 +247,8 @@ PG_HD void udiv2_64(uint64_t n1, uint64_t n2, uint64_t d, uint64_t &q1, uint64_t
     const float rs = mul_f32_rz(rf, 0.999998092651367188f);  // 1 - 2^-19, exact in single precision
     const uint32_t a = f32_to_u32_rz(mul_f32_rz(u64_to_f32_rz(n1), rs));
     const uint32_t b = f32_to_u32_rz(mul_f32_rz(u64_to_f32_rz(n2), rs));
-    if ((a | b) >= (1u << 17)) {
+    if (wide) *wide = (a | b) >= (1u << 17);
+    if (!wide && (a | b) >= (1u << 17)) {
         q1 = n1 / d;
         q2 = n2 / d;
         return;
@@ -823,55 +826,62 @@ struct Entry {
 // moduli the true first entry is below p < 2^32 - 1, so a limit above 2^32 - 1
 // never triggers and clamping it there changes nothing.
 template <typename T>
-PG_HD void quot2(T n1, T n2, T d, T &q1, T &q2) {
+PG_HD void quot2(T n1, T n2, T d, T &q1, T &q2, bool *wide = nullptr) {
     if constexpr (sizeof(T) == 4) {
-        udiv2f_32(n1, n2, d, q1, q2);
+        udiv2f_32(n1, n2, d, q1, q2, 0, wide);
     } else {
-        udiv2_64(n1, n2, d, q1, q2);
+        udiv2_64(n1, n2, d, q1, q2, 0, wide);
     }
 }
 
-template <typename T>
+// kPrime: p is prime, so the tie does not happen and is not tested for.  kExact:
+// wide quotients are divided exactly in the loop.
+template <typename T, bool kPrime = false, bool kExact = !kPrime>
 PG_HD Entry<T> first_entry(T p, T a, T w, T y0, uint64_t t_lim = ~0ull) {
     const bool mir = a < p - a;
     T up = mir ? p - a : a, dn = p - up, kp = 1, kn = 1;
     T y = !mir ? y0 : (y0 < w ? w - 1 - y0 : p - (y0 - (w - 1)));
     const T lim = t_lim < (uint64_t)(T)~(T)0 ? (T)t_lim : (T)~(T)0;
     T rem = lim;
+    bool wide = false;
     // Every level with q >= 1 lowers its big gap by at least small >= 1, so
     // the loop ends; q == 0 only for a tie up == dn (not for a prime modulus).
+    // Straight-line levels with one way out each: a lane that has no entry left
+    // to make (f >= q) or is past the limit (rem = 0) does the same operations as
+    // the others, since some lane of a warp nearly always has one; a quotient too
+    // wide for the single-precision form (about one level in 2^17) leaves too, and
+    // the search starts again with exact divisions.  Large-prime stage with branches
+    // and now: 4.78, 4.31 ms (1e5 m of 1511#/2190 to 2e9), 0.72, 0.66 ms (200 m of
+    // 907#/2190 to 9e8), 53.2, 48.8 ms (1e5 m of 3001#/2190 to 1e10, 64-bit primes).
     for (;;) {
-        if (up < w) break;  // up > dn: both below w
-        {
+        {  // up > dn, up >= w (p > 2w at first)
             const T C = up + dn, n1 = (C - w) < (up - 1) ? (C - w) : (up - 1);
             T q, f;
-            quot2<T>(n1, C - 1 - y, dn, q, f);
-            if (q == 0) break;
-            if (f < q) {
-                const T m = q - f, dt = m * kn;
-                if (dt >= rem) return {(uint64_t)(lim - rem) + dt, y, {kp, up, kn, dn}};
-                y -= m * dn;
-                rem -= dt;
-            }
+            quot2<T>(n1, C - 1 - y, dn, q, f, kExact ? nullptr : &wide);
+            if (!kPrime && q == 0) break;
+            const T m = f < q ? q - f : (T)0, dt = m * kn;
+            const bool on = dt < rem;
+            y -= m * dn;
+            rem = on ? rem - dt : (T)0;
             up -= q * dn;
             kp += q * kn;
+            if (!on | (dn < w) | (!kExact && wide)) break;  // dn > up: both below w
         }
-        if (dn < w) break;  // dn > up: both below w
         {
             const T C = up + dn, n1 = (C - w) < (dn - 1) ? (C - w) : (dn - 1);
             T q, f;
-            quot2<T>(n1, C - 1 - y, up, q, f);
-            if (q == 0) break;
-            if (f < q) {
-                const T dt = kn + f * kp;
-                if (dt >= rem) return {(uint64_t)(lim - rem) + dt, y, {kp, up, kn, dn}};
-                y -= dn - f * up;
-                rem -= dt;
-            }
+            quot2<T>(n1, C - 1 - y, up, q, f, kExact ? nullptr : &wide);
+            if (!kPrime && q == 0) break;
+            const T dt = f < q ? kn + f * kp : (T)0;
+            const bool on = dt < rem;
+            y -= f < q ? dn - f * up : (T)0;
+            rem = on ? rem - dt : (T)0;
             dn -= q * up;
             kn += q * kp;
+            if (!on | (up < w) | (!kExact && wide)) break;  // up > dn: both below w
         }
     }
+    if (!kExact && wide) return first_entry<T, kPrime, true>(p, a, w, y0, t_lim);
     uint64_t t = lim - rem;
     if (y >= w) {  // last level: [0, up + dn) -> [0, w) by one wrap
         y -= dn;

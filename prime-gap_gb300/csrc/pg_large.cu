@@ -180,7 +180,7 @@ __device__ __forceinline__ void large_group(const JobDev &job, const Marker &mar
     const uint64_t minc = job.walk.jmax;  // the walk runs over j, not mi
     uint32_t items = 0;
     if (has) {
-        const Entry<T> e = first_entry<T>(p, step, w, t0, minc);
+        const Entry<T> e = first_entry<T, true>(p, step, w, t0, minc);
         if (e.t < minc && e.y < w) {
             const uint64_t bound = rotation_steps_bound<T>(e.t, minc, e.g, p);
             bool local = true;
@@ -401,7 +401,7 @@ __global__ void __launch_bounds__(kLargeThreads)
         const T p = (T)(base + off[i]);
         T step, t0;
         walk_inputs<T, kIn>(job, kl.limb, nlimbs, p, a_in, b, i, step, t0);
-        const Entry<T> e = first_entry<T>(p, step, w, t0, minc);
+        const Entry<T> e = first_entry<T, true>(p, step, w, t0, minc);
         if (e.t >= minc || e.y >= w) continue;
         const uint64_t bound = rotation_steps_bound<T>(e.t, minc, e.g, p);
         const ThreeGap<uint32_t> g32 = gap32(e.g, (uint32_t)minc);

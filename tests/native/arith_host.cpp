@@ -187,6 +187,15 @@ void ah_first_entry(uint64_t p, uint64_t a, uint64_t w, uint64_t y0, uint64_t *o
     }
 }
 
+// first_entry of a prime modulus, with an early stop at t_lim: out as below
+void ah_first_entry_prime(uint64_t p, uint64_t a, uint64_t w, uint64_t y0, uint64_t t_lim, uint64_t *out6) {
+    auto put = [&](auto e) {
+        out6[0] = e.t, out6[1] = e.y, out6[2] = e.g.kp, out6[3] = e.g.up, out6[4] = e.g.kn, out6[5] = e.g.dn;
+    };
+    if (p < 0xFFFFFFFFull) put(pg::first_entry<uint32_t, true>((uint32_t)p, (uint32_t)a, (uint32_t)w, (uint32_t)y0, t_lim));
+    else put(pg::first_entry<uint64_t, true>(p, a, w, y0, t_lim));
+}
+
 // first_entry with an early stop at t_lim: out = {t, y, kp, up, kn, dn}
 void ah_first_entry_lim(uint64_t p, uint64_t a, uint64_t w, uint64_t y0, uint64_t t_lim,
                         uint64_t *out6) {

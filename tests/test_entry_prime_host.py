@@ -1,0 +1,54 @@
+"""first_entry of a prime modulus (the host build of the device header), the form
+without the tie test, against a walk of the residues and against the general
+form with the same early stop."""
+from __future__ import annotations
+
+import ctypes
+import random
+
+import pytest
+
+import pgo
+from test_arith_host import ah  # noqa: F401 (the host library as a fixture)
+
+u64 = ctypes.c_uint64
+
+
+def _call(fn, *args):
+    out = (u64 * 6)()
+    fn(*[u64(a) for a in args], out)
+    return list(out)
+
+
+@pytest.mark.parametrize("lo", [50, 1000, 60_000, 1_000_003])
+def test_prime_entry_walk(ah, lo):  # noqa: F811
+    rng = random.Random(lo)
+    for p in pgo.primes(lo, lo + 400)[1:]:
+        for _ in range(20):
+            w = rng.randrange(2, max(3, p // 2))
+            if p <= 2 * w:
+                continue
+            a, y0 = rng.randrange(1, p), rng.randrange(p)
+            t, y = 0, y0
+            while y >= w:
+                t, y = t + 1, (y + a) % p
+            got = _call(ah.ah_first_entry_prime, p, a, w, y0, 2**63)
+            assert got[:2] == [t, y], (p, a, w, y0)
+
+
+@pytest.mark.parametrize("bits", [20, 27, 31, 32, 33, 40, 45])
+def test_prime_entry_equals_general_form(ah, bits):  # noqa: F811
+    rng = random.Random(bits)
+    primes = pgo.primes(2**bits - 3000, 2**bits - 1)
+    for _ in range(4000):
+        p = rng.choice(primes)
+        w = rng.choice([2, 3, rng.randrange(2, 2**10), rng.randrange(2, min(p // 2, 2**17))])
+        a = rng.choice([1, 2, w, p - 1, p // 2, rng.randrange(1, p), rng.randrange(1, p)])
+        y0 = rng.choice([0, w - 1, w, p - 1, rng.randrange(p)])
+        t_lim = rng.choice([2**63, 1, 5000, 50_000, rng.randrange(1, p)])
+        full = _call(ah.ah_first_entry, p, a, w, y0)
+        got = _call(ah.ah_first_entry_prime, p, a, w, y0, t_lim)
+        if full[0] < t_lim:
+            assert got == full, (p, a, w, y0, t_lim)
+        else:
+            assert got[0] >= t_lim, (p, a, w, y0, t_lim)
