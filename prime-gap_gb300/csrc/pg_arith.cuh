@@ -851,36 +851,38 @@ PG_HD Entry<T> first_entry(T p, T a, T w, T y0, uint64_t t_lim = ~0ull) {
     // the others, since some lane of a warp nearly always has one; a quotient too
     // wide for the single-precision form (about one level in 2^17) leaves too, and
     // the search starts again with exact divisions.  Large-prime stage with branches
-    // and now: 4.78, 4.31 ms (1e5 m of 1511#/2190 to 2e9), 0.72, 0.66 ms (200 m of
-    // 907#/2190 to 9e8), 53.2, 48.8 ms (1e5 m of 3001#/2190 to 1e10, 64-bit primes).
+    // and now: 4.78, 4.22 ms (1e5 m of 1511#/2190 to 2e9), 0.72, 0.64 ms (200 m of
+    // 907#/2190 to 9e8), 53.2, 48.6 ms (1e5 m of 3001#/2190 to 1e10, 64-bit primes).
+    T z = p - 1 - y;  // C - 1 - y: what the second quotient divides
     for (;;) {
         {  // up > dn, up >= w (p > 2w at first)
-            const T C = up + dn, n1 = (C - w) < (up - 1) ? (C - w) : (up - 1);
+            const T cw = up + dn - w, n1 = cw < up - 1 ? cw : up - 1;
             T q, f;
-            quot2<T>(n1, C - 1 - y, dn, q, f, kExact ? nullptr : &wide);
+            quot2<T>(n1, z, dn, q, f, kExact ? nullptr : &wide);
             if (!kPrime && q == 0) break;
-            const T m = f < q ? q - f : (T)0, dt = m * kn;
-            const bool on = dt < rem;
-            y -= m * dn;
-            rem = on ? rem - dt : (T)0;
+            f = f < q ? f : q;  // q - f subtractions of dn
+            const T dt = (q - f) * kn;
+            rem = (rem > dt ? rem : dt) - dt;
+            z -= f * dn;
             up -= q * dn;
             kp += q * kn;
-            if (!on | (dn < w) | (!kExact && wide)) break;  // dn > up: both below w
+            if ((rem == 0) | (dn < w) | (!kExact && wide)) break;  // dn > up: both below w
         }
         {
-            const T C = up + dn, n1 = (C - w) < (dn - 1) ? (C - w) : (dn - 1);
+            const T cw = up + dn - w, n1 = cw < dn - 1 ? cw : dn - 1;
             T q, f;
-            quot2<T>(n1, C - 1 - y, up, q, f, kExact ? nullptr : &wide);
+            quot2<T>(n1, z, up, q, f, kExact ? nullptr : &wide);
             if (!kPrime && q == 0) break;
-            const T dt = f < q ? kn + f * kp : (T)0;
-            const bool on = dt < rem;
-            y -= f < q ? dn - f * up : (T)0;
-            rem = on ? rem - dt : (T)0;
-            dn -= q * up;
+            const bool wraps = f < q;
+            const T dt = wraps ? kn + f * kp : (T)0, x = q * up;
+            rem = (rem > dt ? rem : dt) - dt;
+            z += (wraps ? dn - f * up : (T)0) - x;
+            dn -= x;
             kn += q * kp;
-            if (!on | (up < w) | (!kExact && wide)) break;  // up > dn: both below w
+            if ((rem == 0) | (up < w) | (!kExact && wide)) break;  // up > dn: both below w
         }
     }
+    y = up + dn - 1 - z;
     if (!kExact && wide) return first_entry<T, kPrime, true>(p, a, w, y0, t_lim);
     uint64_t t = lim - rem;
     if (y >= w) {  // last level: [0, up + dn) -> [0, w) by one wrap
