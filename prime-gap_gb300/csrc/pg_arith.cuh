@@ -1000,6 +1000,25 @@ PG_HD void return_walk32(uint32_t mi, uint32_t y, const ThreeGap<uint32_t> &g, u
     }
 }
 
+// whole_walk32: return_walk32 of every hit below mi_hi from a hit (mi, y), y < w:
+// mi alone ends it (kp, kn >= 1), so no step is counted.  Large-prime stage with
+// the count and without: 4.22, 4.15 ms (1e5 m of 1511#/2190 to 2e9), 48.6, 48.4 ms
+// (1e5 m of 3001#/2190 to 1e10).
+template <typename Emit>
+PG_HD void whole_walk32(uint32_t mi, uint32_t y, const ThreeGap<uint32_t> &g, uint32_t w, uint32_t mi_hi,
+                        Emit &emit) {
+    const uint32_t up = g.up, dn = g.dn;
+    const uint32_t kp = g.kp < mi_hi ? g.kp : mi_hi, kn = g.kn < mi_hi ? g.kn : mi_hi;
+    const uint32_t kpn = kp + kn < mi_hi ? kp + kn : mi_hi;
+    while (mi < mi_hi) {
+        emit(mi, y, true);
+        const uint32_t a = y + up;
+        const bool near = a < w, wrap = y >= dn;
+        y = near ? a : (wrap ? y - dn : a - dn);
+        mi += near ? kp : (wrap ? kn : kpn);
+    }
+}
+
 // ---------------------------------------------------------------------------
 // hit enumeration
 

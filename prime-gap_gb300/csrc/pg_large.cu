@@ -186,8 +186,8 @@ __device__ __forceinline__ void large_group(const JobDev &job, const Marker &mar
             bool local = true;
             if (bound <= job.direct_steps) {
                 // few steps: walk the rotation here
-                return_walk32((uint32_t)e.t, (uint32_t)e.y, gap32(e.g, (uint32_t)minc), (uint32_t)w,
-                                (uint32_t)minc, (uint32_t)bound, mark);
+                whole_walk32((uint32_t)e.t, (uint32_t)e.y, gap32(e.g, (uint32_t)minc), (uint32_t)w,
+                             (uint32_t)minc, mark);
                 local = false;
             } else if (bound > job.heavy_steps) {
                 // very many steps: one CTA of the heavy kernel takes this prime
@@ -421,7 +421,7 @@ __global__ void __launch_bounds__(kLargeThreads)
                 continue;
             }
         }
-        return_walk32((uint32_t)e.t, (uint32_t)e.y, g32, (uint32_t)w, (uint32_t)minc, (uint32_t)bound, mark);
+        whole_walk32((uint32_t)e.t, (uint32_t)e.y, g32, (uint32_t)w, (uint32_t)minc, mark);
     }
 }
 

@@ -332,6 +332,20 @@ int ah_return_walk_agrees(uint32_t mi, uint32_t y, uint32_t kp, uint32_t up, uin
     return 1;
 }
 
+// Every hit below mi_hi, without a count of steps (whole_walk32) and by circle
+// steps (rotation_walk32, bound steps); returns 1 when the two lists agree.
+int ah_whole_walk_agrees(uint32_t mi, uint32_t y, uint32_t kp, uint32_t up, uint32_t kn, uint32_t dn, uint32_t w,
+                         uint32_t mi_hi, uint32_t bound, uint32_t *buf, size_t cap) {
+    const pg::ThreeGap<uint32_t> g{kp, up, kn, dn};
+    HitList a{buf, cap / 2, 0}, b{buf + cap / 2, cap / 2, 0};
+    pg::rotation_walk32(mi, y, g, w, mi_hi, bound, a);
+    pg::whole_walk32(mi, y, g, w, mi_hi, b);
+    if (a.n != b.n) return 0;
+    for (size_t i = 0; i < a.n && i < cap / 2; i++)
+        if (a.out[i] != b.out[i]) return 0;
+    return 1;
+}
+
 void ah_pow64_128(uint64_t p, int skew, uint64_t *out2) { pg::pow64_128_mod(p, out2[0], out2[1], skew); }
 
 uint64_t ah_neg_inv64(uint64_t p) { return pg::neg_inv64(p); }

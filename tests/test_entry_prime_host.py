@@ -52,3 +52,26 @@ def test_prime_entry_equals_general_form(ah, bits):  # noqa: F811
             assert got == full, (p, a, w, y0, t_lim)
         else:
             assert got[0] >= t_lim, (p, a, w, y0, t_lim)
+
+
+@pytest.mark.parametrize("bits,mi_hi", [(10, 1), (16, 700), (24, 5000), (31, 30_000), (45, 2**31 - 1)])
+def test_whole_walk(ah, bits, mi_hi):  # noqa: F811
+    """Every hit of a direct walk, by circle steps within the bound's count."""
+    u32 = ctypes.c_uint32
+    ah.ah_whole_walk_agrees.argtypes = [u32] * 9 + [ctypes.POINTER(u32), ctypes.c_size_t]
+    rng = random.Random(bits)
+    primes = pgo.primes(2**bits - 900, 2**bits - 1)
+    cap = 1 << 20
+    buf = (u32 * cap)()
+    walked = 0
+    for _ in range(300):
+        p = rng.choice(primes)
+        w = rng.choice([2, 3, max(2, p >> 14), rng.randrange(2, min((p - 1) // 2, 2**17))])
+        hi = min(mi_hi, 100_000 * (p // w))
+        t, y, kp, up, kn, dn = _call(ah.ah_first_entry_prime, p, rng.randrange(1, p), w, rng.randrange(p), hi)
+        if t >= hi or y >= w:
+            continue
+        kp, kn = min(kp, hi), min(kn, hi)
+        assert ah.ah_whole_walk_agrees(t, y, kp, up, kn, dn, w, hi, 2**32 - 1, buf, cap) == 1, (p, w, t, y)
+        walked += 1
+    assert walked > 20
