@@ -834,8 +834,54 @@ PG_HD void quot2(T n1, T n2, T d, T &q1, T &q2, bool *wide = nullptr) {
     }
 }
 
-// kPrime: p is prime, so the tie does not happen and is not tested for.  kExact:
-// wide quotients are divided exactly in the loop.
+// The levels from a circle with up >= w and z = C - 1 - y, which is what the second
+// quotient divides.  kPrime: the modulus is prime, so the tie does not happen and
+// is not tested for.  kExact: wide quotients are divided exactly in the loop.
+// Returns true at the descent's end (both gaps below w, or rem = 0); with kUntil32
+// false as soon as the circle is below 2^32.
+//
+// Every level with q >= 1 lowers its big gap by at least small >= 1, so the loop
+// ends; q == 0 only for a tie up == dn (not for a prime modulus).
+// Straight-line levels with one way out each: a lane that has no entry left
+// to make (f >= q) or is past the limit (rem = 0) does the same operations as
+// the others, since some lane of a warp nearly always has one; a quotient too
+// wide for the single-precision form (about one level in 2^17) leaves too, and
+// the search starts again with exact divisions.  Large-prime stage with branches
+// and now: 4.78, 4.22 ms (1e5 m of 1511#/2190 to 2e9), 0.72, 0.64 ms (200 m of
+// 907#/2190 to 9e8), 53.2, 48.6 ms (1e5 m of 3001#/2190 to 1e10, 64-bit primes).
+template <typename T, bool kPrime, bool kExact, bool kUntil32>
+PG_HD bool entry_levels(T &up, T &dn, T &kp, T &kn, T &z, T &rem, T w, bool &wide) {
+    for (;;) {
+        if (kUntil32 && ((uint64_t)(up + dn) >> 32) == 0) return false;
+        {  // up > dn, up >= w (p > 2w at first)
+            const T cw = up + dn - w, n1 = cw < up - 1 ? cw : up - 1;
+            T q, f;
+            quot2<T>(n1, z, dn, q, f, kExact ? nullptr : &wide);
+            if (!kPrime && q == 0) return true;
+            f = f < q ? f : q;  // q - f subtractions of dn
+            const T dt = (q - f) * kn;
+            rem = (rem > dt ? rem : dt) - dt;
+            z -= f * dn;
+            up -= q * dn;
+            kp += q * kn;
+            if ((rem == 0) | (dn < w) | (!kExact && wide)) return true;  // dn > up: both below w
+        }
+        {
+            const T cw = up + dn - w, n1 = cw < dn - 1 ? cw : dn - 1;
+            T q, f;
+            quot2<T>(n1, z, up, q, f, kExact ? nullptr : &wide);
+            if (!kPrime && q == 0) return true;
+            const bool wraps = f < q;
+            const T dt = wraps ? kn + f * kp : (T)0, x = q * up;
+            rem = (rem > dt ? rem : dt) - dt;
+            z += (wraps ? dn - f * up : (T)0) - x;
+            dn -= x;
+            kn += q * kp;
+            if ((rem == 0) | (up < w) | (!kExact && wide)) return true;  // up > dn: both below w
+        }
+    }
+}
+
 template <typename T, bool kPrime = false, bool kExact = !kPrime>
 PG_HD Entry<T> first_entry(T p, T a, T w, T y0, uint64_t t_lim = ~0ull) {
     const bool mir = a < p - a;
@@ -844,43 +890,30 @@ PG_HD Entry<T> first_entry(T p, T a, T w, T y0, uint64_t t_lim = ~0ull) {
     const T lim = t_lim < (uint64_t)(T)~(T)0 ? (T)t_lim : (T)~(T)0;
     T rem = lim;
     bool wide = false;
-    // Every level with q >= 1 lowers its big gap by at least small >= 1, so
-    // the loop ends; q == 0 only for a tie up == dn (not for a prime modulus).
-    // Straight-line levels with one way out each: a lane that has no entry left
-    // to make (f >= q) or is past the limit (rem = 0) does the same operations as
-    // the others, since some lane of a warp nearly always has one; a quotient too
-    // wide for the single-precision form (about one level in 2^17) leaves too, and
-    // the search starts again with exact divisions.  Large-prime stage with branches
-    // and now: 4.78, 4.22 ms (1e5 m of 1511#/2190 to 2e9), 0.72, 0.64 ms (200 m of
-    // 907#/2190 to 9e8), 53.2, 48.6 ms (1e5 m of 3001#/2190 to 1e10, 64-bit primes).
-    T z = p - 1 - y;  // C - 1 - y: what the second quotient divides
-    for (;;) {
-        {  // up > dn, up >= w (p > 2w at first)
-            const T cw = up + dn - w, n1 = cw < up - 1 ? cw : up - 1;
-            T q, f;
-            quot2<T>(n1, z, dn, q, f, kExact ? nullptr : &wide);
-            if (!kPrime && q == 0) break;
-            f = f < q ? f : q;  // q - f subtractions of dn
-            const T dt = (q - f) * kn;
-            rem = (rem > dt ? rem : dt) - dt;
-            z -= f * dn;
-            up -= q * dn;
-            kp += q * kn;
-            if ((rem == 0) | (dn < w) | (!kExact && wide)) break;  // dn > up: both below w
+    T z = p - 1 - y;
+    if constexpr (sizeof(T) == 8 && kPrime && !kExact) {
+        // A 64-bit modulus has a circle below 2^32 after a pair of levels (below p/2
+        // then: p < 2^33) or a few; the others run in 32 bits.  kp dn + kn up = p
+        // bounds the step costs: below 2^32 while the level's small gap is at least
+        // least = floor(p / 2^32) + 1, as it is in every level but the last when
+        // least <= w; the last one's is tested after it.  Whole levels in 64 bits and
+        // this way, large-prime stage with K mod p: 48.4, 43.4 ms (1e5 m of 3001#/2190
+        // to 1e10), 23.4, 19.4 (30000 m of 503#/210 to 9e9), 10.6, 9.7 (200 m of
+        // 907#/2190 to 6e9).
+        const T least = (p >> 32) + 1;
+        if (least <= w && (t_lim >> 32) == 0) {
+            if (!entry_levels<T, true, false, true>(up, dn, kp, kn, z, rem, w, wide)) {
+                uint32_t up32 = (uint32_t)up, dn32 = (uint32_t)dn, kp32 = (uint32_t)kp, kn32 = (uint32_t)kn;
+                uint32_t z32 = (uint32_t)z, rem32 = (uint32_t)rem;
+                entry_levels<uint32_t, true, false, false>(up32, dn32, kp32, kn32, z32, rem32, (uint32_t)w, wide);
+                up = up32, dn = dn32, kp = kp32, kn = kn32, z = z32, rem = rem32;
+                wide |= (up < dn ? up32 : dn32) < (uint32_t)least;
+            }
+        } else {
+            entry_levels<T, kPrime, kExact, false>(up, dn, kp, kn, z, rem, w, wide);
         }
-        {
-            const T cw = up + dn - w, n1 = cw < dn - 1 ? cw : dn - 1;
-            T q, f;
-            quot2<T>(n1, z, up, q, f, kExact ? nullptr : &wide);
-            if (!kPrime && q == 0) break;
-            const bool wraps = f < q;
-            const T dt = wraps ? kn + f * kp : (T)0, x = q * up;
-            rem = (rem > dt ? rem : dt) - dt;
-            z += (wraps ? dn - f * up : (T)0) - x;
-            dn -= x;
-            kn += q * kp;
-            if ((rem == 0) | (up < w) | (!kExact && wide)) break;  // up > dn: both below w
-        }
+    } else {
+        entry_levels<T, kPrime, kExact, false>(up, dn, kp, kn, z, rem, w, wide);
     }
     y = up + dn - 1 - z;
     if (!kExact && wide) return first_entry<T, kPrime, true>(p, a, w, y0, t_lim);

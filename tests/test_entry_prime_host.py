@@ -75,3 +75,26 @@ def test_whole_walk(ah, bits, mi_hi):  # noqa: F811
         assert ah.ah_whole_walk_agrees(t, y, kp, up, kn, dn, w, hi, 2**32 - 1, buf, cap) == 1, (p, w, t, y)
         walked += 1
     assert walked > 20
+
+
+@pytest.mark.parametrize("bits", [33, 34, 36, 40, 44])
+def test_prime_entry_least_gap(ah, bits):  # noqa: F811
+    """64-bit moduli whose descent ends in tiny gaps (step costs past 2^32) and
+    windows at the line where the circle goes to 32 bits, w = floor(p / 2^32) + 1."""
+    rng = random.Random(1000 + bits)
+    primes = pgo.primes(2**bits - 2000, 2**bits - 1)
+    for _ in range(1500):
+        p = rng.choice(primes)
+        least = (p >> 32) + 1
+        w = max(2, rng.choice([least - 1, least, least + 1, 2 * least, 2**14]))
+        k = rng.randrange(1, min(p, 2**rng.randrange(20, bits)))
+        # k steps come to a small residue: gaps of a few units at the end
+        a = rng.choice([pow(k, -1, p), p - pow(k, -1, p), rng.randrange(1, p)])
+        y0 = rng.randrange(p)
+        t_lim = rng.choice([2**31 - 1, 2**32 - 1, 100_000, 2**33])
+        full = _call(ah.ah_first_entry, p, a, w, y0)
+        got = _call(ah.ah_first_entry_prime, p, a, w, y0, t_lim)
+        if full[0] < t_lim:
+            assert got == full, (p, a, w, y0, t_lim)
+        else:
+            assert got[0] >= t_lim, (p, a, w, y0, t_lim)
