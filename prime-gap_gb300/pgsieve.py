@@ -730,7 +730,22 @@ def _forget_copiers() -> None:
 os.register_at_fork(after_in_child=_forget_copiers)
 
 
-def _copy(src):
+class _Block:
+    """The library's block behind a result, given back once: by free(), or with the
+    last reference where threads may still read it (every slice under way holds one)."""
+
+    def __init__(self, lib, u: Unknowns):
+        self.lib, self.u, self.shared = lib, u, False
+
+    def free(self) -> None:
+        u, self.u = self.u, None
+        if u is not None:
+            self.lib.pgs_unknowns_free(ctypes.byref(u))
+
+    __del__ = free
+
+
+def _copy(src, block: _Block):
     import numpy as np
 
     global _copiers
@@ -742,25 +757,37 @@ def _copy(src):
         _copiers = ThreadPoolExecutor(_COPY_THREADS)
     dst = np.empty_like(src)
     step = -(-len(src) // _COPY_THREADS)
+    parts = range(0, len(src), step)
+
+    def part(i, _):
+        np.copyto(dst[i:i + step], src[i:i + step])
+
+    jobs: list = []
     try:
-        list(_copiers.map(lambda i: np.copyto(dst[i:i + step], src[i:i + step]), range(0, len(src), step)))
-    except RuntimeError:  # the interpreter is shutting down: no more work for threads
-        return src.copy()
+        for i in parts:
+            jobs.append(_copiers.submit(part, i, block))
+    except RuntimeError:  # no more work for threads; one of them may have taken this slice all the same
+        block.shared = True
+        for i in parts[len(jobs):]:
+            part(i, block)
+    for j in jobs:
+        j.result()
     return dst
 
 
 def _unknowns_out(lib, u: Unknowns) -> dict:
     import numpy as np
 
-    try:
-        rows, total = u.rows, u.total
-        arr = np.ctypeslib.as_array
-        return {
-            "m": arr(u.m, (max(rows, 1),))[:rows].copy(),
-            "start": arr(u.start, (max(rows, 1),))[:rows].copy(),
-            "n_prev": arr(u.n_prev, (max(rows, 1),))[:rows].copy(),
-            "n_next": arr(u.n_next, (max(rows, 1),))[:rows].copy(),
-            "dist": _copy(arr(u.dist, (max(total, 1),))[:total]),
-        }
-    finally:
-        lib.pgs_unknowns_free(ctypes.byref(u))
+    block = _Block(lib, u)
+    rows, total = u.rows, u.total
+    arr = np.ctypeslib.as_array
+    out = {
+        "m": arr(u.m, (max(rows, 1),))[:rows].copy(),
+        "start": arr(u.start, (max(rows, 1),))[:rows].copy(),
+        "n_prev": arr(u.n_prev, (max(rows, 1),))[:rows].copy(),
+        "n_next": arr(u.n_next, (max(rows, 1),))[:rows].copy(),
+        "dist": _copy(arr(u.dist, (max(total, 1),))[:total], block),
+    }
+    if not block.shared:
+        block.free()
+    return out
