@@ -492,11 +492,11 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t n) {
 }
 
 // Wait for the barrier's completion of the given parity; gives up after about
-// a second (gone: the caller stops waiting altogether).
+// a second, 2^18 tries of 3.8 us (gone: the caller stops waiting altogether).
 __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, bool &gone) {
     if (gone) return;
     uint32_t ok = 0;
-    for (uint32_t i = 0; i < (1u << 20); i++) {
+    for (uint32_t i = 0; i < (1u << 18); i++) {
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
             "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
@@ -541,6 +541,20 @@ __device__ __forceinline__ void commit_pair(uint32_t one, uint32_t bar) {
             "r"(bar),
         "h"((uint16_t)3), "r"(one)
         : "memory");
+}
+
+// The issuing warp's last act: where one of its waits gave up, the products still in
+// flight end before TMEM is given back.  A commit covers what its own thread issued, so
+// it comes from the lane that issued them, whichever lane gave up.
+__device__ __forceinline__ void end_products(bool gone, uint32_t one, uint32_t bar) {
+    if (!__any_sync(0xFFFFFFFFu, gone)) return;
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar),
+        "r"(one)
+        : "memory");
+    bool late = false;
+    mbar_wait(bar, 0, late);
 }
 
 __device__ __forceinline__ void tmem_ld8(uint32_t (&r)[8], uint32_t addr) {
@@ -778,6 +792,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(32 * ChainShape<N>::
     // chunk c of the A operand of product ph: even ones sum xi of B, odd ones of A
     const auto x_at = [](uint32_t ph, uint32_t c) { return 16 * c + ((ph & 1) && c < S::kTwice ? S::kXb : 0u); };
     bool gone = false;
+    uint32_t one = 0;  // the lane that issues the products
 
     if (warp < kWarps) {
         const uint32_t wg = warp / 4;                           // its 8 slots of each chunk
@@ -928,7 +943,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(32 * ChainShape<N>::
             product(std::true_type{}, four, step);   // sums of xi over A -> q in B -> xi in B
         }
     } else if (warp == kWarps && rank == 0) {
-        const uint32_t one = elect_one();
+        one = elect_one();
         // f16 operands, f32 sums, both K-major, M = 256
         constexpr uint32_t kInstr = (1u << 4) | ((256 / 16) << 24);
         const uint32_t base = smem_addr(smem);
@@ -1009,17 +1024,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(32 * ChainShape<N>::
                 mbar_wait(smem_addr(&s_landed[i % kRingSlots]), (i / kRingSlots) & 1, late);
         }
     }
-    if (gone) {
-        atomicExch(a.error, 1ull);
-        if (warp == kWarps && rank == 0) {  // products still in flight end before TMEM is given back
-            if (lane == 0)
-                asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                                 smem_addr(&s_end))
-                             : "memory");
-            bool late = false;
-            mbar_wait(smem_addr(&s_end), 0, late);
-        }
-    }
+    if (gone) atomicExch(a.error, 1ull);
+    if (warp == kWarps && rank == 0) end_products(gone, one, smem_addr(&s_end));
     fence_before();
     __syncthreads();
     cluster_sync();
@@ -1092,6 +1098,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     fence_after();
     const uint32_t tmem = s_tmem;
     bool gone = false;
+    uint32_t one = 0;  // the lane that issues the products
 
     if (warp < kWarps) {
         const uint32_t wg = warp / 4;                           // its 8 slots of each chunk
@@ -1217,7 +1224,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             for (uint32_t t = 0; t < T; t++) product(std::true_type{}, step, t);
         }
     } else if (rank == 0) {
-        const uint32_t one = elect_one();
+        one = elect_one();
         constexpr uint32_t kInstr = (1u << 4) | ((256 / 16) << 24);
         const uint32_t base = smem_addr(smem);
         uint32_t seq = 0;
@@ -1241,17 +1248,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             }
         }
     }
-    if (gone) {
-        atomicExch(a.error, 1ull);
-        if (warp == kWarps && rank == 0) {  // products still in flight end before TMEM is given back
-            if (lane == 0)
-                asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                                 smem_addr(&s_end))
-                             : "memory");
-            bool late = false;
-            mbar_wait(smem_addr(&s_end), 0, late);
-        }
-    }
+    if (gone) atomicExch(a.error, 1ull);
+    if (warp == kWarps && rank == 0) end_products(gone, one, smem_addr(&s_end));
     fence_before();
     __syncthreads();
     cluster_sync();
