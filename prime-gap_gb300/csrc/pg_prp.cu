@@ -294,8 +294,11 @@ __device__ bool prp2(const Grp &g, const Num<L> &n, const uint32_t *sn) {
     }
 }
 
-// list: the items to test where not all are
-template <int L>
+// kListed: the items to test are the listed ones, if there is a list.  Its own instance:
+// the branch costs some widths up to 11 % (16 numbers of 1463 bits 6.57 ms without it,
+// 7.03 with it; 1788 bits 10.5, 11.6).  At three limbs per lane the instance with it is
+// the faster one (735 bits 1.65, 1.50) and takes all calls.
+template <int L, bool kListed>
 __global__ void __launch_bounds__(kPrpThreads)
     prp_kernel(const uint32_t *__restrict__ bases, const PrpItem *__restrict__ items,
                const uint32_t *__restrict__ list, const unsigned long long *count, uint64_t max_items, uint8_t *__restrict__ result) {
@@ -305,7 +308,7 @@ __global__ void __launch_bounds__(kPrpThreads)
     uint64_t i = (uint64_t)blockIdx.x * kGroups + gi;
     const uint64_t n_items = count ? min((uint64_t)*count, max_items) : max_items;
     if (i >= n_items) return;  // the whole group leaves together
-    if (list) i = list[i];
+    if (kListed && list) i = list[i];
     const PrpItem it = items[i];
     const uint32_t *src = bases + (uint64_t)it.row * (8 * L) + g.t * L;
     Num<L> n;
@@ -324,9 +327,12 @@ cudaError_t launch_prp(int L, const uint32_t *bases, const PrpItem *items, const
                        const unsigned long long *count, uint64_t max_items, uint8_t *result, cudaStream_t s) {
     if (max_items == 0) return cudaSuccess;
     const unsigned blocks = (unsigned)((max_items + kGroups - 1) / kGroups);
-#define PG_PRP_CASE(LL)                                                                               \
-    case LL:                                                                                          \
-        prp_kernel<LL><<<blocks, kPrpThreads, 0, s>>>(bases, items, list, count, max_items, result);  \
+#define PG_PRP_CASE(LL)                                                                                       \
+    case LL:                                                                                                  \
+        if (list || LL == 3)                                                                                  \
+            prp_kernel<LL, true><<<blocks, kPrpThreads, 0, s>>>(bases, items, list, count, max_items, result); \
+        else                                                                                                  \
+            prp_kernel<LL, LL == 3><<<blocks, kPrpThreads, 0, s>>>(bases, items, list, count, max_items, result); \
         break;
     switch (L) {
         PG_PRP_CASE(1)
