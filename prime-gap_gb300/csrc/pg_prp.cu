@@ -383,12 +383,14 @@ bool rns_pays(uint32_t bits, uint64_t max_items) {
     return n == 1 || bits >= 765 || max_items >= 4096;
 }
 
+// The residue form's workspace, some 6 KB per number of 2136 bits, is for a wave of
+// numbers: a longer list goes through it in slices.
 PrpPlan prp_plan(uint32_t bits, uint64_t max_items) {
     PrpPlan p;
     p.bits = bits;
     p.L = limbs_per_lane(bits);
     p.rns = rns_pays(bits, max_items);
-    if (p.rns) p.layout = rns_layout(bits, 8u * (uint32_t)p.L, max_items);
+    if (p.rns) p.layout = rns_layout(bits, 8u * (uint32_t)p.L, rns_slice(bits, max_items), max_items);
     return p;
 }
 
@@ -399,8 +401,12 @@ cudaError_t prp_begin(const PrpPlan &p, void *work, cudaStream_t s) {
 cudaError_t prp_launch(const PrpPlan &p, void *work, const uint32_t *bases, const PrpItem *items,
                        const unsigned long long *count, uint64_t max_items, uint8_t *result, cudaStream_t s) {
     if (!p.rns) return launch_prp(p.L, bases, items, nullptr, count, max_items, result, s);
-    const cudaError_t e = rns_test(p.layout, p.bits, work, bases, items, count, max_items, result, s);
-    if (e != cudaSuccess) return e;
+    for (uint64_t first = 0; first < max_items;) {  // a count: one slice, at most a wave
+        const uint64_t n = count ? max_items : rns_slice(p.bits, max_items - first);
+        const cudaError_t e = rns_test(p.layout, p.bits, work, bases, items, first, count, n, result, s);
+        if (e != cudaSuccess) return e;
+        first += n;
+    }
     return launch_prp(p.L, bases, items, rns_fallback_list(p.layout, work), rns_fallback_count(p.layout, work),
                       max_items, result, s);
 }

@@ -24,21 +24,26 @@ uint32_t rns_chunks(uint32_t bits);
 // tiles (0 where rns_chunks is 0 and full is asked).
 uint64_t rns_wave(uint32_t bits, bool full);
 
-// Device workspace of a call over at most max_items numbers.
+// How many of `left` numbers the next rns_test of a long list takes: one wave.
+uint64_t rns_slice(uint32_t bits, uint64_t left);
+
+// Device workspace of rns_test over at most max_items numbers at a time, all_items
+// in all.
 struct RnsLayout {
     uint32_t chunks, limbs;
     uint64_t tiles;  // of kRnsTile numbers
     size_t matrices, num_a, num_b, state, dumps, nums, quot, flag, factor, list, counters, total;
 };
-RnsLayout rns_layout(uint32_t bits, uint32_t limbs, uint64_t max_items);
+RnsLayout rns_layout(uint32_t bits, uint32_t limbs, uint64_t max_items, uint64_t all_items);
 
-// Tests items[0 .. min(*count, max_items)) (count == nullptr: max_items) and
-// writes result; numbers that this form does not decide (their number at
-// rns_fallback_count, their places at rns_fallback_list, their limbs at
-// rns_numbers) are left for the caller.
+// Tests items[first .. first + min(*count, max_items)) (count == nullptr: max_items)
+// and writes their results; numbers that this form does not decide (how many since
+// first = 0 at rns_fallback_count, their places at rns_fallback_list) are left for
+// the caller.
 cudaError_t rns_begin(const RnsLayout &l, uint32_t bits, void *work, cudaStream_t s);
 cudaError_t rns_test(const RnsLayout &l, uint32_t bits, void *work, const uint32_t *bases, const PrpItem *items,
-                     const unsigned long long *count, uint64_t max_items, uint8_t *result, cudaStream_t s);
+                     uint64_t first, const unsigned long long *count, uint64_t max_items, uint8_t *result,
+                     cudaStream_t s);
 inline const unsigned long long *rns_fallback_count(const RnsLayout &l, void *work) {
     return (const unsigned long long *)((char *)work + l.counters);
 }
