@@ -88,6 +88,7 @@ struct DevicePool {
         cudaError_t e = cudaMalloc(p, n);
         if (e == cudaErrorMemoryAllocation) {
             trim();  // give cached blocks back and retry once
+            cudaGetLastError();  // not left for the next launch's check
             e = cudaMalloc(p, n);
         }
         if (e == cudaSuccess) {

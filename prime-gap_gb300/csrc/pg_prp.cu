@@ -368,7 +368,6 @@ struct PrpPlan {
     uint32_t bits = 0;
     bool rns = false;
     RnsLayout layout{};
-    size_t work_bytes() const { return rns ? layout.total : 0; }
 };
 
 // Where the residue form is the faster one, in ms for 16 numbers and for 19456
@@ -392,6 +391,17 @@ PrpPlan prp_plan(uint32_t bits, uint64_t max_items) {
     p.rns = rns_pays(bits, max_items);
     if (p.rns) p.layout = rns_layout(bits, 8u * (uint32_t)p.L, rns_slice(bits, max_items), max_items);
     return p;
+}
+
+// The residue form's workspace; where the device has no room for it, the limb form
+// takes the call.
+cudaError_t prp_workspace(PrpPlan &p, pgh::DevBuf &work) {
+    if (!p.rns) return cudaSuccess;
+    const cudaError_t e = work.ensure(p.layout.total);
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    p.rns = false;
+    return cudaSuccess;
 }
 
 cudaError_t prp_begin(const PrpPlan &p, void *work, cudaStream_t s) {
@@ -735,7 +745,7 @@ int pgs_prp_test(pgs_ctx *ctx, const uint32_t *limbs, uint32_t n_limbs, size_t c
         dev_rows.push_back(i);
     }
     if (dev_rows.empty()) return PGS_OK;
-    const pg::PrpPlan plan = pg::prp_plan(max_bits, dev_rows.size());
+    pg::PrpPlan plan = pg::prp_plan(max_bits, dev_rows.size());
     const uint32_t n = 8u * (uint32_t)plan.L;
     std::vector<uint32_t> packed(dev_rows.size() * n, 0u);
     std::vector<pg::PrpItem> items(dev_rows.size());
@@ -752,7 +762,7 @@ int pgs_prp_test(pgs_ctx *ctx, const uint32_t *limbs, uint32_t n_limbs, size_t c
     cudaError_t e = upload(d_nums, packed, s);
     if (e == cudaSuccess) e = upload(d_items, items, s);
     if (e == cudaSuccess) e = d_res.ensure(dev_rows.size());
-    if (e == cudaSuccess) e = d_work.ensure(plan.work_bytes());
+    if (e == cudaSuccess) e = pg::prp_workspace(plan, d_work);
     if (e == cudaSuccess) e = pg::prp_begin(plan, d_work.p, s);
     if (e == cudaSuccess)
         e = pg::prp_launch(plan, d_work.p, d_nums.as<uint32_t>(), d_items.as<pg::PrpItem>(), nullptr, dev_rows.size(),
@@ -803,8 +813,7 @@ int prp_gaps_core(pgs_ctx *ctx, const pgs_gap_params *prm, uint64_t rows, const 
     const bool may_skip = prm->one_side_skip != 0;
     const uint64_t searches = 2 * rows;
     const uint64_t limb_round = std::max<uint64_t>(searches, kRoundTarget);
-    const pg::PrpPlan plan = pg::prp_plan(bits, std::max<uint64_t>(limb_round, pg::rns_wave(bits, true)));
-    const uint64_t max_items = plan.rns ? pg::rns_wave(bits, true) : limb_round;
+    pg::PrpPlan plan = pg::prp_plan(bits, std::max<uint64_t>(limb_round, pg::rns_wave(bits, true)));
     const uint32_t n = 8u * (uint32_t)plan.L;
     std::vector<uint32_t> skip(rows, 0u);
     if (prm->one_side_skip) {
@@ -819,7 +828,9 @@ int prp_gaps_core(pgs_ctx *ctx, const pgs_gap_params *prm, uint64_t rows, const 
         cudaStreamSynchronize(s);
         for (DevBuf *b : bufs) b->release();
     };
-    cudaError_t e = upload(d_k, k, s);
+    cudaError_t e = pg::prp_workspace(plan, d_work);
+    const uint64_t max_items = plan.rns ? pg::rns_wave(bits, true) : limb_round;
+    if (e == cudaSuccess) e = upload(d_k, k, s);
     if (e == cudaSuccess) e = upload(d_kp, kprimes, s);
     if (e == cudaSuccess && may_skip) e = upload(d_skip, skip, s);
     if (e == cudaSuccess) e = d_past.ensure(pg::kPastBits / 8);
@@ -829,7 +840,6 @@ int prp_gaps_core(pgs_ctx *ctx, const pgs_gap_params *prm, uint64_t rows, const 
     if (e == cudaSuccess) e = d_res.ensure(max_items);
     if (e == cudaSuccess) e = d_out.ensure(rows * sizeof(pgs_gap_result));
     if (e == cudaSuccess) e = d_ctr.ensure(40);
-    if (e == cudaSuccess) e = d_work.ensure(plan.work_bytes());
     if (e == cudaSuccess) e = pg::prp_begin(plan, d_work.p, s);
     if (e != cudaSuccess) {
         cleanup();
