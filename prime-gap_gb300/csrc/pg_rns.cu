@@ -793,7 +793,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(32 * ChainShape<N>::
     // chunk c of the A operand of product ph: even ones sum xi of B, odd ones of A
     const auto x_at = [](uint32_t ph, uint32_t c) { return 16 * c + ((ph & 1) && c < S::kTwice ? S::kXb : 0u); };
     bool gone = false;
-    uint32_t one = 0;  // the lane that issues the products
 
     if (warp < kWarps) {
         const uint32_t wg = warp / 4;                           // its 8 slots of each chunk
@@ -944,7 +943,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(32 * ChainShape<N>::
             product(std::true_type{}, four, step);   // sums of xi over A -> q in B -> xi in B
         }
     } else if (warp == kWarps && rank == 0) {
-        one = elect_one();
+        const uint32_t one = elect_one();
         // f16 operands, f32 sums, both K-major, M = 256
         constexpr uint32_t kInstr = (1u << 4) | ((256 / 16) << 24);
         const uint32_t base = smem_addr(smem);
@@ -990,6 +989,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(32 * ChainShape<N>::
                 if constexpr (S::kRing) commit_pair(one, smem_addr(&s_empty[ring]));
             }
         }
+        end_products(gone, one, smem_addr(&s_end));
     } else if (S::kRing && warp == kWarps && lane == 0) {
         // the other CTA's half of each block has landed: tell the one that multiplies
         uint32_t peer0;
@@ -1026,7 +1026,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(32 * ChainShape<N>::
         }
     }
     if (gone) atomicExch(a.error, 1ull);
-    if (warp == kWarps && rank == 0) end_products(gone, one, smem_addr(&s_end));
     fence_before();
     __syncthreads();
     cluster_sync();
@@ -1099,7 +1098,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     fence_after();
     const uint32_t tmem = s_tmem;
     bool gone = false;
-    uint32_t one = 0;  // the lane that issues the products
 
     if (warp < kWarps) {
         const uint32_t wg = warp / 4;                           // its 8 slots of each chunk
@@ -1225,7 +1223,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             for (uint32_t t = 0; t < T; t++) product(std::true_type{}, step, t);
         }
     } else if (rank == 0) {
-        one = elect_one();
+        const uint32_t one = elect_one();
         constexpr uint32_t kInstr = (1u << 4) | ((256 / 16) << 24);
         const uint32_t base = smem_addr(smem);
         uint32_t seq = 0;
@@ -1248,9 +1246,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                 }
             }
         }
+        end_products(gone, one, smem_addr(&s_end));
     }
     if (gone) atomicExch(a.error, 1ull);
-    if (warp == kWarps && rank == 0) end_products(gone, one, smem_addr(&s_end));
     fence_before();
     __syncthreads();
     cluster_sync();
