@@ -370,16 +370,32 @@ struct PrpPlan {
     RnsLayout layout{};
 };
 
-// Where the residue form is the faster one, in ms for 16 numbers and for 19456
-// (limbs, residues): 200 bits 0.21, 0.32 and 0.44, 0.51; 256 bits 0.46, 0.39 and
-// 1.21, 0.61; 712 bits 1.61, 1.74 and 4.94, 2.07 (5000 numbers: 2.15, 1.85); 1100
-// bits 4.36, 3.58; 1400 bits 6.33, 5.01 and 29.9, 5.7; 2136 bits 16.0, 11.1 and 105,
-// 12.3; 2838 bits (9001 numbers) 106, 26.  So from two limbs per lane on; with two or three chunks of slots and
-// fewer than three limbs per lane only for enough numbers to fill the limb form.
-bool rns_pays(uint32_t bits, uint64_t max_items) {
+// Where the residue form is the faster one: from so many numbers of one width on.
+// Whole calls in ms (limbs, residues) at the widths where a step up of one form's time
+// comes before the other's, elsewhere the residue form is ahead from one number on:
+//   253-360 bits, a chunk: 300 bits, one number 0.32, 0.39; two 0.40, 0.39
+//   361-508, two chunks and two limbs per lane: 430 bits, 9728 numbers 0.97, 1.03;
+//     19456 1.75, 1.17; at 1.3 waves of single tiles 2.1, 2.1
+//   509-735, two and three: 735 bits, two 1.30, 1.45; four 1.49, 1.45
+//   736-764, three and three: 764 bits, 4864 1.87, 1.98; 7296 2.23, 2.02
+//   1104-1276, four and five: 1276 bits, one 4.44, 4.53; two 4.65, 4.53
+//   1464-1532, five and six: 1464 bits, two 6.18, 6.26; four 6.57, 6.27
+// and the others: 765 bits, one 1.97, 1.87; 1100 bits 3.83, 2.67; 2136 bits 15.0, 11.0;
+// 2838 bits 52.4, 24.7; 200 bits 0.20, 0.32.
+bool rns_pays(uint32_t bits, uint64_t items) {
     const uint32_t n = rns_chunks(bits);
     if (bits < 253 || n == 0) return false;
-    return n == 1 || bits >= 765 || max_items >= 4096;
+    const int L = limbs_per_lane(bits);
+    const uint64_t wave = rns_wave(bits, false);
+    switch (16 * n + (uint32_t)L) {
+        case 16 * 1 + 2: return items >= 2;
+        case 16 * 2 + 2: return items >= 5 * wave / 8 && !(items > wave && items < 7 * wave / 5);
+        case 16 * 2 + 3: return items >= 4;
+        case 16 * 3 + 3: return items >= 3 * wave / 10;
+        case 16 * 4 + 5: return items >= 2;
+        case 16 * 5 + 6: return items >= 4;
+        default: return true;
+    }
 }
 
 // The residue form's workspace, some 6 KB per number of 2136 bits, is for a wave of
