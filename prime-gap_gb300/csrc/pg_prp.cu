@@ -30,8 +30,10 @@
 // after x = 2^d, up to s squarings (one more than the textbook s - 1).  The
 // extra squaring never changes a verdict (2^(N-1) = -1 mod N has no odd
 // solution N > 1).
+#include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <numeric>
 #include <vector>
 
 #include "pg_arith.cuh"
@@ -398,26 +400,118 @@ bool rns_pays(uint32_t bits, uint64_t items) {
     }
 }
 
-// The residue form's workspace, some 6 KB per number of 2136 bits, is for a wave of
-// numbers: a longer list goes through it in slices.
-PrpPlan prp_plan(uint32_t bits, uint64_t max_items) {
+PrpPlan limb_plan(uint32_t bits) {
     PrpPlan p;
     p.bits = bits;
     p.L = limbs_per_lane(bits);
+    return p;
+}
+
+// The residue form's workspace, some 6 KB per number of 2136 bits, is for a wave of
+// numbers: a longer list goes through it in slices.
+PrpPlan prp_plan(uint32_t bits, uint64_t max_items) {
+    PrpPlan p = limb_plan(bits);
     p.rns = rns_pays(bits, max_items);
     if (p.rns) p.layout = rns_layout(bits, 8u * (uint32_t)p.L, rns_slice(bits, max_items), max_items);
     return p;
 }
 
-// The residue form's workspace; where the device has no room for it, the limb form
-// takes the call.
-cudaError_t prp_workspace(PrpPlan &p, pgh::DevBuf &work) {
-    if (!p.rns) return cudaSuccess;
-    const cudaError_t e = work.ensure(p.layout.total);
-    if (e != cudaErrorMemoryAllocation) return e;
+// The limb form at the limbs per lane of `bits`: microseconds per bit of a chain of
+// squarings (16 numbers), nanoseconds per bit of each of many numbers (4864 to 38912;
+// above 3068 bits put low).
+double limb_step_us(uint32_t bits) {
+    constexpr double kStep[kMaxL + 1] = {0,   0.49, 1.15, 1.88, 2.84, 3.8,  4.38, 5.81, 7.6,
+                                         7.4, 8.6,  10.3, 18.9, 14,   15.6, 19.3, 20.4};
+    return kStep[limbs_per_lane(bits)];
+}
+double limb_bit_ns(uint32_t bits) {
+    constexpr double kNs[kMaxL + 1] = {0, 0.1, 0.17, 0.31, 0.5, 0.76, 1.04, 1.45, 1.74, 2.4, 2.95, 2.95, 2.95, 4, 5, 5, 5};
+    return kNs[limbs_per_lane(bits)];
+}
+// ... and of a launch over numbers up to `bits` wide whose widths add up to `sum`.
+double limb_us(uint32_t bits, double sum) {
+    return std::max(bits * limb_step_us(bits), 1e-3 * sum * limb_bit_ns(bits));
+}
+
+// Numbers that are tested with one plan: `count` of the call's order from `first` on.
+struct PrpPart {
+    uint64_t first, count;
+    PrpPlan plan;
+};
+
+// The parts of a list of numbers of these widths; `order` becomes the order in which
+// they are tested.  The residue form takes numbers of nearly one width.  Where a list
+// spreads further, it takes the bands of kRnsSpread bits whose many numbers are worth a
+// wave of their own, with or without the widest numbers' band; one launch of the limb
+// form takes the rest, at the rest's own width; or the limb form takes all, where that is
+// the fastest.  (All through the residue form at the widest number's width and what it
+// left through the limb form as well, the limb form for all, and in parts, in ms: 15
+// numbers of 2136 bits and one of 2161 29.0, 16.1, 16.1; 2000 of 300 to 2800 bits 53, 29,
+// 29; 9000 of 2838 and one of 2863 132, 106, 51; 9000 of 2136 and 9000 of 1400 51,
+// 78, 17.)
+std::vector<PrpPart> prp_parts(const std::vector<uint32_t> &width, std::vector<uint64_t> &order) {
+    const uint64_t n = width.size();
+    order.resize(n);
+    std::iota(order.begin(), order.end(), 0ull);
+    const auto [min, max] = std::minmax_element(width.begin(), width.end());
+    const uint32_t lo = *min, hi = *max;
+    if (hi - lo <= kRnsSpread) return {{0, n, prp_plan(hi, n)}};
+    // numbers of each width below w, and the sum of their widths
+    std::vector<uint64_t> below(hi + 2, 0), sum(hi + 2, 0);
+    for (uint32_t w : width) below[w + 1]++;
+    for (uint32_t w = 0; w <= hi; w++) {
+        sum[w + 1] = sum[w] + below[w + 1] * w;
+        below[w + 1] += below[w];
+    }
+    std::vector<PrpPart> best{{0, n, limb_plan(hi)}};
+    std::vector<uint32_t> best_of;  // a width's part
+    double best_us = 0.95 * limb_us(hi, (double)sum[hi + 1]);
+    for (const bool widest : {false, true}) {
+        constexpr uint32_t kRest = ~0u;
+        std::vector<PrpPart> parts;
+        std::vector<uint32_t> of(hi + 1, kRest);
+        double us = 0, rest_sum = 0;
+        uint32_t rest_bits = 0;
+        for (uint32_t w = hi; w >= lo;) {
+            const uint32_t from = std::max(lo, w - std::min(w, kRnsSpread));
+            const uint64_t here = below[w + 1] - below[w], count = below[w + 1] - below[from];
+            if (here && rns_pays(w, count) &&
+                ((widest && w == hi) || rns_us(w, count) < 1e-3 * (double)(sum[w + 1] - sum[from]) * limb_bit_ns(w))) {
+                std::fill(of.begin() + from, of.begin() + w + 1, (uint32_t)parts.size());
+                parts.push_back({0, count, prp_plan(w, count)});
+                us += rns_us(w, count);
+                w = from;
+            } else if (here) {
+                rest_bits = std::max(rest_bits, w);
+                rest_sum += (double)here * w;
+            }
+            w--;
+        }
+        if (rest_bits) {
+            uint64_t count = n;
+            for (const PrpPart &p : parts) count -= p.count;
+            us += limb_us(rest_bits, rest_sum);
+            std::replace(of.begin(), of.end(), kRest, (uint32_t)parts.size());
+            parts.push_back({0, count, limb_plan(rest_bits)});
+        }
+        if (us < best_us && parts.size() > 1) best_us = us, best = parts, best_of = of;
+    }
+    if (best.size() == 1) return best;
+    std::vector<uint64_t> at(best.size());
+    for (size_t i = 1; i < best.size(); i++) best[i].first = best[i - 1].first + best[i - 1].count;
+    for (size_t i = 0; i < best.size(); i++) at[i] = best[i].first;
+    for (uint64_t i = 0; i < n; i++) order[at[best_of[width[i]]]++] = i;
+    return best;
+}
+
+// The residue form's workspace; false where the device has no room for it: then the
+// limb form takes the call.
+bool prp_workspace(pgh::DevBuf &work, size_t bytes, cudaError_t &e) {
+    e = work.ensure(bytes);
+    if (e != cudaErrorMemoryAllocation) return true;
+    e = cudaSuccess;
     cudaGetLastError();
-    p.rns = false;
-    return cudaSuccess;
+    return false;
 }
 
 cudaError_t prp_begin(const PrpPlan &p, void *work, cudaStream_t s) {
@@ -736,8 +830,8 @@ int pgs_prp_test(pgs_ctx *ctx, const uint32_t *limbs, uint32_t n_limbs, size_t c
     std::lock_guard<std::mutex> g(ctx->mu);
     CK(cudaSetDevice(ctx->device));
     if (count == 0) return PGS_OK;
-    // width from the largest number; tiny, even and too wide numbers on the host
-    uint32_t max_bits = 0;
+    // the widths; tiny, even and too wide numbers on the host
+    std::vector<uint32_t> widths;
     std::vector<uint64_t> dev_rows;
     for (size_t i = 0; i < count; i++) {
         const uint32_t *v = limbs + i * n_limbs;
@@ -757,44 +851,60 @@ int pgs_prp_test(pgs_ctx *ctx, const uint32_t *limbs, uint32_t n_limbs, size_t c
             out[i] = 0;
             continue;
         }
-        max_bits = std::max(max_bits, bits);
+        widths.push_back(bits);
         dev_rows.push_back(i);
     }
     if (dev_rows.empty()) return PGS_OK;
-    pg::PrpPlan plan = pg::prp_plan(max_bits, dev_rows.size());
-    const uint32_t n = 8u * (uint32_t)plan.L;
-    std::vector<uint32_t> packed(dev_rows.size() * n, 0u);
-    std::vector<pg::PrpItem> items(dev_rows.size());
-    for (size_t j = 0; j < dev_rows.size(); j++) {
-        const uint32_t *v = limbs + dev_rows[j] * n_limbs;
-        std::memcpy(&packed[j * n], v, std::min(n, n_limbs) * 4u);
-        items[j] = pg::PrpItem{(uint32_t)j, 0};
+    std::vector<uint64_t> order;
+    std::vector<pg::PrpPart> parts = pg::prp_parts(widths, order);
+    size_t words = 0, work_bytes = 0;
+    for (const auto &part : parts) {
+        words += part.count * 8u * (size_t)part.plan.L;
+        if (part.plan.rns) work_bytes = std::max(work_bytes, part.plan.layout.total);
     }
     const cudaStream_t s = ctx->stream;
     DevBuf d_nums, d_items, d_res, d_work;
     DevBuf *bufs[] = {&d_nums, &d_items, &d_res, &d_work};
     for (DevBuf *b : bufs) b->pool = &ctx->dpool;
+    cudaError_t e = cudaSuccess;
+    if (work_bytes && !pg::prp_workspace(d_work, work_bytes, e)) {
+        for (auto &part : parts) part.plan.rns = false;
+    }
+    std::vector<uint32_t> packed(words, 0u);
+    std::vector<pg::PrpItem> items(dev_rows.size());
+    uint32_t *to = packed.data();
+    for (const auto &part : parts) {
+        const uint32_t n = 8u * (uint32_t)part.plan.L;
+        for (uint64_t j = 0; j < part.count; j++, to += n) {
+            std::memcpy(to, limbs + dev_rows[order[part.first + j]] * n_limbs, std::min(n, n_limbs) * 4u);
+            items[part.first + j] = pg::PrpItem{(uint32_t)j, 0};
+        }
+    }
     std::vector<uint8_t> res(dev_rows.size());
-    cudaError_t e = upload(d_nums, packed, s);
+    std::vector<unsigned long long> gave_up(parts.size(), 0ull);
+    if (e == cudaSuccess) e = upload(d_nums, packed, s);
     if (e == cudaSuccess) e = upload(d_items, items, s);
     if (e == cudaSuccess) e = d_res.ensure(dev_rows.size());
-    if (e == cudaSuccess) e = pg::prp_workspace(plan, d_work);
-    if (e == cudaSuccess) e = pg::prp_begin(plan, d_work.p, s);
-    if (e == cudaSuccess)
-        e = pg::prp_launch(plan, d_work.p, d_nums.as<uint32_t>(), d_items.as<pg::PrpItem>(), nullptr, dev_rows.size(),
-                           d_res.as<uint8_t>(), s);
-    unsigned long long gave_up = 0;
-    if (e == cudaSuccess) e = pg::prp_error(plan, d_work.p, &gave_up, s);
+    const uint32_t *nums = d_nums.as<uint32_t>();
+    for (size_t i = 0; i < parts.size() && e == cudaSuccess; i++) {
+        const pg::PrpPart &part = parts[i];
+        e = pg::prp_begin(part.plan, d_work.p, s);
+        if (e == cudaSuccess)
+            e = pg::prp_launch(part.plan, d_work.p, nums, d_items.as<pg::PrpItem>() + part.first, nullptr, part.count,
+                               d_res.as<uint8_t>() + part.first, s);
+        if (e == cudaSuccess) e = pg::prp_error(part.plan, d_work.p, &gave_up[i], s);
+        nums += part.count * 8u * (size_t)part.plan.L;
+    }
     if (e == cudaSuccess) e = cudaMemcpyAsync(res.data(), d_res.p, res.size(), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     cudaStreamSynchronize(s);
     for (DevBuf *b : bufs) b->release();
     if (e != cudaSuccess) return fail(ctx, e, "pgs_prp_test");
-    if (gave_up) {
+    if (std::any_of(gave_up.begin(), gave_up.end(), [](unsigned long long g) { return g != 0; })) {
         ctx->err = "pgs_prp_test: a wait on the device gave up";
         return PGS_ETIMEOUT;
     }
-    for (size_t j = 0; j < dev_rows.size(); j++) out[dev_rows[j]] = res[j];
+    for (size_t j = 0; j < dev_rows.size(); j++) out[dev_rows[order[j]]] = res[j];
     return PGS_OK;
 }
 
@@ -844,7 +954,8 @@ int prp_gaps_core(pgs_ctx *ctx, const pgs_gap_params *prm, uint64_t rows, const 
         cudaStreamSynchronize(s);
         for (DevBuf *b : bufs) b->release();
     };
-    cudaError_t e = pg::prp_workspace(plan, d_work);
+    cudaError_t e = cudaSuccess;
+    if (plan.rns) plan.rns = pg::prp_workspace(d_work, plan.layout.total, e);
     const uint64_t max_items = plan.rns ? pg::rns_wave(bits, true) : limb_round;
     if (e == cudaSuccess) e = upload(d_k, k, s);
     if (e == cudaSuccess) e = upload(d_kp, kprimes, s);

@@ -1412,6 +1412,21 @@ uint64_t rns_slice(uint32_t bits, uint64_t left) {
     return std::min(left, rns_wave(bits, group_pays(rns_chunks(bits), tiles)));
 }
 
+// A launch of one wave: per bit a step's time of one tile or of a group (the widest
+// numbers of each chunk count, 16 and 38912 of them), and the set-up and verdicts.
+double rns_us(uint32_t bits, uint64_t items) {
+    constexpr double kStep[kRnsMaxChunks + 1] = {0, 1.05, 1.88, 2.36, 3.5, 4.22, 5.13, 5.95, 7.43, 8.75};
+    constexpr double kGroupStep[kRnsMaxChunks + 1] = {0, 4.2, 4.6, 4.8, 6.5, 8.6, 9.6};
+    const uint32_t n = rns_chunks(bits);
+    double us = 0;
+    for (uint64_t left = items; left > 0;) {
+        const uint64_t take = rns_slice(bits, left);
+        us += 70 + bits * (group_pays(n, (left + kRnsTile - 1) / kRnsTile) ? kGroupStep[n] : kStep[n]);
+        left -= take;
+    }
+    return us + 0.0025 * n * (double)items;
+}
+
 RnsLayout rns_layout(uint32_t bits, uint32_t limbs, uint64_t max_items, uint64_t all_items) {
     RnsLayout l{};
     l.chunks = rns_chunks(bits);

@@ -11,6 +11,7 @@ constexpr uint32_t kRnsMaxChunks = 9;   // 32 residue slots each
 constexpr uint32_t kRnsDumps = 12;      // last values kept for the strong test's verdict
 constexpr uint32_t kRnsTile = 256;      // numbers of a tile, half in each CTA of a pair
 constexpr uint32_t kRnsGroup = 4;       // most tiles that a pair takes in turn
+constexpr uint32_t kRnsSpread = 22;     // numbers this many bits narrower than the widest are taken with it
 
 struct PrpItem {
     uint32_t row;  // row of the base numbers
@@ -23,6 +24,9 @@ uint32_t rns_chunks(uint32_t bits);
 // Numbers that run at once in one wave, of single tiles or of full groups of
 // tiles (0 where rns_chunks is 0 and full is asked).
 uint64_t rns_wave(uint32_t bits, bool full);
+
+// Microseconds that rns_test takes, over slices of a long list.
+double rns_us(uint32_t bits, uint64_t items);
 
 // How many of `left` numbers the next rns_test of a long list takes: one wave.
 uint64_t rns_slice(uint32_t bits, uint64_t left);
