@@ -416,21 +416,26 @@ PrpPlan prp_plan(uint32_t bits, uint64_t max_items) {
     return p;
 }
 
+// Numbers of one block on each SM.
+uint64_t limb_layer() { return rns_wave(0, false) * kGroups / kRnsTile * 2; }
+
 // The limb form at the limbs per lane of `bits`: microseconds per bit of a chain of
 // squarings (16 numbers), nanoseconds per bit of each of many numbers (4864 to 38912;
 // above 3068 bits put low).
 double limb_step_us(uint32_t bits) {
-    constexpr double kStep[kMaxL + 1] = {0,   0.49, 1.15, 1.88, 2.84, 3.8,  4.38, 5.81, 7.6,
-                                         7.4, 8.6,  10.3, 18.9, 14,   15.6, 19.3, 20.4};
+    constexpr double kStep[kMaxL + 1] = {0,   0.5, 1.3,  1.95, 2.87, 3.82, 4.4,  5.83, 7.6,
+                                         7.4, 8.6, 10.3, 18.9, 14,   15.6, 19.3, 20.4};
     return kStep[limbs_per_lane(bits)];
 }
 double limb_bit_ns(uint32_t bits) {
     constexpr double kNs[kMaxL + 1] = {0, 0.1, 0.17, 0.31, 0.5, 0.76, 1.04, 1.45, 1.74, 2.4, 2.95, 2.95, 2.95, 4, 5, 5, 5};
     return kNs[limbs_per_lane(bits)];
 }
-// ... and of a launch over numbers up to `bits` wide whose widths add up to `sum`.
+// ... and of a launch over numbers up to `bits` wide whose widths add up to `sum`: one
+// block of 16 numbers on each SM after another.
 double limb_us(uint32_t bits, double sum) {
-    return std::max(bits * limb_step_us(bits), 1e-3 * sum * limb_bit_ns(bits));
+    const double layer = (double)limb_layer() * bits;
+    return std::max(bits * limb_step_us(bits), 1e-3 * std::ceil(sum / layer) * layer * limb_bit_ns(bits));
 }
 
 // Numbers that are tested with one plan: `count` of the call's order from `first` on.
@@ -580,7 +585,8 @@ struct GapLists {
     const uint32_t *n_prev, *n_next, *dist;
 };
 
-// Distances past the sieve length that are coprime to K, a bit each from sl + 1.
+// Distances past the sieve length that are coprime to K, a bit each from sl + 1 (for the
+// residue form's rounds, which nearly all look at some).
 constexpr uint32_t kPastBits = 1u << 17;
 
 __device__ __forceinline__ bool coprime_to_k(uint32_t x, const uint32_t *kp, uint32_t nkp) {
@@ -597,12 +603,14 @@ __global__ void past_kernel(const uint32_t *kp, uint32_t nkp, uint32_t sl, uint3
 }
 
 // A round's candidates, nearest first: spec for each active search and one more
-// for the first `extra` that ask.  Where the unknowns end, the round goes on past
-// the sieve length with the next distances that keep N odd and coprime to K (a
-// round is a whole wave: a search that ends there does not wait for another one).
-// A warp per search.
+// for the first `extra` that ask; past the sieve length, the next distances that keep N
+// odd and coprime to K.  With go_on, a round goes on past the sieve length where the
+// unknowns end (a round of the residue form is a whole wave: a search that ends there
+// does not wait for another one).  Without, a search has its unknowns tested first: the
+// limb form's time grows with the candidates (10 searches of 2503#/30030: 131 ms with 512
+// each, 55 with 64).  A warp per search.
 __global__ void select_kernel(GapSearch *searches, uint64_t rows, GapLists ls, const uint32_t *centers, uint32_t n,
-                              uint32_t spec, uint32_t extra, const uint32_t *kp, uint32_t nkp,
+                              uint32_t spec, uint32_t extra, bool go_on, const uint32_t *kp, uint32_t nkp,
                               const uint32_t *__restrict__ past_bits, uint32_t sl, uint32_t x_limit, PrpItem *items,
                               uint64_t max_items, unsigned long long *n_items, unsigned long long *asked,
                               unsigned long long *errors) {
@@ -622,6 +630,7 @@ __global__ void select_kernel(GapSearch *searches, uint64_t rows, GapLists ls, c
         want += __shfl_sync(0xFFFFFFFFu, more, 0);
     }
     const uint32_t nlist = next ? ls.n_next[r] : ls.n_prev[r];
+    if (!go_on && !st.past) want = min(want, nlist - st.idx);
     unsigned long long base = 0;
     if (lane == 0 && want) base = atomicAdd(n_items, (unsigned long long)want);
     base = __shfl_sync(0xFFFFFFFFu, base, 0);
@@ -641,7 +650,7 @@ __global__ void select_kernel(GapSearch *searches, uint64_t rows, GapLists ls, c
             // 1024 distances, 32 a lane (32 past the bitmap, one a lane): those
             // coprime to K, not before x, of the other parity than m*K
             const uint32_t at = x - (sl + 1);
-            const bool table = at < kPastBits;
+            const bool table = past_bits && at < kPastBits;
             uint32_t from, word;
             if (table) {
                 const uint32_t w = (at >> 5) + lane;
@@ -817,7 +826,7 @@ uint32_t skip_threshold(double klog, uint64_t m, float min_merit) {
 }
 
 constexpr uint64_t kRoundTarget = 1ull << 15;  // candidates per round of the limb form
-constexpr uint32_t kMaxSpec = 512;             // candidates per search and round
+constexpr uint32_t kMaxSpec = 512;             // most candidates per search and round
 constexpr uint32_t kPastScanSpan = 1u << 24;   // distances scanned past SL before giving up
 
 }  // namespace
@@ -912,11 +921,55 @@ int pgs_prp_test(pgs_ctx *ctx, const uint32_t *limbs, uint32_t n_limbs, size_t c
 
 namespace {
 
-// Device lists of rows (d_m .. d_dist, as pgs_unknowns) and the host copy of
-// their m: the gap search.  The caller holds ctx->mu and checked the lists.
+// What a search's rounds are expected to take, in microseconds, with so many unknowns on
+// each side and a chance that one is prime (sl / lnN primes on a side): round after round
+// of so many candidates, shared by the sides that are left, until there is none.
+struct RoundCost {
+    uint32_t bits;
+    double unknowns, chance;
+    double us(uint64_t searches, uint64_t items, bool residues) const {
+        double total = 0, left = (double)searches;
+        for (int round = 0; round < 100 && left >= 0.2; round++) {
+            double each = std::min((double)items / left, (double)kMaxSpec);
+            if (!residues) each = std::min(each, unknowns);
+            const double count = std::ceil(each * left);
+            total += 130 + (residues ? pg::rns_us(bits, (uint64_t)count) : pg::limb_us(bits, count * bits));
+            left *= std::exp(-each * chance);
+        }
+        return total;
+    }
+    // Candidates of a round of the limb form: blocks on each SM that are full.  (Both
+    // sides of 5 rows of 2503#/30030: 7 rounds of 64 for each side 386 ms, one of 512 131,
+    // 243 111; of 20 rows 417, 372, 142.)
+    uint64_t limb_items(uint64_t searches) const {
+        uint64_t best = 0;
+        double best_us = 0;
+        for (uint64_t items = pg::limb_layer(); items <= kRoundTarget; items += pg::limb_layer()) {
+            const double t = us(searches, items, false);
+            if (!best || t < best_us) best = items, best_us = t;
+        }
+        return best;
+    }
+};
+
+// Whether a search's rounds are the residue form's, which a search of few rows leaves
+// mostly empty or fills with what is not needed (7 rows of 307#/210: 0.70 ms limb by limb,
+// 1.00 in residues).  Rows with m far below the largest are tested limb by limb in every
+// round: more than a few, and the whole search is.
+bool residue_rounds(const RoundCost &c, uint64_t rows, const uint64_t *h_m, uint64_t searches) {
+    if (c.bits < 253 || pg::rns_chunks(c.bits) == 0) return false;
+    uint64_t max_m = 0, narrow = 0;
+    for (uint64_t r = 0; r < rows; r++) max_m = std::max(max_m, h_m[r]);
+    for (uint64_t r = 0; r < rows; r++) narrow += h_m[r] >> 1 < max_m >> pg::kRnsSpread;
+    if (narrow > rows / 256) return false;
+    return c.us(searches, pg::rns_wave(c.bits, false), true) < 1.1 * c.us(searches, c.limb_items(searches), false);
+}
+
+// Device lists of rows (d_m .. d_dist, as pgs_unknowns; `listed` unknowns in all) and the
+// host copy of their m: the gap search.  The caller holds ctx->mu and checked the lists.
 int prp_gaps_core(pgs_ctx *ctx, const pgs_gap_params *prm, uint64_t rows, const uint64_t *h_m,
                   const uint64_t *d_m, const uint64_t *d_start, const uint32_t *d_np, const uint32_t *d_nn,
-                  const uint32_t *d_dist, pgs_gap_result *out, pgs_gap_stats *stats) {
+                  const uint32_t *d_dist, uint64_t listed, pgs_gap_result *out, pgs_gap_stats *stats) {
     if (prm->p < 2 || !is_prime_u64(prm->p) || prm->d == 0 || prm->sieve_length == 0 ||
         prm->sieve_length >= (1u << 30)) {
         ctx->err = "pgs_prp_gaps: bad p, d or sieve_length";
@@ -937,9 +990,15 @@ int prp_gaps_core(pgs_ctx *ctx, const pgs_gap_params *prm, uint64_t rows, const 
     // A round is a wave of the residue form (its time is the same for fewer), or
     // enough to fill the GPU with the limb form
     const bool may_skip = prm->one_side_skip != 0;
-    const uint64_t searches = 2 * rows;
+    const uint64_t searches = 2 * rows, wave = pg::rns_wave(bits, true);
     const uint64_t limb_round = std::max<uint64_t>(searches, kRoundTarget);
-    pg::PrpPlan plan = pg::prp_plan(bits, std::max<uint64_t>(limb_round, pg::rns_wave(bits, true)));
+    RoundCost cost{bits, std::max(1.0, (double)listed / (double)searches), 1.0};
+    cost.chance = std::min(1.0, prm->sieve_length / (0.693 * bits) / cost.unknowns);
+    pg::PrpPlan plan = pg::limb_plan(bits);
+    if (residue_rounds(cost, rows, h_m, may_skip ? rows : searches)) {
+        plan.rns = true;
+        plan.layout = pg::rns_layout(bits, 8u * (uint32_t)plan.L, wave, wave);
+    }
     const uint32_t n = 8u * (uint32_t)plan.L;
     std::vector<uint32_t> skip(rows, 0u);
     if (prm->one_side_skip) {
@@ -956,7 +1015,7 @@ int prp_gaps_core(pgs_ctx *ctx, const pgs_gap_params *prm, uint64_t rows, const 
     };
     cudaError_t e = cudaSuccess;
     if (plan.rns) plan.rns = pg::prp_workspace(d_work, plan.layout.total, e);
-    const uint64_t max_items = plan.rns ? pg::rns_wave(bits, true) : limb_round;
+    const uint64_t max_items = plan.rns ? wave : limb_round;
     if (e == cudaSuccess) e = upload(d_k, k, s);
     if (e == cudaSuccess) e = upload(d_kp, kprimes, s);
     if (e == cudaSuccess && may_skip) e = upload(d_skip, skip, s);
@@ -978,8 +1037,9 @@ int prp_gaps_core(pgs_ctx *ctx, const pgs_gap_params *prm, uint64_t rows, const 
     const unsigned rb = (unsigned)((rows + 255) / 256), sb = (unsigned)((searches + 7) / 8);
     pg::centers_kernel<<<rb, 256, 0, s>>>(d_k.as<uint32_t>(), (uint32_t)k.size(), d_m, rows, n,
                                           d_centers.as<uint32_t>());
-    pg::past_kernel<<<pg::kPastBits / 256, 256, 0, s>>>(d_kp.as<uint32_t>(), (uint32_t)kprimes.size(),
-                                                        prm->sieve_length, d_past.as<uint32_t>());
+    if (plan.rns)
+        pg::past_kernel<<<pg::kPastBits / 256, 256, 0, s>>>(d_kp.as<uint32_t>(), (uint32_t)kprimes.size(),
+                                                            prm->sieve_length, d_past.as<uint32_t>());
     pg::gap_init_kernel<<<(unsigned)((searches + 255) / 256), 256, 0, s>>>(
         d_state.as<pg::GapSearch>(), rows, ls, may_skip, prm->sieve_length, d_out.as<pgs_gap_result>());
     uint64_t active = may_skip ? rows : searches, rounds = 0, launched = 0;
@@ -987,8 +1047,10 @@ int prp_gaps_core(pgs_ctx *ctx, const pgs_gap_params *prm, uint64_t rows, const 
     e = cudaMemcpyAsync(ctr, host_ctr, 40, cudaMemcpyHostToDevice, s);
     const uint32_t x_limit = prm->sieve_length + kPastScanSpan;
     while (e == cudaSuccess && active > 0) {
-        uint64_t quota = limb_round;
-        if (plan.rns) {
+        uint64_t quota = active;
+        if (!plan.rns) {
+            quota = std::max(active, std::min(cost.limb_items(active), active * kMaxSpec));
+        } else {
             // A wave of several tiles per pair tests 1.1-1.2 times as many a second as
             // a single one, but what lies past a search's end is wasted: with s
             // candidates per search in the single wave and a chance p of each (found
@@ -996,15 +1058,14 @@ int prp_gaps_core(pgs_ctx *ctx, const pgs_gap_params *prm, uint64_t rows, const 
             // (2136 bits, p 1/39, 20.5 and 12.4 ms: 33 searches a ms each at s p = 0.43).
             const uint64_t one = pg::rns_wave(bits, false);
             const double chance = launched ? (double)host_ctr[4] / (double)launched : 1.0 / 32;
-            quota = (double)one * chance < 0.45 * (double)active ? max_items : one;
+            quota = std::min((double)one * chance < 0.45 * (double)active ? max_items : one, active * kMaxSpec);
         }
-        quota = std::min(quota, active * kMaxSpec);
         const uint32_t spec = (uint32_t)(quota / active), extra = (uint32_t)(quota % active);
         e = cudaMemsetAsync(ctr, 0, 16, s);  // items, asked
         if (e) break;
         pg::select_kernel<<<sb, 256, 0, s>>>(d_state.as<pg::GapSearch>(), rows, ls, d_centers.as<uint32_t>(), n, spec,
-                                             extra, d_kp.as<uint32_t>(), (uint32_t)kprimes.size(),
-                                             d_past.as<uint32_t>(), prm->sieve_length, x_limit,
+                                             extra, plan.rns, d_kp.as<uint32_t>(), (uint32_t)kprimes.size(),
+                                             plan.rns ? d_past.as<uint32_t>() : nullptr, prm->sieve_length, x_limit,
                                              d_items.as<pg::PrpItem>(), quota, ctr, ctr + 1, ctr + 3);
         e = pg::prp_launch(plan, d_work.p, d_centers.as<uint32_t>(), d_items.as<pg::PrpItem>(), ctr, quota,
                            d_res.as<uint8_t>(), s);
@@ -1068,11 +1129,14 @@ int pgs_prp_gaps(pgs_ctx *ctx, const pgs_gap_params *prm, const pgs_unknowns *li
         ctx->err = "pgs_prp_gaps: bad lists";
         return PGS_EINVAL;
     }
-    for (uint64_t r = 0; r < rows; r++)
+    uint64_t listed = 0;
+    for (uint64_t r = 0; r < rows; r++) {
         if (lists->m[r] == 0 || lists->start[r] + lists->n_prev[r] + lists->n_next[r] > lists->total) {
             ctx->err = "pgs_prp_gaps: row outside the distance array";
             return PGS_EINVAL;
         }
+        listed += lists->n_prev[r] + (uint64_t)lists->n_next[r];
+    }
     const cudaStream_t s = ctx->stream;
     PackedLists pk;
     pk.block.pool = &ctx->dpool;
@@ -1086,7 +1150,7 @@ int pgs_prp_gaps(pgs_ctx *ctx, const pgs_gap_params *prm, const pgs_unknowns *li
     if (e == cudaSuccess) e = up(pk.n_next, lists->n_next, rows * 4);
     if (e == cudaSuccess) e = up(pk.dist, lists->dist, lists->total * 4);
     int rc = e == cudaSuccess ? prp_gaps_core(ctx, prm, rows, lists->m, pk.m, pk.start, pk.n_prev, pk.n_next,
-                                              pk.dist, out, stats)
+                                              pk.dist, listed, out, stats)
                               : fail(ctx, e, "pgs_prp_gaps upload");
     cudaStreamSynchronize(s);
     pk.block.release();
@@ -1112,7 +1176,8 @@ int pgs_prp_gaps_prepared(pgs_ctx *ctx, pgs_prepared *prep, const pgs_gap_params
     PackedLists pk;
     int rc = job_lists_device(ctx, prep, s, pk);
     if (rc == PGS_OK)
-        rc = prp_gaps_core(ctx, &jp, rows, m.data(), pk.m, pk.start, pk.n_prev, pk.n_next, pk.dist, out, stats);
+        rc = prp_gaps_core(ctx, &jp, rows, m.data(), pk.m, pk.start, pk.n_prev, pk.n_next, pk.dist, pk.total, out,
+                           stats);
     cudaStreamSynchronize(s);
     pk.block.release();
     return rc;

@@ -1421,7 +1421,7 @@ double rns_us(uint32_t bits, uint64_t items) {
     double us = 0;
     for (uint64_t left = items; left > 0;) {
         const uint64_t take = rns_slice(bits, left);
-        us += 70 + bits * (group_pays(n, (left + kRnsTile - 1) / kRnsTile) ? kGroupStep[n] : kStep[n]);
+        us += 20 + bits * (group_pays(n, (left + kRnsTile - 1) / kRnsTile) ? kGroupStep[n] : kStep[n]);
         left -= take;
     }
     return us + 0.0025 * n * (double)items;
