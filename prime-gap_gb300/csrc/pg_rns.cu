@@ -347,7 +347,11 @@ __device__ bool near_widest(const uint32_t *n, int top, uint32_t bits, double a_
 // form of 1).  A block takes 8 numbers; a thread one slot of each base.
 // A prime m of base A that divides N leaves no inverse there.  N can still be a
 // pseudoprime only if 2^(N-1) = 1 mod m; then the chain runs mod N/m (the
-// exponent stays N's) and the verdict looks at both.
+// exponent stays N's) and the verdict looks at both; so too for two primes.  It is
+// composite if m^2 divides it: 2's order mod m^2 would divide N - 1, hence be prime to m,
+// hence divide m - 1, as it does below 4096 for m = 1093 and 3511 alone.  (Of unsieved
+// numbers of 2900 bits, where A goes down to 17, one in 2000 is such a multiple; the limb
+// form took 54 ms more for a single one.)
 // Bound by the remainders' multiplies, one per 16 bits, number and modulus.
 constexpr uint32_t kSetupNumbers = 8;
 __global__ void setup_kernel(const __grid_constant__ RnsSlots p, uint32_t chunks, uint32_t bits, double a_mant,
@@ -419,15 +423,19 @@ __global__ void setup_kernel(const __grid_constant__ RnsSlots p, uint32_t chunks
         }
         pa = mod_small(qa << 16, ma, ia), pb = mod_small(qb << 16, mb, ib);
     }
-    const auto slots = [&](uint32_t g, uint32_t ra, uint32_t rb) {
+    const auto slots = [&](uint32_t g, uint32_t ra, uint32_t rb, uint32_t by) {  // by: what N was divided by
         const uint64_t at = slot_at(chunks, first + g, t);
         int ca = 0;
         if (ma > 1 && ra == 0) {
-            uint32_t r = limbs_mod(s_n[g], limbs, ma - 1, inv32_of(ma - 1));
-            r = r ? r - 1 : ma - 2;
             atomicAdd(&s_divide[g], 1u);
             s_by[g] = ma;
-            if (pow_small(2, r, ma, ia) != 1) s_out[g] = 1;
+            if (by == 1) {
+                uint32_t r = limbs_mod(s_n[g], limbs, ma - 1, inv32_of(ma - 1));
+                r = r ? r - 1 : ma - 2;
+                if (pow_small(2, r, ma, ia) != 1) s_out[g] = 1;
+            } else if ((ma == (by & 0xFFFFu) || ma == by >> 16) && ma != 1093 && ma != 3511) {
+                s_out[g] = 1;
+            }
         } else if (ma > 1) {  // -1 / (N (A/m))
             const uint32_t d = mod_small(ra * p.am[t], ma, ia);
             ca = -balance(pow_small(d, ma - 2, ma, ia), ma);
@@ -445,7 +453,7 @@ __global__ void setup_kernel(const __grid_constant__ RnsSlots p, uint32_t chunks
     for (uint32_t g = 0; g < kSetupNumbers; g++) {
         if (s_f[g] == kFlagRun) {
             const uint32_t a = mod_lazy(ra[g], ma, ia), b = mod_lazy(rb[g], mb, ib);
-            slots(g, mod_small(a, ma, ia), mod_small(b, mb, ib));
+            slots(g, mod_small(a, ma, ia), mod_small(b, mb, ib), 1);
         } else {  // an all-zero lane
             const uint64_t at = slot_at(chunks, first + g, t);
             num_a[at] = num_b[at] = state[at] = __half(0.0f);
@@ -454,28 +462,34 @@ __global__ void setup_kernel(const __grid_constant__ RnsSlots p, uint32_t chunks
     __syncthreads();
     for (uint32_t g = 0; g < kSetupNumbers; g++) {
         if (s_f[g] != kFlagRun || s_divide[g] == 0 || s_out[g]) continue;  // the same for the whole block
-        const bool one = s_divide[g] == 1;
-        __syncthreads();
-        if (t == 0) {
-            uint64_t r = 0;
-            int top = -1;
-            for (int w = (int)limbs - 1; w >= 0; w--) {
-                r = r << 32 | s_n[g][w];
-                s_n[g][w] = (uint32_t)(r / s_by[g]);
-                if (top < 0 && s_n[g][w]) top = w;
-                r %= s_by[g];
+        uint32_t by = 1;  // one or two primes of A, 16 bits each
+        for (;;) {
+            __syncthreads();
+            const uint32_t m = s_by[g];
+            const bool take = by == 1 || (by >> 16 == 0 && m != by);
+            if (t == 0) {
+                uint64_t r = 0;
+                int top = -1;
+                for (int w = (int)limbs - 1; w >= 0; w--) {
+                    r = r << 32 | s_n[g][w];
+                    s_n[g][w] = (uint32_t)(r / m);
+                    if (top < 0 && s_n[g][w]) top = w;
+                    r %= m;
+                }
+                s_divide[g] = 0;
+                s_f[g] = take && near_widest(s_n[g], top, bits, a_mant, a_exp, s_q[g]) ? kFlagRun : kFlagOther;
             }
-            s_divide[g] = 0;
-            s_f[g] = one && near_widest(s_n[g], top, bits, a_mant, a_exp, s_q[g]) ? kFlagRun : kFlagOther;
+            __syncthreads();
+            if (s_f[g] != kFlagRun) break;
+            by = by == 1 ? m : by | m << 16;
+            slots(g, limbs_mod(s_n[g], limbs, ma, ia), limbs_mod(s_n[g], limbs, mb, ib), by);
+            __syncthreads();
+            if (s_divide[g] == 0 || s_out[g]) break;
         }
         __syncthreads();
-        const uint32_t by = s_by[g];
-        if (s_f[g] == kFlagRun) slots(g, limbs_mod(s_n[g], limbs, ma, ia), limbs_mod(s_n[g], limbs, mb, ib));
-        __syncthreads();
-        if (t == 0 && s_divide[g]) s_f[g] = kFlagOther;  // another factor of A in N / m
-        if (t == 0) s_by[g] = by, s_out[g] = 0;
-        __syncthreads();
+        if (t == 0) s_by[g] = by;
     }
+    __syncthreads();
     if (t < kSetupNumbers && first + t < n_items) {
         flag[first + t] = s_out[t] ? kFlagComposite : s_f[t];
         quot[first + t] = s_q[t];
@@ -1320,9 +1334,9 @@ __global__ void verdict_kernel(const __grid_constant__ RnsSlots p, uint32_t chun
                 }
             }
             if (!have) break;                                     // N shares a factor with them all
-            const uint32_t by = factor[i];
-            if (ok && by > 1) {
-                // the chain ran mod N / by: the value mod by, 2^((N - 1) / 2^(d + 1)), has to agree
+            for (uint32_t rest = factor[i]; ok && rest > 1; rest >>= 16) {
+                // the chain ran without this factor: 2^((N - 1) / 2^(d + 1)) mod it has to agree
+                const uint32_t by = rest & 0xFFFFu;
                 const uint32_t e = by - 1, ie = inv32_of(e), sh = d + 1;
                 uint32_t r = 0;
                 for (int w = (int)limbs - 1; w >= 0; w--) {
