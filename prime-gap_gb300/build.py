@@ -41,6 +41,7 @@ ORACLE_LIB = ORACLE_BUILD / "libm2oracle.so"
 ORACLE_BIN = ORACLE_BUILD / "m2_oracle"
 ARITH_HOST_LIB = BUILD / "libpgarith_host.so"
 TUNE_HOST_LIB = BUILD / "libpgtune_host.so"
+RNS_HOST_LIB = BUILD / "libpgrns_host.so"
 
 
 def _run(cmd: list[str]) -> None:
@@ -130,10 +131,19 @@ def build_tune_host() -> Path:
     return TUNE_HOST_LIB
 
 
+def build_rns_host() -> Path:
+    """Host build of the residue system's moduli, for CPU unit tests."""
+    BUILD.mkdir(parents=True, exist_ok=True)
+    src = TESTS_NATIVE / "rns_host.cpp"
+    if src.exists() and _stale(RNS_HOST_LIB, [src] + _headers()):
+        _run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", f"-I{CSRC}", str(src), "-o", str(RNS_HOST_LIB)])
+    return RNS_HOST_LIB
+
+
 def build_all(jobs: int = 8, verbose: bool = False, reference: bool = True) -> None:
     with cf.ThreadPoolExecutor(max_workers=3) as ex:
         futs = [ex.submit(build_lib, jobs, verbose), ex.submit(build_oracle),
-                ex.submit(build_arith_host), ex.submit(build_tune_host)]
+                ex.submit(build_arith_host), ex.submit(build_tune_host), ex.submit(build_rns_host)]
         if reference:
             futs.append(ex.submit(build_reference))
         for f in futs:

@@ -21,7 +21,8 @@
 // Exact arithmetic in floating point.  Residues are balanced, |xi| <= 2048, so
 // one f16 holds one; a matrix entry is split as c = lo + hi, |lo| <= 32 and hi a
 // multiple of 64, each exact in f16, and the two sums stay below 2^24 (times 64
-// for hi): the tensor core's f32 accumulators hold them exactly.  Everything
+// for hi), which the choice of the moduli sees to (pg_rns_moduli.h): the tensor
+// core's f32 accumulators hold them exactly.  Everything
 // between the products is f32 multiply-adds whose results are whole numbers
 // below 2^24 (the remainder of T by m: q = rint(T/m) by adding 1.5 2^23, then
 // T - q m, exact in a fused multiply-add).
@@ -40,6 +41,7 @@
 // alone take 2.9 (128 columns cost 78 cycles per 16 of K; 64 columns cost the same,
 // the A operand's read, hence blocks of 128) and the residues' f32 operations 3.4.
 #include "pg_rns.h"
+#include "pg_rns_moduli.h"
 
 #include <cuda_fp16.h>
 
@@ -56,7 +58,6 @@ namespace pg {
 
 namespace {
 
-constexpr uint32_t kSlots = 32;                        // residue slots per chunk
 constexpr uint32_t kMaxK = kSlots * kRnsMaxChunks;     // 288
 constexpr uint32_t kWarps = 16;                        // warps that compute residues
 constexpr uint32_t kThreads = 32 * (kWarps + 1);       // and one that issues products
@@ -84,7 +85,7 @@ struct RnsSlots {
 struct RnsPlan {
     RnsConst k;
     RnsSlots s;
-    double a_mant;        // A = a_mant 2^a_exp, a_mant in [1, 2)
+    double a_mant;        // A = a_mant 2^a_exp, a_mant in [1/2, 1)
     int a_exp;
     uint32_t t_max;       // largest multiple of N between two values of one residue
 };
@@ -100,87 +101,6 @@ uint32_t inverse(uint32_t a, uint32_t m) {  // extended Euclid; a and m coprime
 }
 
 float balanced(uint32_t x, uint32_t m) { return x > m / 2 ? (float)x - (float)m : (float)x; }
-
-// The moduli of 32n slots in each base and the bits that they hold.  A takes
-// primes alone (N has to be a unit there); B ends with composite moduli near
-// 4096 made of small primes of their own, which hold more than the primes that
-// they stand in for (2136-bit numbers fit six chunks, not seven).
-struct RnsModuli {
-    std::vector<uint32_t> a, b;
-    uint32_t b_primes = 0;
-    double bits = 0;  // numbers below 2^bits
-};
-
-double log2_product(const std::vector<uint32_t> &v) {
-    double l = 0;
-    for (uint32_t q : v) l += std::log2((double)q);
-    return l;
-}
-
-// |x| <= c N; 4 c^2 N <= A and c N <= B / 4
-double coefficient(size_t k) { return 0.5 * (double)k + 1; }
-double a_capacity(double log_a, size_t k) { return log_a - 2 - 2 * std::log2(coefficient(k)); }
-
-RnsModuli make_moduli(uint32_t n) {
-    const uint32_t k = kSlots * n;
-    std::vector<uint8_t> comp(4097, 0), used(4097, 0);
-    std::vector<uint32_t> primes, extra;
-    for (uint32_t q = 2; q <= 4096; q++) {
-        if (comp[q]) continue;
-        primes.push_back(q);
-        for (uint32_t t = q * q; t <= 4096; t += q) comp[t] = 1;
-    }
-    for (uint32_t c = 4096; c > 3900; c--) {
-        std::vector<uint32_t> f;
-        uint32_t rest = c;
-        for (uint32_t q : primes) {
-            if (q > 200) break;
-            if (rest % q == 0 && !used[q]) f.push_back(q);
-            while (rest % q == 0 && !used[q]) rest /= q;
-        }
-        if (!comp[c] || rest != 1) continue;
-        for (uint32_t q : f) used[q] = 1;
-        extra.push_back(c);
-    }
-    // A needs log2 c + 2 more bits than B: it gets the first `lead` primes
-    RnsModuli best;
-    for (uint32_t lead = 0; lead < 24; lead++) {
-        RnsModuli m;
-        size_t top = primes.size();
-        while (top > 0 && (m.a.size() + 1 < k || m.b.size() + extra.size() < k)) {
-            const uint32_t q = primes[--top];
-            if (used[q]) continue;
-            const bool b_full = m.b.size() + extra.size() >= k;
-            (m.a.size() + 1 < k && (b_full || m.a.size() < m.b.size() + lead) ? m.a : m.b).push_back(q);
-        }
-        m.b_primes = (uint32_t)m.b.size();
-        m.b.insert(m.b.end(), extra.begin(), extra.end());
-        const double c = coefficient(m.a.size());
-        m.bits = std::fmin(a_capacity(log2_product(m.a), m.a.size()), log2_product(m.b) - 2 - std::log2(c));
-        m.b.resize(k, 1);  // slots left over: modulus 1, all zero
-        if (m.bits > best.bits) best = m;
-    }
-    return best;
-}
-
-const RnsModuli &moduli_of(uint32_t n) {
-    static const std::vector<RnsModuli> all = [] {
-        std::vector<RnsModuli> v(kRnsMaxChunks + 1);
-        for (uint32_t i = 1; i <= kRnsMaxChunks; i++) v[i] = make_moduli(i);
-        return v;
-    }();
-    return all[n];
-}
-
-// How many of A's moduli numbers below 2^bits take: no more, so that A / N stays
-// small (the start needs A mod N).
-uint32_t a_count(uint32_t n, uint32_t bits) {
-    const RnsModuli &mod = moduli_of(n);
-    double la = 0;
-    uint32_t k = 0;
-    while (k < mod.a.size() && (k == 0 || a_capacity(la, k) - 1e-6 < (double)bits)) la += std::log2((double)mod.a[k++]);
-    return k;
-}
 
 void make_plan(uint32_t n, uint32_t ka, RnsPlan &p) {
     const RnsModuli &mod = moduli_of(n);

@@ -7,7 +7,6 @@
 
 namespace pg {
 
-constexpr uint32_t kRnsMaxChunks = 9;   // 32 residue slots each
 constexpr uint32_t kRnsDumps = 12;      // last values kept for the strong test's verdict
 constexpr uint32_t kRnsTile = 256;      // numbers of a tile, half in each CTA of a pair
 constexpr uint32_t kRnsGroup = 4;       // most tiles that a pair takes in turn
