@@ -33,7 +33,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <numeric>
 #include <vector>
 
 #include "pg_arith.cuh"
@@ -445,7 +444,7 @@ struct PrpPart {
 };
 
 // The parts of a list of numbers of these widths; `order` becomes the order in which
-// they are tested.  The residue form takes numbers of nearly one width.  Where a list
+// they are tested, where it is not the list's.  The residue form takes numbers of nearly one width.  Where a list
 // spreads further, it takes the bands of kRnsSpread bits whose many numbers are worth a
 // wave of their own, with or without the widest numbers' band; one launch of the limb
 // form takes the rest, at the rest's own width; or the limb form takes all, where that is
@@ -456,8 +455,6 @@ struct PrpPart {
 // 78, 17.)
 std::vector<PrpPart> prp_parts(const std::vector<uint32_t> &width, std::vector<uint64_t> &order) {
     const uint64_t n = width.size();
-    order.resize(n);
-    std::iota(order.begin(), order.end(), 0ull);
     const auto [min, max] = std::minmax_element(width.begin(), width.end());
     const uint32_t lo = *min, hi = *max;
     if (hi - lo <= kRnsSpread) return {{0, n, prp_plan(hi, n)}};
@@ -502,6 +499,7 @@ std::vector<PrpPart> prp_parts(const std::vector<uint32_t> &width, std::vector<u
         if (us < best_us && parts.size() > 1) best_us = us, best = parts, best_of = of;
     }
     if (best.size() == 1) return best;
+    order.resize(n);
     std::vector<uint64_t> at(best.size());
     for (size_t i = 1; i < best.size(); i++) best[i].first = best[i - 1].first + best[i - 1].count;
     for (size_t i = 0; i < best.size(); i++) at[i] = best[i].first;
@@ -866,6 +864,7 @@ int pgs_prp_test(pgs_ctx *ctx, const uint32_t *limbs, uint32_t n_limbs, size_t c
     if (dev_rows.empty()) return PGS_OK;
     std::vector<uint64_t> order;
     std::vector<pg::PrpPart> parts = pg::prp_parts(widths, order);
+    const auto at = [&](uint64_t i) { return order.empty() ? i : order[i]; };
     size_t words = 0, work_bytes = 0;
     for (const auto &part : parts) {
         words += part.count * 8u * (size_t)part.plan.L;
@@ -885,7 +884,7 @@ int pgs_prp_test(pgs_ctx *ctx, const uint32_t *limbs, uint32_t n_limbs, size_t c
     for (const auto &part : parts) {
         const uint32_t n = 8u * (uint32_t)part.plan.L;
         for (uint64_t j = 0; j < part.count; j++, to += n) {
-            std::memcpy(to, limbs + dev_rows[order[part.first + j]] * n_limbs, std::min(n, n_limbs) * 4u);
+            std::memcpy(to, limbs + dev_rows[at(part.first + j)] * n_limbs, std::min(n, n_limbs) * 4u);
             items[part.first + j] = pg::PrpItem{(uint32_t)j, 0};
         }
     }
@@ -913,7 +912,7 @@ int pgs_prp_test(pgs_ctx *ctx, const uint32_t *limbs, uint32_t n_limbs, size_t c
         ctx->err = "pgs_prp_test: a wait on the device gave up";
         return PGS_ETIMEOUT;
     }
-    for (size_t j = 0; j < dev_rows.size(); j++) out[dev_rows[order[j]]] = res[j];
+    for (size_t j = 0; j < dev_rows.size(); j++) out[dev_rows[at(j)]] = res[j];
     return PGS_OK;
 }
 
