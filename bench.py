@@ -810,9 +810,16 @@ def run_prp(args, rank, world, local):
     import prp_oracle as po
 
     bits = po.primorial_k(job["p"], job["d"]).bit_length() + int(max(lists["m"])).bit_length()
-    k = 32 * next(i + 1 for i, b in enumerate(RNS_WIDTHS) if bits <= b)
-    ops = launched / args.steps * bits * 2 * (2 * k * 2 * k)
-    tensor_peak, tensor_source = _tensor_peak()
+    chunks = next((i + 1 for i, b in enumerate(RNS_WIDTHS) if bits <= b), None)
+    roofline = None  # wider numbers are tested limb by limb, without the tensor cores
+    if chunks:
+        k = 32 * chunks
+        ops = launched / args.steps * bits * 2 * (2 * k * 2 * k)
+        tensor_peak, tensor_source = _tensor_peak()
+        roofline = {"kernel": f"chain_tiles_kernel<{chunks}>, chain_kernel<{chunks}>", "bound": "tensor",
+                    "achieved": ops / dt, "peak": tensor_peak, "unit": "FLOP/s", "frac": ops / dt / tensor_peak,
+                    "traffic": None, "peak_source": tensor_source,
+                    "note": "the f32 pipe, which turns the products' sums into residues, is the busier one"}
     cpu = None
     if not args.no_cpu:
         c = _prp_cpu_sample(lists, job, 1, rows=16)
@@ -830,10 +837,7 @@ def run_prp(args, rank, world, local):
                    "value_is": "lists on the host to gaps on the host"},
         "prp_tests_per_s": counted / args.steps / dt, "prp_launched_per_s": launched / args.steps / dt,
         "rounds_per_step": rounds / args.steps, "from_prepared_job_ms": prepared_ms,
-        "roofline": {"kernel": f"chain_tiles_kernel<{k // 32}>, chain_kernel<{k // 32}>", "bound": "tensor",
-                     "achieved": ops / dt, "peak": tensor_peak, "unit": "FLOP/s", "frac": ops / dt / tensor_peak,
-                     "traffic": None, "peak_source": tensor_source,
-                     "note": "the f32 pipe, which turns the products' sums into residues, is the busier one"},
+        "roofline": roofline,
         "cpu_baseline": cpu, "clocks": clock_info, "gpu_launches": args.steps * (4 + 6 * rounds // args.steps),
         "e2e": {"value": value, "unit": "m/s", "h2d_bytes_per_step": rows * 24 + 4 * int(len(lists["dist"])),
                 "d2h_bytes_per_step": rows * 20},
