@@ -443,21 +443,19 @@ struct PrpPart {
     PrpPlan plan;
 };
 
-// The parts of a list of numbers of these widths; `order` becomes the order in which
-// they are tested, where it is not the list's.  The residue form takes numbers of nearly one width.  Where a list
-// spreads further, it takes the bands of kRnsSpread bits whose many numbers are worth a
-// wave of their own, with or without the widest numbers' band; one launch of the limb
-// form takes the rest, at the rest's own width; or the limb form takes all, where that is
-// the fastest.  (All through the residue form at the widest number's width and what it
-// left through the limb form as well, the limb form for all, and in parts, in ms: 15
-// numbers of 2136 bits and one of 2161 29.0, 16.1, 16.1; 2000 of 300 to 2800 bits 53, 29,
-// 29; 9000 of 2838 and one of 2863 132, 106, 51; 9000 of 2136 and 9000 of 1400 51,
-// 78, 17.)
-std::vector<PrpPart> prp_parts(const std::vector<uint32_t> &width, std::vector<uint64_t> &order) {
+// The parts of a list of numbers of these widths, `lo` to `hi`, that spread over more than
+// kRnsSpread; `order` becomes the order in which they are tested, where it is not the
+// list's.  The residue form, which takes numbers of nearly one width, gets the bands of
+// kRnsSpread bits whose many numbers are worth a wave of their own, with or without the
+// widest numbers' band; one launch of the limb form takes the rest, at the rest's own
+// width; or the limb form takes all, where that is the fastest.  (All through the residue
+// form at the widest number's width and what it left through the limb form as well, the
+// limb form for all, and in parts, in ms: 15 numbers of 2136 bits and one of 2161 29.0,
+// 16.1, 16.1; 2000 of 300 to 2800 bits 53, 29, 29; 9000 of 2838 and one of 2863 132, 106,
+// 51; 9000 of 2136 and 9000 of 1400 51, 78, 17.)
+std::vector<PrpPart> prp_parts(const std::vector<uint32_t> &width, uint32_t lo, uint32_t hi,
+                               std::vector<uint64_t> &order) {
     const uint64_t n = width.size();
-    const auto [min, max] = std::minmax_element(width.begin(), width.end());
-    const uint32_t lo = *min, hi = *max;
-    if (hi - lo <= kRnsSpread) return {{0, n, prp_plan(hi, n)}};
     // numbers of each width below w, and the sum of their widths
     std::vector<uint64_t> below(hi + 2, 0), sum(hi + 2, 0);
     for (uint32_t w : width) below[w + 1]++;
@@ -838,19 +836,24 @@ int pgs_prp_test(pgs_ctx *ctx, const uint32_t *limbs, uint32_t n_limbs, size_t c
     CK(cudaSetDevice(ctx->device));
     if (count == 0) return PGS_OK;
     // the widths; tiny, even and too wide numbers on the host
-    std::vector<uint32_t> widths;
+    uint32_t lo = ~0u, hi = 0;
     std::vector<uint64_t> dev_rows;
-    for (size_t i = 0; i < count; i++) {
+    dev_rows.reserve(count);
+    const auto width = [&](size_t i) {
         const uint32_t *v = limbs + i * n_limbs;
         uint32_t top = n_limbs;
         while (top > 0 && v[top - 1] == 0) top--;
-        const uint32_t bits = top ? 32u * (top - 1) + (32u - (uint32_t)__builtin_clz(v[top - 1])) : 0u;
+        return top ? 32u * (top - 1) + (32u - (uint32_t)__builtin_clz(v[top - 1])) : 0u;
+    };
+    for (size_t i = 0; i < count; i++) {
+        const uint32_t *v = limbs + i * n_limbs;
+        const uint32_t bits = width(i);
         if (bits > 8u * pg::kMaxL * 32u - 4u) {
             ctx->err = "pgs_prp_test: numbers above 4092 bits";
             return PGS_EINVAL;
         }
         if (bits <= 3) {  // 0..7: the reference's answers for 2, 3, 5, 7 are prime
-            const uint32_t v0 = top ? v[0] : 0u;
+            const uint32_t v0 = bits ? v[0] : 0u;
             out[i] = (v0 == 2 || v0 == 3 || v0 == 5 || v0 == 7) ? 1 : 0;
             continue;
         }
@@ -858,12 +861,20 @@ int pgs_prp_test(pgs_ctx *ctx, const uint32_t *limbs, uint32_t n_limbs, size_t c
             out[i] = 0;
             continue;
         }
-        widths.push_back(bits);
+        lo = std::min(lo, bits);
+        hi = std::max(hi, bits);
         dev_rows.push_back(i);
     }
     if (dev_rows.empty()) return PGS_OK;
     std::vector<uint64_t> order;
-    std::vector<pg::PrpPart> parts = pg::prp_parts(widths, order);
+    std::vector<pg::PrpPart> parts;
+    if (hi - lo <= pg::kRnsSpread) {
+        parts.push_back({0, dev_rows.size(), pg::prp_plan(hi, dev_rows.size())});
+    } else {
+        std::vector<uint32_t> widths(dev_rows.size());
+        for (size_t j = 0; j < widths.size(); j++) widths[j] = width(dev_rows[j]);
+        parts = pg::prp_parts(widths, lo, hi, order);
+    }
     const auto at = [&](uint64_t i) { return order.empty() ? i : order[i]; };
     size_t words = 0, work_bytes = 0;
     for (const auto &part : parts) {

@@ -46,6 +46,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -1282,12 +1283,18 @@ __global__ void verdict_kernel(const __grid_constant__ RnsSlots p, uint32_t chun
 // Tiles per pair: enough that their residues take longer than one tile's exchange.
 constexpr uint32_t kTilesOf[kRnsMaxChunks + 1] = {0, 4, 3, 2, 2, 2, 2, 1, 1, 1};
 
-// Pairs of CTAs that run at once, one CTA per SM.
+// Pairs of CTAs that run at once, one CTA per SM (asked of each device once: the search's
+// expectations ask hundreds of times).
 uint64_t pairs_at_once() {
+    static std::atomic<int> known[64];
     int device = 0, sms = 0;
-    if (cudaGetDevice(&device) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms < 2)
-        return 76;
+    if (cudaGetDevice(&device) != cudaSuccess) return 76;
+    const bool keep = device >= 0 && device < 64;
+    if (keep) sms = known[device].load(std::memory_order_relaxed);
+    if (sms == 0) {
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms < 2) return 76;
+        if (keep) known[device].store(sms, std::memory_order_relaxed);
+    }
     return (uint64_t)sms / 2;
 }
 
