@@ -975,8 +975,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(32 * ChainShape<N>::
 // operand in TMEM: the next one replaces it when its product's last sums are in,
 // so a product's residues wait in registers; B's residues, needed again for the
 // next square, are kept in shared memory (what does not fit, in TMEM).
-// 38912 numbers of 2136 bits: 22.3 ms against 24.4 ms in two single waves (58368
-// of 712 bits: 4.6 against 5.4), the f32 pipe 68 % busy, the tensor cores 47 %.
+// 38912 numbers of 2120 bits: 19.4 ms against 21.9 ms in two single waves (38912 of 1060
+// bits 5.2, 5.1; 58368 of 700 bits 3.4, three waves 4.0; 77824 of 340 bits 1.33, four
+// waves 1.47), the f32 pipe 68 % busy, the tensor cores 52 %.
 // Reading the next sums while residues are computed made it slower here (24.9 ms;
 // two chunks at once 24.1).
 template <uint32_t N, uint32_t T>
