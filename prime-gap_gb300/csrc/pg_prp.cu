@@ -453,7 +453,7 @@ struct PrpPart {
 // limb form for all, and in parts, in ms: 15 numbers of 2136 bits and one of 2161 29.0,
 // 16.1, 16.1; 2000 of 300 to 2800 bits 53, 29, 29; 9000 of 2838 and one of 2863 132, 106,
 // 51; 9000 of 2136 and 9000 of 1400 51, 78, 17.)
-std::vector<PrpPart> prp_parts(const std::vector<uint32_t> &width, uint32_t lo, uint32_t hi,
+std::vector<PrpPart> prp_parts(const std::vector<uint16_t> &width, uint32_t lo, uint32_t hi,
                                std::vector<uint64_t> &order) {
     const uint64_t n = width.size();
     // numbers of each width below w, and the sum of their widths
@@ -837,17 +837,15 @@ int pgs_prp_test(pgs_ctx *ctx, const uint32_t *limbs, uint32_t n_limbs, size_t c
     if (count == 0) return PGS_OK;
     // the widths; tiny, even and too wide numbers on the host
     uint32_t lo = ~0u, hi = 0;
+    std::vector<uint16_t> widths;
     std::vector<uint64_t> dev_rows;
+    widths.reserve(count);
     dev_rows.reserve(count);
-    const auto width = [&](size_t i) {
+    for (size_t i = 0; i < count; i++) {
         const uint32_t *v = limbs + i * n_limbs;
         uint32_t top = n_limbs;
         while (top > 0 && v[top - 1] == 0) top--;
-        return top ? 32u * (top - 1) + (32u - (uint32_t)__builtin_clz(v[top - 1])) : 0u;
-    };
-    for (size_t i = 0; i < count; i++) {
-        const uint32_t *v = limbs + i * n_limbs;
-        const uint32_t bits = width(i);
+        const uint32_t bits = top ? 32u * (top - 1) + (32u - (uint32_t)__builtin_clz(v[top - 1])) : 0u;
         if (bits > 8u * pg::kMaxL * 32u - 4u) {
             ctx->err = "pgs_prp_test: numbers above 4092 bits";
             return PGS_EINVAL;
@@ -863,6 +861,7 @@ int pgs_prp_test(pgs_ctx *ctx, const uint32_t *limbs, uint32_t n_limbs, size_t c
         }
         lo = std::min(lo, bits);
         hi = std::max(hi, bits);
+        widths.push_back((uint16_t)bits);
         dev_rows.push_back(i);
     }
     if (dev_rows.empty()) return PGS_OK;
@@ -871,8 +870,6 @@ int pgs_prp_test(pgs_ctx *ctx, const uint32_t *limbs, uint32_t n_limbs, size_t c
     if (hi - lo <= pg::kRnsSpread) {
         parts.push_back({0, dev_rows.size(), pg::prp_plan(hi, dev_rows.size())});
     } else {
-        std::vector<uint32_t> widths(dev_rows.size());
-        for (size_t j = 0; j < widths.size(); j++) widths[j] = width(dev_rows[j]);
         parts = pg::prp_parts(widths, lo, hi, order);
     }
     const auto at = [&](uint64_t i) { return order.empty() ? i : order[i]; };
