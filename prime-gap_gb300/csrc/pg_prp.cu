@@ -936,13 +936,15 @@ struct RoundCost {
     double unknowns, chance;
     double us(uint64_t searches, uint64_t items, bool residues) const {
         double total = 0, left = (double)searches;
-        for (int round = 0; round < 100 && left >= 0.2; round++) {
+        for (int round = 0; round < 20 && left >= 0.2; round++) {
             double each = std::min((double)items / left, (double)kMaxSpec);
             if (!residues) each = std::min(each, unknowns);
             const double count = std::ceil(each * left);
             total += 130 + (residues ? pg::rns_us(bits, (uint64_t)count) : pg::limb_us(bits, count * bits));
             left *= std::exp(-each * chance);
         }
+        if (left >= 0.2)  // many more rounds like these
+            total *= std::log(5.0 * (double)searches) / std::log((double)searches / left);
         return total;
     }
     // Candidates of a round of the limb form: blocks on each SM that are full.  (Both
