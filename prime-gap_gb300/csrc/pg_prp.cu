@@ -375,10 +375,11 @@ struct PrpPlan {
 // Whole calls in ms (limbs, residues) at the widths where a step up of one form's time
 // comes before the other's, elsewhere the residue form is ahead from one number on:
 //   253-360 bits, a chunk: 300 bits, one number 0.32, 0.39; two 0.40, 0.39
-//   361-508, two chunks and two limbs per lane: 430 bits, 9728 numbers 0.97, 1.03;
-//     19456 1.75, 1.17; at 1.3 waves of single tiles 2.1, 2.1
+//   361-508, two chunks and two limbs per lane: 430 bits, 9728 numbers (four blocks on
+//     each SM) 0.97, 1.03; 9729 1.14, 1.03; 19456 1.75, 1.15; 24320 (a wave and a
+//     quarter of single tiles) 2.11, 2.11, 26752 2.29, 2.11
 //   509-735, two and three: 735 bits, two 1.30, 1.45; four 1.49, 1.45
-//   736-764, three and three: 764 bits, 4864 1.87, 1.98; 7296 2.23, 2.02
+//   736-764, three and three: 764 bits, 4864 (two blocks) 1.87, 1.98; 5000 2.20, 1.99
 //   1104-1276, four and five: 1276 bits, one 4.44, 4.53; two 4.65, 4.53
 //   1464-1532, five and six: 1464 bits, two 6.18, 6.26; four 6.57, 6.27
 // and the others: 765 bits, one 1.97, 1.87; 1100 bits 3.83, 2.67; 2136 bits 15.0, 11.0;
@@ -390,9 +391,9 @@ bool rns_pays(uint32_t bits, uint64_t items) {
     const uint64_t wave = rns_wave(bits, false);
     switch (16 * n + (uint32_t)L) {
         case 16 * 1 + 2: return items >= 2;
-        case 16 * 2 + 2: return items >= 5 * wave / 8 && !(items > wave && items < 7 * wave / 5);
+        case 16 * 2 + 2: return items > wave / 2 && !(items > wave && items <= 5 * wave / 4);
         case 16 * 2 + 3: return items >= 4;
-        case 16 * 3 + 3: return items >= 3 * wave / 10;
+        case 16 * 3 + 3: return items > wave / 4;
         case 16 * 4 + 5: return items >= 2;
         case 16 * 5 + 6: return items >= 4;
         default: return true;
@@ -872,7 +873,7 @@ int pgs_prp_test(pgs_ctx *ctx, const uint32_t *limbs, uint32_t n_limbs, size_t c
     } else {
         parts = pg::prp_parts(widths, lo, hi, order);
     }
-    const auto at = [&](uint64_t i) { return order.empty() ? i : order[i]; };
+    const auto at = [from = order.empty() ? nullptr : order.data()](uint64_t i) { return from ? from[i] : i; };
     size_t words = 0, work_bytes = 0;
     for (const auto &part : parts) {
         words += part.count * 8u * (size_t)part.plan.L;
